@@ -73,25 +73,36 @@ struct JobParam {
 };
 constexpr int kJobCounters = 2 + kStages + 1;  // leaves, steps, deaths by stage 0..9
 
-// Control block of one search (device memory).
+// Control block of one search (device memory).  Words that many warps add to
+// or poll during a launch have a cache line each: L2 takes one access to a
+// line at a time.
 struct Ctl {
   long long top;                 // nodes on the frontier stack
   long long batch;               // this launch's input: stack[top - batch .. top)
-  unsigned long long cursor;     // input nodes taken
-  unsigned long long nout;       // nodes written to the output buffer
   long long peak;
   unsigned long long nsurv;      // survivors found (records kept: min(nsurv, cap))
-  int dump;                      // persistent: end the epoch now
-  int busy;                      // persistent: warps holding work or claiming it
-  int idle;                      // persistent: warps waiting for work (starved)
-  int deep;                      // persistent: warps holding 2 or more stack nodes (work a dump would spread)
   int error;                     // kErr* bits
   int launches;
   // utilisation counters: warp rounds, running lanes summed over rounds,
   // pool donations and claims, idle-warp polls
   u64 rounds, lane_rounds, donations, claims, polls;
+  alignas(128) unsigned long long cursor;  // input nodes taken
+  alignas(128) unsigned long long nout;    // nodes written to the output buffer
+  alignas(128) int dump;         // persistent: end the epoch now
+  int busy;                      // persistent: warps holding work or claiming it
+  int idle;                      // persistent: warps waiting for work (starved)
+  int deep;                      // persistent: warps holding 2 or more stack nodes (work a dump would spread)
+  // persistent: machines handed to the long-machine kernel in this epoch; in
+  // that kernel, fork nodes kept, children queued, and queue items taken and
+  // finished
+  alignas(128) int nlong;
+  int long_nodes;
+  alignas(128) int long_head;
+  alignas(128) int long_more;
+  alignas(128) int long_done;
   // persistent: nodes donated by warps with deep stacks to warps without work
-  // (slots [pool_head, pool_tail) are waiting; each counter on its own cache line)
+  // (slots [pool_head, pool_tail) are waiting, pool_avail of them written)
+  alignas(128) int pool_avail;
   alignas(128) unsigned long long pool_head;
   alignas(128) unsigned long long pool_tail;
 };

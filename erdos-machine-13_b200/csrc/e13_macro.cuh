@@ -1,0 +1,391 @@
+// e13_macro.cuh -- long machines: one warp runs one machine a tape word at a
+// time.
+//
+// A machine that lives for thousands of steps sweeps over tape it has written
+// before, so the same things happen inside the same words again and again.
+// What a machine does inside one 32-cell word depends only on its state, the
+// side it enters from and the word's content, so the warp remembers the
+// outcome of each such visit (new content, exit side and state, steps) in a
+// small direct-mapped table in shared memory and applies it in one go the next
+// time.  An entry is made when it is first needed by running the machine
+// inside the word.  A visit that leaves the word as it was and goes on into an
+// equal word in the same state is a sweep: the lanes look at the next words
+// together and the whole run is one action.
+//
+// What bounds it: the latency of one chain of dependent instructions, not
+// issue slots.  All 32 lanes run the same scalar code; what can wait is put
+// off and done by the lanes together: each visit is noted in one lane, and
+// every 32 visits the lanes test all of them against the stage hash at once.
+//
+// Every result equals single-stepping (src/e13search.c:134-177):
+//  * a remembered visit is applied only if all its steps pass the deadline;
+//  * words 0 and 42, which hold the window's ends, are single-stepped;
+//  * the stage test compares a 64-bit hash before every step.  Inside word b
+//    the hash can only take values hb ^ s with s in the span (over GF(2)) of
+//    the keys of b's cells.  32 linear functionals per word vanish on that
+//    span, so if any of them is 1 on hb ^ TGT[nt], no step of the visit can
+//    match.  Visits are undone back to the first one that fails this, and that
+//    one is single-stepped with the test;
+//  * a machine whose whole configuration repeats (inside one word, or inside
+//    three words that it has not left since) with no stage reached on the way
+//    runs on to its deadline and dies there (src/e13search.c:161).
+#pragma once
+#include "e13_device.cuh"
+
+namespace e13dev {
+
+constexpr int kMemoBits = 9;
+constexpr int kMemoSize = 1 << kMemoBits;
+constexpr int kMemoMaxSteps = 2048;  // longest remembered visit
+constexpr int kSnapEvery = 32;       // single-stepped visits between configuration snapshots
+constexpr int kLastWord = kTapeWords - 1;
+constexpr int kSpans = 32;           // functionals per word
+constexpr u32 kAll = 0xFFFFFFFFu;
+
+// What one warp needs in shared memory.  memo entry: x content on entry;
+// y bits 0..5 the key (state, side entered from: 16 = right, 32 = valid), bits
+// 6..11 the same for the word entered next, 16..31 steps (0: single-step this
+// visit); z content on exit; w table cells read (bit per cell; bare runs only).
+struct MacroMem {
+  uint4 memo[kMemoSize];
+  u32 tape[kTapeWords + 1];
+  uint2 act[16];  // the table for macro_visit: what each state does on 0 and on 1
+  u32 rows[16];
+  u32 pad[4];
+};
+
+// act words: bit 0 flip, bits 3..6 next state, bit 7 not a plain move, bits
+// 24..31 the head's move (64 for anything but a plain move: leaves the word)
+constexpr u32 kActSpecial = 0x80u;
+__device__ __forceinline__ u32 act_word(u32 code, u32 sym) {
+  if (code & kEntSpecial) return 0x40000000u | kActSpecial;
+  return ((code ^ sym) & 1u) | ((code << 1) & 0x78u) | ((code & 2u) ? 0x01000000u : 0xFF000000u);
+}
+
+// The functionals, [functional][word].
+__device__ u64 d_span[kSpans * kTapeWords];
+
+__device__ __forceinline__ unsigned long long macro_clock() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+// After a change of M.rows: the expanded table, and an empty memory of visits.
+__device__ __forceinline__ void macro_table(MacroMem &M, int lane) {
+  __syncwarp();
+  reinterpret_cast<u32 *>(M.act)[lane] = act_word((M.rows[lane >> 1] >> ((lane & 1) << 4)) & 0xFFu, (u32)lane & 1u);
+  for (int i = lane; i < kMemoSize; i += 32) M.memo[i] = make_uint4(0u, 0u, 0u, 0u);
+  __syncwarp();
+}
+
+// Runs the machine inside one word of content c until it leaves it: the entry
+// to remember.  sk: the key (state and side).
+template <bool READS>
+static __device__ __noinline__ uint4 macro_visit(const uint2 *act, u32 c, u32 sk) {
+  u32 w = c, reads = 0, x = 0;
+  int st = (int)(sk & 15u), q = (sk & 16u) ? 31 : 0, n = 0;
+  do {
+    const uint2 a = act[st];
+    const u32 sym = (w >> q) & 1u;
+    x = sym ? a.y : a.x;
+    if (READS) reads |= 1u << (2 * st + (int)sym);
+    w ^= (x & 1u) << q;
+    q += (int)x >> 24;
+    st = (int)((x >> 3) & 15u);
+    ++n;
+  } while ((unsigned)q <= 31u && n < kMemoMaxSteps);
+  if ((unsigned)q <= 31u || (x & kActSpecial)) return make_uint4(c, sk, c, 0u);
+  return make_uint4(c, sk | ((u32)(st | 32 | (q < 0 ? 16 : 0)) << 6) | ((u32)n << 16), w, reads);
+}
+
+__device__ __forceinline__ u32 span_bit(u64 v, u64 f) {
+  const u64 x = v & f;
+  return __popc((u32)x ^ (u32)(x >> 32)) & 1u;
+}
+
+// Runs a machine (L, hb, M.tape, M.rows; the same in every lane) to its next
+// event: kEvDead, kEvSurv, kEvCell (cell, ecell) or kEvRun when the clock
+// passes t_end (HASH only).  HASH: the filter, hb being the full 64-bit hash.
+// Otherwise the bare table runs until L.t is past L.deadline (kEvDead), and
+// kEvOff says that a step left the window (L.p is then outside it, that step
+// not counted); reads collects the table cells read.
+enum { kEvOff = 5 };
+
+template <bool HASH>
+__device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const KeyTabs &K, const u64 *span, int lane,
+                                         u32 &reads, int &cell, u32 &ecell, unsigned long long t_end) {
+  int p = L.p, b = L.p >> 5;
+  int left = L.deadline + 1 - L.t;  // steps that still pass the deadline test
+  u64 tgt = HASH ? s_tgt[L.nt] : 0ull;
+  u32 sk = (u32)L.st | 32u | ((p & 31) ? 16u : 0u);
+  bool single = (p & 31) != 0 && (p & 31) != 31;  // this visit step by step
+  bool inside = single;                           // the head is inside the word (at p), not on its edge
+  bool rep = false;                 // the last visit left its word alone and goes on in the same way,
+  u32 rep_c = 0;                    // from content rep_c
+  // visits not yet tested: lane j holds the j-th (its word, key, steps left
+  // before it and the cells it changed)
+  int noted = 0, v_b = 0, v_left = 0;
+  u32 v_sk = 0, v_d = 0;
+  int snap_b = 0, snap_left = 0, snaps = 0;
+  u32 snap_at = 0, snap0 = 0, snap1 = 0, snap2 = 0;  // words snap_b - 1 .. snap_b + 1
+  bool far = true;                  // left those words, or reached a stage, since the snapshot
+  for (;;) {
+    if (!single) {
+      // remembered visits, one after another.  Nothing in this loop branches
+      // but its end: what the visit changes is selected by `ok`
+      u32 c, n;
+      uint4 *slot, e;
+      bool ok, in_range, sweep;
+      do {
+        c = M.tape[b];
+        slot = M.memo + ((c * 0x9E3779B1u + sk * 0x85EBCA6Bu) >> (32 - kMemoBits));
+        e = *slot;
+        n = e.y >> 16;
+        in_range = (unsigned)(b - 1) < (unsigned)(kLastWord - 1);
+        sweep = rep && c == rep_c;
+        ok = in_range && !sweep && e.x == c && (e.y & 63u) == sk && n - 1u < (u32)left;
+        const bool mine = ok && lane == noted;
+        v_b = mine ? b : v_b;
+        v_sk = mine ? sk : v_sk;
+        v_left = mine ? left : v_left;
+        v_d = mine ? c ^ e.z : v_d;
+        if (!HASH && ok) reads |= e.w;
+        if (ok) M.tape[b] = e.z;  // every lane writes the same value
+        const u32 next = (e.y >> 6) & 63u;
+        left = ok ? left - (int)n : left;
+        noted = ok ? noted + 1 : noted;
+        rep = ok && e.z == c && next == sk;
+        rep_c = c;
+        sk = ok ? next : sk;
+        b = ok ? b + 1 - (int)((next >> 3) & 2u) : b;
+      } while (ok && noted < 32);
+      if (!ok) {
+        const bool known = e.x == c && (e.y & 63u) == sk;
+        if (in_range && sweep && known) {
+          // the i-th free lane looks at the i-th word ahead
+          const int dir = 1 - (int)((sk >> 3) & 2u), i = lane - noted;
+          const int w = b + dir * i;
+          const bool same = i >= 0 && (unsigned)(w - 1) < (unsigned)(kLastWord - 1) && M.tape[w] == c;
+          const u32 m = __ballot_sync(kAll, !same) >> noted;
+          int run = m ? __ffs(m) - 1 : 32 - noted;
+          if (run * (int)n > left) run = 0;
+          if (i >= 0 && i < run) {
+            v_b = w;
+            v_sk = sk;
+            v_left = left - i * (int)n;
+            v_d = 0;
+          }
+          noted += run;
+          left -= run * (int)n;
+          b += dir * run;
+          if (noted < 32) continue;
+        } else if (in_range && !known) {
+          const uint4 v = macro_visit<!HASH>(M.act, c, sk);
+          __syncwarp();
+          if (lane == 0) *slot = v;
+          __syncwarp();
+          if (v.y >> 16) continue;
+          single = true;
+        } else {
+          single = true;  // an end of the window, a visit to be single-stepped, or too few steps left
+        }
+      }
+    }
+
+    if (noted) {
+      // test the visits noted
+      __syncwarp();
+      const bool mine = lane < noted;
+      bool bad = false;
+      u64 sum = 0;
+      const u64 start = hb;
+      if (HASH) {
+        u32 lo = 0, hi = 0;
+        for (u32 d = mine ? v_d : 0u; d; d &= d - 1) {
+          const int i = 32 * v_b + __ffs(d) - 1;
+          lo ^= K.lo[i];
+          hi ^= K.hi[i];
+        }
+        const u32 lo0 = lo, hi0 = hi;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {  // running hash changes
+          const u32 a = __shfl_up_sync(kAll, lo, o), c = __shfl_up_sync(kAll, hi, o);
+          if (lane >= o) {
+            lo ^= a;
+            hi ^= c;
+          }
+        }
+        sum = ((u64)(hi ^ hi0) << 32) | (lo ^ lo0);  // before this lane's visit
+        const u64 v = hb ^ sum ^ tgt;
+        bad = mine;
+        for (int j = 0; j < kSpans && __any_sync(kAll, bad); j += 4) {
+          u32 any = 0;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) any |= span_bit(v, span[(j + k) * kTapeWords + v_b]);
+          if (any) bad = false;
+        }
+        hb ^= ((u64)__shfl_sync(kAll, hi, 31) << 32) | __shfl_sync(kAll, lo, 31);
+      }
+      u32 m = __ballot_sync(kAll, bad);
+      if (m) {
+        // back to the first visit that a stage start might fall into
+        const int j = __ffs(m) - 1;
+        if (mine && lane >= j && v_d) atomicXor(&M.tape[v_b], v_d);
+        __syncwarp();
+        b = __shfl_sync(kAll, v_b, j);
+        sk = __shfl_sync(kAll, v_sk, j);
+        left = __shfl_sync(kAll, v_left, j);
+        hb = start ^ (((u64)__shfl_sync(kAll, (u32)(sum >> 32), j) << 32) | __shfl_sync(kAll, (u32)sum, j));
+        single = true;
+        noted = j;
+      }
+      // do the visits that stand contain a turn of a loop?  Visit j enters the
+      // same word in the same way as visit 0, and between them only visit 0's
+      // word and its neighbours were entered and ended as they were
+      const int b0 = __shfl_sync(kAll, v_b, 0);
+      const u32 sk0 = __shfl_sync(kAll, v_sk, 0);
+      if (__any_sync(kAll, lane < noted && (unsigned)(v_b - snap_b + 1) > 2u)) far = true;
+      m = __ballot_sync(kAll, lane > 0 && lane < noted && v_b == b0 && v_sk == sk0);
+      if (m) {
+        const int j = __ffs(m) - 1;
+        const bool in = lane < j;
+        const bool out = __any_sync(kAll, in && (unsigned)(v_b - b0 + 1) > 2u);
+        if (!out) {
+          const u32 x0 = __reduce_xor_sync(kAll, (in && v_b == b0 - 1) ? v_d : 0u);
+          const u32 x1 = __reduce_xor_sync(kAll, (in && v_b == b0) ? v_d : 0u);
+          const u32 x2 = __reduce_xor_sync(kAll, (in && v_b == b0 + 1) ? v_d : 0u);
+          if ((x0 | x1 | x2) == 0u) {
+            if (HASH) {
+              L.t = L.deadline + 1;
+              return kEvDead;
+            }
+            const int period = __shfl_sync(kAll, v_left, 0) - __shfl_sync(kAll, v_left, j);
+            left %= period;
+          }
+        }
+      }
+      noted = 0;
+      rep = false;
+      if (HASH && macro_clock() > t_end) {
+        L.p = b * 32 + ((sk & 16u) ? 31 : 0);
+        L.st = (int)(sk & 15u);
+        L.t = L.deadline + 1 - left;
+        return kEvRun;
+      }
+    }
+    if (!single) continue;
+
+    // single steps until the head is in another word
+    int st = (int)(sk & 15u);
+    if (!inside) p = b * 32 + ((sk & 16u) ? 31 : 0);
+    // a loop that passes through here every turn: the same configuration
+    // again, on words not left since the snapshot?
+    if ((unsigned)(b - snap_b + 1) > 2u) far = true;
+    const u32 at_here = ((u32)p << 4) | (u32)st;
+    if (!far && at_here == snap_at && M.tape[b] == snap1 && M.tape[b - 1] == snap0 && M.tape[b + 1] == snap2) {
+      if (HASH) left = 0;
+      else left %= snap_left - left;
+      far = true;
+    }
+    if (--snaps < 0 && (unsigned)(b - 1) < (unsigned)(kLastWord - 1)) {
+      snaps = kSnapEvery;
+      snap_b = b;
+      snap_at = at_here;
+      snap_left = left;
+      snap0 = M.tape[b - 1];
+      snap1 = M.tape[b];
+      snap2 = M.tape[b + 1];
+      far = false;
+      if (HASH && macro_clock() > t_end) {
+        L.p = p;
+        L.st = st;
+        L.t = L.deadline + 1 - left;
+        return kEvRun;
+      }
+    }
+    u32 word = M.tape[b];
+    u32 lw = 0;  // a configuration inside this word seen earlier
+    int lat = -1, lleft = 0, lk = 0, lnext = 32, ev = -1;
+    do {
+      if (left <= 0) {
+        ev = kEvDead;
+        break;
+      }
+      const uint2 a = M.act[st];
+      const u32 sym = (word >> (p & 31)) & 1u;
+      const u32 x = sym ? a.y : a.x;
+      if (x & kActSpecial) {
+        cell = (st << 1) | (int)sym;
+        ecell = (M.rows[st] >> (sym << 4)) & 0xFFu;
+        ev = kEvCell;
+        break;
+      }
+      if (!HASH) reads |= 1u << ((st << 1) | (int)sym);
+      if (x & 1u) {
+        word ^= 1u << (p & 31);
+        if (HASH) hb ^= ((u64)K.hi[p] << 32) | K.lo[p];
+      }
+      const int np = p + ((int)x >> 24);
+      if ((unsigned)(np - 1) >= (unsigned)(kTapeCells - 2)) {  // head <= -64 or >= 1299
+        ev = kEvDead;
+        if (!HASH) {
+          p = np;
+          ev = kEvOff;
+        }
+        break;
+      }
+      p = np;
+      st = (int)((x >> 3) & 15u);
+      --left;
+      if (HASH && hb == tgt) {
+        M.tape[b] = word;
+        L.hb = (u32)hb;
+        L.p = p;
+        L.st = st;
+        L.t = L.deadline + 1 - left;
+        const int nt = L.nt;
+        ev = stage_check(L, M.tape, K, 1);
+        if (ev) break;
+        ev = -1;
+        if (L.nt != nt) {
+          left = L.deadline + 1 - L.t;
+          tgt = s_tgt[L.nt];
+          lat = -1;
+          far = true;
+        }
+      }
+      if (++lk >= lnext) {  // (the first 31 steps are not looked at)
+        const int at = (p << 4) | st;
+        if (at == lat && word == lw) {  // it loops inside this word
+          if (HASH) {
+            left = 0;
+            ev = kEvDead;
+            break;
+          }
+          left %= lleft - left;
+          lat = -1;
+        } else if (lk >= 2 * lnext || lat < 0) {
+          lat = at;
+          lw = word;
+          lleft = left;
+          lnext = lk;
+        }
+      }
+    } while ((p >> 5) == b);
+    M.tape[b] = word;
+    if (ev >= 0) {
+      L.p = p;
+      L.st = st;
+      L.t = L.deadline + 1 - left;
+      __syncwarp();
+      return ev;
+    }
+    b = p >> 5;
+    sk = (u32)st | 32u | ((p & 31) ? 16u : 0u);
+    single = inside = false;
+    rep = false;
+  }
+}
+
+}  // namespace e13dev

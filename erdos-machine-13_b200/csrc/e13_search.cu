@@ -15,9 +15,11 @@
 //    is deep donates its oldest node to a device pool when the pool runs low;
 //    warps without work take pool nodes.  An epoch takes the whole frontier as
 //    its input and ends on a time bound (or when every warp is out of work):
-//    warps then dump live lanes and stack nodes back to the frontier.  Epochs
-//    are replayed from a captured CUDA graph; the host reads the control block
-//    once per graph.
+//    warps then dump live lanes and stack nodes back to the frontier.  Old
+//    machines are handed over to long_kernel, which follows in the same epoch
+//    and runs one machine per warp a tape word at a time.  Epochs are replayed
+//    from a captured CUDA graph; the host reads the control block once per
+//    graph.
 //
 // In both, a machine whose budget is spent takes first reads of cells that
 // can no longer fork as plain steps (clear_unread); survivors get their read
@@ -39,6 +41,7 @@
 
 #include "e13.h"
 #include "e13_device.cuh"
+#include "e13_macro.cuh"
 #include "e13_node.cuh"
 
 using namespace e13dev;
@@ -50,13 +53,41 @@ constexpr long long kPoolNodes = 1LL << 18;  // donation pool: 256 Ki nodes (80 
 constexpr long long kWholeFrontier = 1LL << 62;  // persistent batch when e13_tuning::batch is 0
 constexpr long long kPoolWaitNs = 200000000;     // 200 ms: a donor publishes a claimed slot within microseconds
 constexpr long long kMinEpochNs = 200000;        // 200 us: the shortest epoch a starvation dump may end
-// A warp with at most kLoneLanes running machines (the tail of a search:
-// a few long machines, the rest of the GPU idle) runs each of them in the
-// tight single-machine loop step_slice, up to kLoneSteps steps per
-// iteration: its speed is then bound by one machine's dependent chain, not
-// by issue slots, and the lock-step loop's control would only lengthen it.
+// A warp with at most kLoneLanes running machines runs each of them in the
+// tight single-machine loop step_slice, up to kLoneSteps steps per iteration
+// (kLoneStepsShort in the persistent kernel): its speed is then bound by one
+// machine's dependent chain, not by issue slots, and the lock-step loop's
+// control would only lengthen it.
 constexpr int kLoneLanes = 2;
 constexpr int kLoneSteps = 512;
+constexpr int kLoneStepsShort = 64;  // persistent: its long machines are handed over between slices
+
+// Long machines.  In lock-step a long machine costs a lane 0.3 us a step; alone
+// in a warp of long_kernel (e13_macro.cuh) one of 835,000 steps takes 1.5-3 ms,
+// but one of 2,000 steps as long as in lock-step, with a warp to itself.  So
+// while there is other work a machine is handed over only after run_skip x 2
+// steps since its load, and while an eighth of the warps wait for work after
+// kParkMin (machines that die at the deadline of stage 4, 1137 steps, are
+// never worth it: with 512 the FMAX = 3 search of X = 8 took 28 ms, with 1536
+// 18 ms, everything else equal).
+// The counter neighbourhoods (FMAX = 2, 61 machines) went from 20-240 ms to
+// 8-12 ms, their tails being in-place loops and zigzag sweeps to the deadline.
+constexpr int kLongCap = 1 << 14;        // machines handed over per epoch, at most
+constexpr int kLongNodes = 1 << 14;      // fork nodes long_kernel keeps for its own queue
+constexpr int kLongItems = 1 << 15;      // children it queues
+constexpr int kLongOut = kLongCap + kLongItems;  // most nodes it puts on the outputs
+constexpr int kLongBlock = 256;
+constexpr int kLongPerSm = 2;            // 96 KB of shared memory a block
+constexpr long long kLongMinNs = 1000000;  // shortest time bound of long_kernel: 1 ms (else a tenth of the epoch)
+constexpr int kIdlePark = 8;             // many warps wait: an eighth
+constexpr int kParkMin = 1536;
+// Taking input and pool nodes.  One word of L2 takes an atomic or a polling
+// read at a time, so blocks claim input in chunks (at most kInputChunk nodes,
+// at least kInputChunks claims a block) and a warp donates up to kGive stack
+// nodes at once while many warps wait.
+constexpr int kInputChunk = 32;
+constexpr int kInputChunks = 16;
+constexpr int kGive = 8;
 
 // steps a lane gets between warp-level refill rounds is Params::slice
 
@@ -65,8 +96,14 @@ struct Params {
   unsigned long long *jobcnt;  // kMaxJobs x kJobCounters totals
   int nq;
   int slice, step_cap, wdepth, pool_low, run_skip;
-  int skip_after;            // run skip only in slices of warps with a machine of at least this many steps
+  int park_after, park_idle; // persistent: hand a machine over after this many steps since its load (while
+                             // warps wait for work)
   long long out_cap, out_soft, surv_cap, pool_cap;
+  long long stack_cap;       // frontier capacity of this search
+  long long out_nodes;       // frontier room an epoch's own outputs may need
+  long long long_ns;         // long_kernel: unfinished machines go back to the frontier after this long
+  Node *longq;               // kLongCap machines handed over, then kLongNodes fork nodes
+  unsigned long long *long_items;  // queued children: launch tag, node, move
   long long epoch_ns;
   long long wait_ns;         // persistent: limit of the wait for a claimed pool slot's data
   long long min_epoch_ns;    // persistent: an epoch may end early for starvation only after this long
@@ -114,23 +151,23 @@ static __device__ __noinline__ u32 survivor_reads(u32 *tcol, const u32 *rcol, in
   return read;
 }
 
-// Appends a survivor record (kept only below the cap).  reads: the persistent
-// kernel has the lane re-run the table for the read mask (its warp goes on
-// alone, the others are not held up); the plain kernel, whose launch would
-// wait for that lane, records the flags as they are and leaves the mask to
-// survivor_read_masks() once the search is over.  Out of line: it is rare, and
-// the step loop keeps its registers.
+// Appends a survivor record (kept only below the cap).  reads: the cells its
+// run read (survivor_reads in the persistent kernel, whose warp goes on alone;
+// macro_run in the long-machine kernel), or 0 in the plain kernel, whose
+// launch would wait for that lane: it records the flags as they are and
+// leaves the mask to survivor_read_masks() once the search is over.  Out of
+// line: it is rare, and the step loop keeps its registers.
 static __device__ __noinline__ void record_survivor(Ctl *ctl, SurvRec *surv, long long surv_cap, int st0, int p0,
                                                     int flags, int t, int job, u32 *tcol, const u32 *rcol,
-                                                    int stride, bool reads) {
+                                                    int stride, u32 reads) {
   const unsigned long long k = atomicAdd(&ctl->nsurv, 1ull);
   if ((long long)k >= surv_cap) return;
   SurvRec *r = surv + k;
-  const u32 read = reads ? survivor_reads(tcol, rcol, stride, t) : 0u;
+  if (tcol) reads = survivor_reads(tcol, rcol, stride, t);
   for (int c = 0; c < 32; ++c) {
     const u32 e = (rcol[(c >> 1) * stride] >> ((c & 1) << 4)) & 0xFFu;
     if (!reads) r->ent[c] = (unsigned char)e;
-    else r->ent[c] = (unsigned char)(e == kEntFree ? e : (((read >> c) & 1u) ? (e & 0x7Fu) : (e | kEntUnread)));
+    else r->ent[c] = (unsigned char)(e == kEntFree ? e : (((reads >> c) & 1u) ? (e & 0x7Fu) : (e | kEntUnread)));
   }
   r->st0 = st0;
   r->head0 = p0 - kLeft;
@@ -142,10 +179,101 @@ static __device__ __noinline__ void record_survivor(Ctl *ctl, SurvRec *surv, lon
 
 enum { kStRun = 0, kStIdle = 1, kStFork = 2, kStCap = 3, kStDead = 4, kStSurv = 5 };
 
+// A block's view of the persistent kernel's control words.  All warps of the
+// GPU polling the same few words of L2 held up the warps at work (the first
+// epoch of a search of 1000 machines took 408 us, with one poller per block
+// 210 us), so each block keeps a copy in shared memory that one of its warps
+// renews.
+struct View {
+  int lock;
+  int dump;      // end the epoch now
+  int more;      // work may still come: some warp holds work, or the pool does
+  int tokens;    // pool nodes waiting that this block's idle warps have not gone for
+  int starving;  // many warps wait for work, and the pool holds less than one node for each
+  unsigned time;  // of the last renewal, SM cycles
+};
+constexpr unsigned kViewCycles = 1000;  // a younger view is not renewed
+
+// By one lane: renews the view (and ends the epoch where it is due) unless
+// another warp of the block is at it.
+static __device__ __noinline__ void refresh_view(View *s_view, const Params &P, unsigned long long t_begin) {
+  volatile View *v = s_view;
+  if ((unsigned)clock64() - v->time < kViewCycles || v->lock || atomicCAS(&s_view->lock, 0, 1) != 0) return;
+  Ctl *ctl = P.ctl;
+  const unsigned long long now = globaltimer();
+  const int busy = *((volatile int *)&ctl->busy);  // before the pool: work in flight is seen in one of the two
+  const int idle = *((volatile int *)&ctl->idle), deep = *((volatile int *)&ctl->deep);
+  int d = *((volatile int *)&ctl->dump);
+  const long long nout = (long long)*((volatile unsigned long long *)&ctl->nout);
+  __threadfence();
+  const int wait = max(0, *((volatile int *)&ctl->pool_avail));
+  const int busy2 = *((volatile int *)&ctl->busy);
+  const int nwarps = (int)(((long long)gridDim.x * blockDim.x) >> 5);
+  if (!d) {
+    d = now - t_begin > (unsigned long long)P.epoch_ns || nout > P.out_soft;
+    // starving.  Work spreads inside an epoch only through donated nodes,
+    // which a few deep warps hand out one at a time: a job whose subtrees
+    // are shallow would run on a few warps for a long time.  When more
+    // than half of the warps wait for work and some warp holds a stack
+    // of 2 or more nodes, end the epoch (after a shortest length): the
+    // dump puts every warp's stack on the frontier and the next epoch
+    // deals it out over all warps.  (With no deep stack left, the work
+    // is a few long-running machines that a dump would not spread.)
+    if (now - t_begin > (unsigned long long)P.min_epoch_ns && 2 * idle > nwarps && deep > 0) d = 1;
+    if (d) *((volatile int *)&ctl->dump) = 1;
+  }
+  v->dump = d;
+  v->more = busy != 0 || wait > 0 || busy2 != 0;
+  v->tokens = (wait + (int)gridDim.x - 1) / (int)gridDim.x;
+  v->starving = kIdlePark * idle > nwarps && wait < idle;
+  v->time = (unsigned)clock64();
+  __threadfence_block();
+  v->lock = 0;
+}
+
+// A block's share of the input: nodes [next, end) claimed from ctl->cursor in
+// chunks, so that warps taking one node at a time do not queue for one word.
+struct Input {
+  unsigned long long range;  // next in the low half, end in the high half
+  int lock, done;
+};
+
+// By one lane: the next input node of this block (batch: none left).
+static __device__ __noinline__ long long next_input(Input *in, Ctl *ctl, long long batch, int chunk) {
+  volatile Input *v = in;
+  for (;;) {
+    unsigned long long r = v->range;
+    while ((u32)r < (u32)(r >> 32)) {
+      const unsigned long long got = atomicCAS(&in->range, r, r + 1);
+      if (got == r) return (long long)(u32)r;
+      r = got;
+    }
+    if (v->done) return batch;
+    if (atomicCAS(&in->lock, 0, 1) == 0) {
+      r = v->range;
+      if ((u32)r >= (u32)(r >> 32) && !v->done) {
+        const unsigned long long k = atomicAdd(&ctl->cursor, (unsigned long long)chunk);
+        if ((long long)k >= batch) {
+          v->done = 1;
+        } else {
+          const unsigned long long e = min((unsigned long long)batch, k + chunk);
+          atomicExch(&in->range, (e << 32) | k);
+        }
+      }
+      __threadfence_block();
+      v->lock = 0;
+    } else {
+      __nanosleep(50);
+    }
+  }
+}
+
 __device__ __forceinline__ int wrap(int s, int d) { return s >= d ? s - d : s; }
 
 template <bool PERSIST>
-__global__ void __launch_bounds__(768, 1) search_kernel(const Params P) {
+__global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ Params P) {
+  // an epoch with nothing to do (the search ended inside its graph of epochs)
+  if (P.ctl->top == 0 && P.ctl->pool_tail == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const KeyTabs K = key_tables(smem_raw);
   u32 *tape = reinterpret_cast<u32 *>(smem_raw + kKeySmemBytes);
@@ -157,6 +285,21 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const Params P) {
   __shared__ int4 s_jp[kMaxJobs];                              // per-job moves and symmetry range
   __shared__ unsigned long long s_jc[kMaxJobs][kJobCounters];  // per-job leaves, steps, deaths by stage
 
+  // persistent: the block's view of the control words (refresh_view)
+  __shared__ View s_view;
+  __shared__ Input s_in;
+  __shared__ unsigned long long s_stat[5];
+  if (threadIdx.x < 5) s_stat[threadIdx.x] = 0;
+  if (PERSIST && threadIdx.x == 0) {
+    s_in.range = 0;
+    s_in.lock = 0;
+    s_in.done = 0;
+    s_view.lock = 0;
+    s_view.time = (unsigned)clock64() - kViewCycles;
+    s_view.dump = 0;
+    s_view.more = 1;
+    s_view.starving = kIdlePark * P.ctl->batch < ((long long)gridDim.x * blockDim.x >> 5);
+  }
   fill_key_tables(K);
   if (threadIdx.x < kMaxJobs) {
     const JobParam jp = P.jobs[threadIdx.x];
@@ -175,7 +318,11 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const Params P) {
   Ctl *ctl = P.ctl;
   const long long top0 = ctl->top;
   const long long batch = ctl->batch;
+  const int chunk = (int)max(1ll, min((long long)kInputChunk, batch / (kInputChunks * (long long)gridDim.x)));
   const int tag = ctl->launches + 1;  // marks pool slots written in this launch
+  // handed-over machines come back to the frontier: no more of them than it
+  // has room for beside an epoch's outputs
+  const int long_cap = PERSIST ? (int)max(0ll, min((long long)kLongCap, P.stack_cap - top0 - P.out_nodes)) : 0;
   const int D = P.wdepth;
   Node *wst = PERSIST ? P.wstack + gwarp * D : nullptr;
   const unsigned long long t_begin = PERSIST ? globaltimer() : 0ull;
@@ -205,6 +352,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const Params P) {
   L.job = 0;
 
   // warp-uniform state
+  const int nwarps_all = (int)(((long long)gridDim.x * stride) >> 5);
   int sp = 0, wbot = 0;        // persistent: this warp's DFS stack, a ring of D slots from wbot
   bool have_cur = false;       // cursor registers hold the children left of the current node
   const Node *cur = nullptr;   // plain: the current input node
@@ -215,9 +363,8 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const Params P) {
   bool top_dirty = false;      // persistent: the stack top lives only in the shared copy (its HBM slot is stale)
   bool counted_idle = false;   // persistent, lane 0: this warp is counted in ctl->idle
   bool counted_deep = false;   // persistent, lane 0: this warp is counted in ctl->deep
-  const int nwarps_all = (int)(((long long)gridDim.x * stride) >> 5);
+  bool starving = PERSIST && kIdlePark * batch < nwarps_all;  // persistent: many warps wait for work
   int rounds = 0;              // slices run: a warp dumps only after one (progress every epoch)
-  unsigned backoff = 256;
   unsigned long long st_lane_rounds = 0, st_polls = 0;
   unsigned st_donations = 0, st_claims = 0;
 
@@ -337,36 +484,39 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const Params P) {
               busy = true;
             }
             long long k = batch;
-            // once an epoch is ending, leave the rest of the input where it is
-            if (lane == 0 && !(PERSIST && *((volatile int *)&ctl->dump)))
-              k = (long long)atomicAdd(&ctl->cursor, 1ull);
+            if (!PERSIST) {
+              if (lane == 0) k = (long long)atomicAdd(&ctl->cursor, 1ull);
+            } else if (lane == 0 && !((volatile View *)&s_view)->dump) {
+              // once an epoch is ending, the rest of the input is left where it is
+              k = next_input(&s_in, ctl, batch, chunk);
+            }
             k = __shfl_sync(kFull, k, 0);
             if (k >= batch) input_done = true;
             else src = P.stack + (top0 - 1 - k);
           }
-          if (PERSIST && !src && (im == kFull || (rounds & 3) == 0)) {
+          if (PERSIST && !src && (im == kFull || (rounds & 3) == 0 || starving)) {
             long long h = -1;
             int inc = 0;
-            if (lane == 0 && !*((volatile int *)&ctl->dump)) {
-              unsigned long long hh = *((volatile unsigned long long *)&ctl->pool_head);
-              const unsigned long long tl = *((volatile unsigned long long *)&ctl->pool_tail);
-              const unsigned long long lim = tl < (unsigned long long)P.pool_cap ? tl : (unsigned long long)P.pool_cap;
-              if (hh < lim && !busy) {
-                atomicAdd(&ctl->busy, 1);  // only when there is something to take
-                inc = 1;
-              }
-              while (hh < lim) {
-                const unsigned long long got = atomicCAS(&ctl->pool_head, hh, hh + 1);
-                if (got == hh) {
-                  h = (long long)hh;
-                  break;
+            if (lane == 0 && !((volatile View *)&s_view)->dump) {
+              // a claim takes one off the count of written slots and then the
+              // next slot.  (Thousands of warps in a compare-and-swap loop on
+              // the head got 2 nodes a microsecond out of the pool, as every
+              // success failed all the others: warps spent 74-94 % of the
+              // short epochs of an FMAX = 3 search there, now 5-18 % in the
+              // whole refill.)
+              if (*((volatile int *)&ctl->pool_avail) > 0) {
+                if (!busy) {
+                  atomicAdd(&ctl->busy, 1);  // only when there is something to take
+                  inc = 1;
                 }
-                hh = got;
+                if (atomicSub(&ctl->pool_avail, 1) > 0) h = (long long)atomicAdd(&ctl->pool_head, 1ull);
+                else atomicAdd(&ctl->pool_avail, 1);
               }
               if (h >= 0) {
-                // the donor claimed the slot before writing it; wait (bounded) for its data
-                const unsigned long long t0 = globaltimer();
+                // slots are counted in any order: wait (bounded) for this one's data
+                unsigned long long t0 = 0;
                 while (*((volatile int *)&P.pool_ready[h]) != tag) {
+                  if (t0 == 0) t0 = globaltimer();
                   if (globaltimer() - t0 > (unsigned long long)P.wait_ns) {
                     atomicOr(&ctl->error, kErrTimeout);
                     h = -1;
@@ -409,7 +559,6 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const Params P) {
             cur_vm = src->vmask;
           }
           have_cur = true;
-          backoff = 256;
         }
       }
       const Node *N = PERSIST ? mytop : cur;
@@ -448,50 +597,36 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const Params P) {
         atomicAdd(&ctl->deep, counted_deep ? -1 : 1);
         counted_deep = !counted_deep;
       }
-      int d = 0;
-      if (!has_work || (rounds & 7) == 0) {  // the control words are in L2: read them every 8th round
-        if (lane == 0) {
-          d = *((volatile int *)&ctl->dump);
-          if (!d && globaltimer() - t_begin > (unsigned long long)P.epoch_ns) d = 1;
-          if (!d && (long long)*((volatile unsigned long long *)&ctl->nout) > P.out_soft) d = 1;
-          if (d) *((volatile int *)&ctl->dump) = 1;
-        }
-        d = __shfl_sync(kFull, d, 0);
-      }
       if (!has_work) {
-        // nothing here: done when no warp holds work and the pool is empty, else wait for a donation
-        int done = d;
-        if (lane == 0 && !done && input_done) {
-          const int b = *((volatile int *)&ctl->busy);
-          const unsigned long long hh = *((volatile unsigned long long *)&ctl->pool_head);
-          const unsigned long long tl = *((volatile unsigned long long *)&ctl->pool_tail);
-          const unsigned long long lim = tl < (unsigned long long)P.pool_cap ? tl : (unsigned long long)P.pool_cap;
-          done = (b == 0 && hh >= lim);
-        }
-        done = __shfl_sync(kFull, done, 0);
-        if (done) break;
-        // starving.  Work spreads inside an epoch only through donated nodes,
-        // which a few deep warps hand out one at a time: a job whose subtrees
-        // are shallow would run on a few warps for a long time.  When more
-        // than half of the warps wait for work and some warp holds a stack
-        // of 2 or more nodes, end the epoch (after a shortest length): the
-        // dump puts every warp's stack on the frontier and the next epoch
-        // deals it out over all warps.  (With no deep stack left, the work
-        // is a few long-running machines that a dump would not spread.)
+        // nothing here: done when no warp holds work and the pool is empty,
+        // else wait for a node of the pool
+        int done = 0;
         if (lane == 0) {
           if (!counted_idle) {
             atomicAdd(&ctl->idle, 1);
             counted_idle = true;
-          } else if (backoff >= 1024 && globaltimer() - t_begin > (unsigned long long)P.min_epoch_ns &&
-                     2 * *((volatile int *)&ctl->idle) > nwarps_all && *((volatile int *)&ctl->deep) > 0) {
-            *((volatile int *)&ctl->dump) = 1;
+          }
+          volatile View *v = &s_view;
+          for (;;) {
+            refresh_view(&s_view, P, t_begin);
+            done = v->dump || !v->more;
+            if (done || (v->tokens > 0 && atomicSub(&s_view.tokens, 1) > 0)) break;
+            __nanosleep(100);
           }
         }
         ++st_polls;
-        __nanosleep(backoff);
-        backoff = backoff < 8192 ? 2 * backoff : 8192;
+        done = __shfl_sync(kFull, done, 0);
+        if (done) break;
         continue;
       }
+      int d = 0;
+      if (lane == 0) {
+        if ((rounds & 7) == 0) refresh_view(&s_view, P, t_begin);  // the control words are in L2: every 8th round
+        d = ((volatile View *)&s_view)->dump | (((volatile View *)&s_view)->starving << 1);
+      }
+      d = __shfl_sync(kFull, d, 0);
+      starving = d & 2;
+      d &= 1;
       if (d && rounds > 0) {
         // dump: live lanes as resume nodes, then this warp's stack
         if (status == kStRun) {
@@ -523,24 +658,29 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const Params P) {
         if (busy && lane == 0) atomicSub(&ctl->busy, 1);
         break;
       }
-      // donate the oldest node of a deep stack when the pool runs low
-      if (sp >= 2 && (rounds & 3) == 0) {
+      // donate the oldest node of a deep stack when the pool runs low, or
+      // several while many warps wait
+      if (sp >= 2 && (starving || (rounds & 3) == 0)) {
         long long s = -1;
+        const int give = starving ? min(sp - 1, kGive) : 1;
         if (lane == 0) {
-          const unsigned long long hh = *((volatile unsigned long long *)&ctl->pool_head);
-          const unsigned long long tl = *((volatile unsigned long long *)&ctl->pool_tail);
-          if (tl < (unsigned long long)P.pool_cap && tl - hh < (unsigned long long)P.pool_low)
-            s = (long long)atomicAdd(&ctl->pool_tail, 1ull);
+          const int low = starving ? max(P.pool_low, *((volatile int *)&ctl->idle)) : P.pool_low;
+          if (*((volatile int *)&ctl->pool_avail) < low &&
+              *((volatile unsigned long long *)&ctl->pool_tail) < (unsigned long long)P.pool_cap)
+            s = (long long)atomicAdd(&ctl->pool_tail, (unsigned long long)give);
         }
         s = __shfl_sync(kFull, s, 0);
-        if (s >= 0 && s < P.pool_cap) {
-          copy_node(P.pool + s, wst + wbot, lane);
+        if (s >= 0) {
+          const int n = (int)min((long long)give, max(0ll, P.pool_cap - s));
+          for (int i = 0; i < n; ++i) copy_node(P.pool + s + i, wst + wrap(wbot + i, D), lane);
           __threadfence();
           __syncwarp();
-          if (lane == 0) atomicExch(&P.pool_ready[s], tag);
-          wbot = wrap(wbot + 1, D);
-          --sp;
-          ++st_donations;
+          if (lane < n) atomicExch(&P.pool_ready[s + lane], tag);
+          __syncwarp();
+          if (lane == 0) atomicAdd(&ctl->pool_avail, n);
+          wbot = wrap(wbot + n, D);
+          sp -= n;
+          st_donations += n;
         }
       }
     }
@@ -549,10 +689,11 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const Params P) {
     ++rounds;
     {
       const unsigned rm = __ballot_sync(kFull, status == kStRun);
-      // word-at-a-time run skips pay off only for machines that have built
-      // long runs: the warp uses them in this slice when one of its machines
-      // has run skip_after steps (a warp-uniform choice: no divergence)
-      const bool skip_w = P.run_skip && __any_sync(kFull, status == kStRun && L.t >= P.skip_after);
+      // the plain kernel's launches wait for their slowest lane, the oldest
+      // machine: it skips over runs a tape word at a time, and a warp with at
+      // most kLoneLanes machines runs each in the single-machine loop.  The
+      // persistent kernel hands old machines over instead (below), and on
+      // young ones the skip arithmetic costs more than it saves.
       const bool lone_w = __popc(rm) <= kLoneLanes;
       st_lane_rounds += __popc(rm);
       if (rm) {
@@ -568,10 +709,10 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const Params P) {
               // the same steps and events as lane_act (step_slice follows
               // src/e13search.c:134-177 too); a hash match ends the iteration
               // and goes to the one stage test below
-              int n = kLoneSteps;
+              int n = PERSIST ? kLoneStepsShort : kLoneSteps;
               ev = step_slice(L.p, L.st, L.t, L.deadline, L.hb, L.tgt, tcol, rcol, K.lo, stride, n, cell);
               if (ev == kEvCell) e = get_entry(rcol, stride, cell);
-            } else if (skip_w) {
+            } else if (!PERSIST && P.run_skip) {
               ev = lane_act<true>(L, tcol, rcol, K, stride, cell, e);
               if (!ev) ev = lane_act<true>(L, tcol, rcol, K, stride, cell, e);
             } else {
@@ -626,10 +767,23 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const Params P) {
                 atomicAdd(&s_jc[L.job][2 + L.stage], 1ull);
               }
             } else {
-              record_survivor(P.ctl, P.surv, P.surv_cap, L.st0, L.p0, L.flags, L.t, L.job, tcol, rcol, stride,
-                              PERSIST);
+              record_survivor(P.ctl, P.surv, P.surv_cap, L.st0, L.p0, L.flags, L.t, L.job,
+                              PERSIST ? tcol : nullptr, rcol, stride, 0u);
             }
             status = kStIdle;
+          }
+        }
+        if (PERSIST) {
+          const bool old = status == kStRun && L.t - L.tseg >= (starving ? P.park_idle : P.park_after);
+          if (__any_sync(kFull, old) && old && *((volatile int *)&ctl->nlong) < long_cap) {
+            const int k = atomicAdd(&ctl->nlong, 1);
+            if (k < long_cap) {
+              acc_steps += (u32)(L.t - L.tseg);
+              L.tseg = L.t;
+              if (acc_steps >= 0x80000000u) flush_counts();
+              lane_store(L, P.longq + k, tcol, rcol, stride, P.nq, -1, 1, 0ull);
+              status = kStIdle;
+            }
           }
         }
         if (!PERSIST && status == kStRun && L.t - L.tseg >= P.step_cap) {
@@ -645,16 +799,279 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const Params P) {
   // ---- totals
   flush_counts();
   if (lane == 0) {
-    atomicAdd(&ctl->rounds, (unsigned long long)rounds);
-    atomicAdd(&ctl->lane_rounds, st_lane_rounds);
-    atomicAdd(&ctl->polls, st_polls);
-    if (st_donations) atomicAdd(&ctl->donations, (unsigned long long)st_donations);
-    if (st_claims) atomicAdd(&ctl->claims, (unsigned long long)st_claims);
+    atomicAdd(&s_stat[0], (unsigned long long)rounds);
+    atomicAdd(&s_stat[1], st_lane_rounds);
+    atomicAdd(&s_stat[2], st_polls);
+    atomicAdd(&s_stat[3], (unsigned long long)st_donations);
+    atomicAdd(&s_stat[4], (unsigned long long)st_claims);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < kMaxJobs * kJobCounters; i += stride) {
     const unsigned long long v = (&s_jc[0][0])[i];
     if (v) atomicAdd(P.jobcnt + i, v);
+  }
+  if (threadIdx.x < 5) {
+    unsigned long long *const to[5] = {&ctl->rounds, &ctl->lane_rounds, &ctl->polls, &ctl->donations, &ctl->claims};
+    atomicAdd(to[threadIdx.x], s_stat[threadIdx.x]);
+  }
+  if (PERSIST) {
+    // input this block claimed but did not take before the epoch ended
+    const unsigned k0 = (unsigned)s_in.range, k1 = (unsigned)(s_in.range >> 32);
+    for (unsigned k = k0 + (threadIdx.x >> 5); k < k1; k += stride >> 5) {
+      unsigned long long o = 0;
+      if (lane == 0) o = atomicAdd(&ctl->nout, 1ull);
+      o = __shfl_sync(kFull, o, 0);
+      if ((long long)o < P.out_cap) copy_node(P.out + o, P.stack + (top0 - 1 - (long long)k), lane);
+      else if (lane == 0) atomicOr(&ctl->error, kErrOutFull);
+    }
+  }
+}
+
+// One warp's shared memory in long_kernel.
+struct LongMem {
+  MacroMem m;
+  Node node;
+};
+
+// A warp's machine takes a child of its first read of `cell` (entry e): -1 the
+// table's own move, now read, else move v.
+static __device__ __noinline__ void take_child(Lane &L, u32 *rows, int lane, int cell, u32 e, int v,
+                                               const JobParam &jp, bool run_skip) {
+  __syncwarp();
+  if (v < 0) {
+    if (lane == 0) set_entry(rows, 1, cell, e & 0x7Fu, run_skip);
+  } else {
+    if (e != kEntFree) {
+      L.budget -= 1;
+      if (L.budget == 0 && lane == 0) clear_unread(rows, 1);  // no first read can fork any more
+    }
+    L.nintro = sym_after(v, L.nintro, jp.sym_lo, jp.sym_hi);
+    if (lane == 0) set_entry(rows, 1, cell, (u32)v, run_skip);
+  }
+  __syncwarp();
+}
+
+// The machines the persistent kernel handed over in this epoch, one warp each
+// (e13_macro.cuh).  At a fork the warp goes on with the first child in place
+// and queues the others for any warp: an old machine's children are mostly
+// old machines too, and handing them back to the search kernel would make an
+// epoch of every fork on the longest path.  A warp without work waits while
+// some machine is queued or running.  After the time bound, or where the
+// queue is full, machines and forks go to the epoch's outputs instead.  Runs
+// between the search kernel and move_outputs.
+__global__ void __launch_bounds__(kLongBlock) long_kernel(const __grid_constant__ Params P) {
+  Ctl *ctl = P.ctl;
+  const long long slack = P.stack_cap - ctl->top - P.out_nodes;
+  const int n = (int)min((long long)ctl->nlong, max(0ll, min((long long)kLongCap, slack)));
+  if (n == 0) return;
+  // each machine and each queued child may come back as one frontier node
+  const int item_cap = (int)min((long long)kLongItems, slack - n);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const KeyTabs K = key_tables(smem_raw);
+  u64 *span = reinterpret_cast<u64 *>(smem_raw + kKeySmemBytes);
+  const int lane = threadIdx.x & 31;
+  LongMem &W = reinterpret_cast<LongMem *>(span + kSpans * kTapeWords)[threadIdx.x >> 5];
+  MacroMem &M = W.m;
+  const Node *N = &W.node;
+  fill_key_tables(K);
+  load_stage_tables();
+  for (int i = threadIdx.x; i < kSpans * kTapeWords; i += blockDim.x) span[i] = d_span[i];
+  __syncthreads();
+  const u32 tag = (u32)ctl->launches + 1u;
+  const unsigned long long t_end = macro_clock() + (unsigned long long)P.long_ns;
+  unsigned backoff = 128;
+  for (;;) {
+    // ---- take an item: a machine handed over (child -2), or a queued child
+    int k = -1, child = -2, stop = 0;
+    if (lane == 0) {
+      const int done = *((volatile int *)&ctl->long_done);
+      __threadfence();  // a finished item's children were queued before it counted as done
+      const int total = n + *((volatile int *)&ctl->long_more);
+      int h = *((volatile int *)&ctl->long_head);
+      while (h < total) {
+        const int got = atomicCAS(&ctl->long_head, h, h + 1);
+        if (got == h) {
+          k = h;
+          break;
+        }
+        h = got;
+      }
+      if (k < 0) stop = done == total || macro_clock() > t_end;
+      if (k >= n) {
+        // its warp has reserved the item and writes it next; wait (bounded)
+        const unsigned long long t0 = macro_clock();
+        unsigned long long it;
+        while ((u32)((it = *((volatile unsigned long long *)&P.long_items[k - n])) >> 32) != tag) {
+          if (macro_clock() - t0 > (unsigned long long)P.wait_ns) {
+            atomicOr(&ctl->error, kErrTimeout);
+            stop = 1;
+            break;
+          }
+        }
+        __threadfence();
+        k = (int)((it >> 8) & 0xFFFFFFu);
+        child = (int)(it & 0xFFu);
+      }
+    }
+    stop = __shfl_sync(kFull, stop, 0);
+    if (stop) break;
+    k = __shfl_sync(kFull, k, 0);
+    child = __shfl_sync(kFull, child, 0);
+    if (k < 0) {
+      __nanosleep(backoff);
+      backoff = backoff < 2048 ? 2 * backoff : 2048;
+      continue;
+    }
+    backoff = 128;
+    if (lane < kNodeChunks) reinterpret_cast<uint4 *>(&W.node)[lane] = __ldcg(reinterpret_cast<const uint4 *>(P.longq + k) + lane);
+    __syncwarp();
+
+    // ---- load it
+    Lane L;
+    L.p = N->p;
+    L.st = N->st;
+    L.t = N->t;
+    L.deadline = N->deadline;
+    L.hb = (u32)N->hb;
+    L.nt = N->nt;
+    L.stage = N->stage;
+    L.st0 = N->st0;
+    L.p0 = N->p0;
+    L.flags = N->flags & 31;
+    L.ch0 = N->ch[0];
+    L.ch1 = N->ch[1];
+    L.ch2 = N->ch[2];
+    L.nintro = N->nintro;
+    L.budget = N->budget;
+    L.job = N->job;
+    L.tgt = (u32)s_tgt[L.nt];
+    L.tseg = L.t;
+    const JobParam jp = P.jobs[L.job];
+    int lo, hi;
+    tape_extent(L.t, lo, hi);
+    u32 hh = 0;  // high half of the hash, from the tape
+    for (int w = lane; w < kTapeWords; w += 32) {
+      u32 x = (w >= lo && w <= hi) ? N->tape[w] : 0u;
+      M.tape[w] = x;
+      while (x) {
+        hh ^= K.hi[32 * w + __ffs(x) - 1];
+        x &= x - 1;
+      }
+    }
+    u64 hb = ((u64)__reduce_xor_sync(kFull, hh) << 32) | L.hb;
+    if (lane < 16) M.rows[lane] = (u32)N->cellv[2 * lane] | ((u32)N->cellv[2 * lane + 1] << 16);
+    __syncwarp();
+    // a queued child is a move of its fork node (the keep child goes on in place)
+    if (child >= 0) take_child(L, M.rows, lane, N->pend, N->cellv[N->pend] & 0xFFu, child, jp, P.run_skip);
+    macro_table(M, lane);
+
+    // ---- run it
+    int ev = kEvRun, cell = 0;
+    u32 ecell = 0, reads = 0;
+    while (macro_clock() <= t_end) {
+      ev = macro_run<true>(L, hb, M, K, span, lane, reads, cell, ecell, t_end);
+      if (ev != kEvCell) break;
+      if (ecell == kEntHalt) {
+        ev = kEvDead;
+        break;
+      }
+      int first = -1;  // a first read with nothing to branch on fixes the cell
+      if (ecell == kEntFree || L.budget > 0) {
+        int keep = 0;
+        u64 vm = 0;
+        child_set(ecell, L.budget, L.nintro, jp.nv, jp.sym_lo, jp.sym_hi, keep, vm);
+        if (!keep) {
+          first = __ffsll((long long)vm) - 1;
+          vm &= vm - 1;
+        }
+        const int rest = __popcll(vm);
+        if (rest) {
+          int slot = -1, at = 0;
+          if (lane == 0 && macro_clock() <= t_end && *((volatile int *)&ctl->long_nodes) < kLongNodes &&
+              *((volatile int *)&ctl->long_more) + rest <= item_cap) {
+            slot = atomicAdd(&ctl->long_nodes, 1);
+            if (slot < kLongNodes) {
+              L.hb = (u32)hb;
+              slot += kLongCap;
+              lane_store(L, P.longq + slot, M.tape, M.rows, 1, P.nq, cell, 0, vm);
+              __threadfence();
+              at = *((volatile int *)&ctl->long_more);
+              for (;;) {
+                if (at + rest > item_cap) {
+                  slot = -1;
+                  break;
+                }
+                const int got = atomicCAS(&ctl->long_more, at, at + rest);
+                if (got == at) break;
+                at = got;
+              }
+            } else {
+              slot = -1;
+            }
+          }
+          slot = __shfl_sync(kFull, slot, 0);
+          at = __shfl_sync(kFull, at, 0);
+          if (slot < 0) break;  // no room or no time: the whole fork goes to the frontier
+          for (int i = lane; i < rest; i += 32) {
+            *((volatile unsigned long long *)&P.long_items[at + i]) =
+                ((unsigned long long)tag << 32) | ((unsigned long long)slot << 8) | (unsigned)nth_bit64(vm, i);
+          }
+        }
+      }
+      take_child(L, M.rows, lane, cell, ecell, first, jp, P.run_skip);
+      macro_table(M, lane);  // visits that met the cell are remembered as slow
+      if (first < 0 && (ecell & 0x7Fu) == kEntHalt) {
+        ev = kEvDead;
+        break;
+      }
+      ev = kEvRun;
+    }
+
+    // ---- its end
+    L.hb = (u32)hb;
+    unsigned long long *cnt = P.jobcnt + (size_t)L.job * kJobCounters;
+    if (lane == 0) atomicAdd(cnt + 1, (unsigned long long)(L.t - L.tseg));
+    if (ev == kEvDead) {
+      if (lane == 0) {
+        atomicAdd(cnt, 1ull);
+        atomicAdd(cnt + 2 + L.stage, 1ull);
+      }
+    } else if (ev == kEvSurv) {
+      // its read mask: the final table again from the blank tape, for t steps
+      __syncwarp();
+      for (int w = lane; w < kTapeWords; w += 32) M.tape[w] = 0;
+      macro_table(M, lane);  // the visits remembered so far do not know the cells they read
+      Lane R = L;
+      R.p = kLeft;
+      R.st = 0;
+      R.t = 0;
+      R.deadline = L.t - 1;
+      reads = 0;
+      macro_run<false>(R, hb, M, K, span, lane, reads, cell, ecell, t_end);
+      if (lane == 0) {
+        atomicAdd(cnt, 1ull);
+        record_survivor(ctl, P.surv, P.surv_cap, L.st0, L.p0, L.flags, L.t, L.job, nullptr, M.rows, 1, reads);
+      }
+    } else {
+      // a fork, or out of time: to the frontier
+      int keep = 1, pend = -1;
+      u64 vm = 0;
+      if (ev == kEvCell) {
+        child_set(ecell, L.budget, L.nintro, jp.nv, jp.sym_lo, jp.sym_hi, keep, vm);
+        pend = cell;
+      }
+      __syncwarp();
+      if (lane == 0) {
+        const unsigned long long o = atomicAdd(&ctl->nout, 1ull);
+        if ((long long)o < P.out_cap + kLongOut) lane_store(L, P.out + o, M.tape, M.rows, 1, P.nq, pend, keep, vm);
+        else atomicOr(&ctl->error, kErrOutFull);
+      }
+    }
+    __syncwarp();
+    if (lane == 0) {
+      __threadfence();
+      atomicAdd(&ctl->long_done, 1);
+    }
   }
 }
 
@@ -759,6 +1176,12 @@ __global__ void finish_launch(Ctl *ctl, long long cap, long long batch_max, long
   ctl->busy = 0;
   ctl->idle = 0;
   ctl->deep = 0;
+  ctl->nlong = 0;
+  ctl->long_nodes = 0;
+  ctl->long_head = 0;
+  ctl->long_more = 0;
+  ctl->long_done = 0;
+  ctl->pool_avail = 0;
   ctl->pool_head = 0;
   ctl->pool_tail = 0;
   ctl->launches += 1;
@@ -834,6 +1257,10 @@ struct e13_ctx {
   long long pool_cap;
   int *pool_ready;
   long long pool_ready_cap;
+  Node *longq;  // machines handed to long_kernel
+  long long longq_cap;
+  unsigned long long *long_items;
+  long long long_items_cap;
   SurvRec *surv;
   long long surv_cap;
   Ctl *ctl;
@@ -866,9 +1293,47 @@ static cudaError_t d2h(e13_ctx *c, void *dst, const void *src, size_t bytes) {
   return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, c->stream);
 }
 
+// The functionals of macro_run's stage-test check: for every tape word, 32
+// independent 64-bit vectors f with popcount(f & key) even for each key of the
+// word's cells (the orthogonal complement of their span over GF(2), which
+// holds at least 32 dimensions as a word has at most 32 keys).
+static cudaError_t upload_span_functionals() {
+  uint64_t key[kTapeCells], tgt[E13_STAGES + 1];
+  e13_keys(key, tgt);
+  std::vector<u64> f((size_t)kSpans * kTapeWords);
+  for (int w = 0; w < kTapeWords; ++w) {
+    u64 row[32];     // the keys in reduced row echelon form
+    int pivot[32], rank = 0;
+    for (int i = 0; i < 32; ++i) {
+      const int cell = 32 * w + i;
+      u64 v = (cell >= kCounterCells && cell < kTapeCells) ? key[cell] : 0ull;
+      for (int r = 0; r < rank; ++r)
+        if ((v >> pivot[r]) & 1) v ^= row[r];
+      if (!v) continue;
+      int p = 0;
+      while (!((v >> p) & 1)) ++p;
+      for (int r = 0; r < rank; ++r)
+        if ((row[r] >> p) & 1) row[r] ^= v;
+      row[rank] = v;
+      pivot[rank++] = p;
+    }
+    u64 pivots = 0;
+    for (int r = 0; r < rank; ++r) pivots |= 1ull << pivot[r];
+    int n = 0;
+    for (int j = 0; j < 64 && n < kSpans; ++j) {
+      if ((pivots >> j) & 1) continue;
+      u64 v = 1ull << j;  // free coordinate j: its pivot coordinates follow
+      for (int r = 0; r < rank; ++r)
+        if ((row[r] >> j) & 1) v |= 1ull << pivot[r];
+      f[(size_t)kTapeWords * n++ + w] = v;
+    }
+  }
+  return cudaMemcpyToSymbol(d_span, f.data(), sizeof(u64) * f.size());
+}
+
 static int ensure_consts(e13_ctx *c) {
   if (c->consts_ready) return E13_OK;
-  if (upload_filter_tables() != cudaSuccess) return E13_ERR_CUDA;
+  if (upload_filter_tables() != cudaSuccess || upload_span_functionals() != cudaSuccess) return E13_ERR_CUDA;
   c->consts_ready = true;
   return E13_OK;
 }
@@ -907,6 +1372,8 @@ extern "C" void e13_ctx_destroy(e13_ctx *c) {
   cudaFree(c->wstack);
   cudaFree(c->pool);
   cudaFree(c->pool_ready);
+  cudaFree(c->longq);
+  cudaFree(c->long_items);
   cudaFree(c->surv);
   cudaFree(c->ctl);
   cudaFreeHost(c->ctl_host);
@@ -948,6 +1415,12 @@ static int grow(T **p, long long *cap, long long want) {
   return E13_OK;
 }
 
+// The long-machine kernel's buffers.
+static int grow_long(e13_ctx *c) {
+  const int rc = grow(&c->longq, &c->longq_cap, (long long)kLongCap + kLongNodes);
+  return rc ? rc : grow(&c->long_items, &c->long_items_cap, (long long)kLongItems);
+}
+
 static void decode_survivor(const SurvRec &r, int nq, e13_survivor *s) {
   memset(s, 0, sizeof *s);
   for (int i = 0; i < E13_MAXCELLS; ++i) s->tab[i] = E13_HALT;
@@ -972,7 +1445,8 @@ static void decode_survivor(const SurvRec &r, int nq, e13_survivor *s) {
 
 // Kernel parameters of a search or serve session over the context's buffers.
 // dump_room: frontier nodes the warps may write when an epoch ends.
-static Params make_params(const e13_ctx *c, const e13_tuning &tu, int nq, long long nwarps, long long dump_room) {
+static Params make_params(const e13_ctx *c, const e13_tuning &tu, int nq, long long nwarps, long long dump_room,
+                          long long stack_cap) {
   Params P;
   memset(&P, 0, sizeof P);
   P.jobs = c->d_jobs;
@@ -980,17 +1454,22 @@ static Params make_params(const e13_ctx *c, const e13_tuning &tu, int nq, long l
   P.nq = nq;
   P.slice = tu.slice;
   P.run_skip = tu.run_skip ? 1 : 0;
-  // the plain kernel's launches wait for their slowest lane, which is the
-  // oldest machine: it skips in every slice
-  P.skip_after = (tu.run_skip >= 2 && tu.kernel == E13_KERNEL_PERSISTENT) ? tu.run_skip : 0;
+  P.park_after = tu.run_skip ? std::max(kParkMin, 2 * std::min(tu.run_skip, 1 << 29)) : 0x7FFFFFFF;
+  P.park_idle = tu.run_skip ? kParkMin : 0x7FFFFFFF;
+  P.longq = c->longq;
+  P.long_items = c->long_items;
+  P.long_ns = std::max(kLongMinNs, (long long)tu.epoch_us * 1000LL / 10);
   P.step_cap = tu.step_cap;
   P.wdepth = tu.warp_stack;
   P.pool_low = (int)std::max<long long>(1, nwarps * tu.pool_low_pct / 100);
   P.pool_cap = c->pool_cap;
   P.pool = c->pool;
   P.pool_ready = c->pool_ready;
-  P.out_cap = c->out_cap;
-  P.out_soft = c->out_cap - dump_room - 1024;
+  // the persistent kernel's outputs leave kLongOut slots to long_kernel
+  P.out_cap = c->out_cap - (tu.kernel == E13_KERNEL_PERSISTENT ? kLongOut : 0);
+  P.out_soft = P.out_cap - dump_room - 1024;
+  P.out_nodes = 2 * dump_room + 65536;
+  P.stack_cap = stack_cap;
   P.surv_cap = c->surv_cap;
   P.epoch_ns = (long long)tu.epoch_us * 1000LL;
   P.wait_ns = kPoolWaitNs;
@@ -1003,8 +1482,20 @@ static Params make_params(const e13_ctx *c, const e13_tuning &tu, int nq, long l
   return P;
 }
 
+static size_t long_smem() {
+  return kKeySmemBytes + sizeof(u64) * kSpans * kTapeWords + sizeof(LongMem) * (kLongBlock / 32);
+}
+
 static size_t search_smem(int block) {
   return kKeySmemBytes + (size_t)(kTapeWords + 16) * block * 4 + (size_t)(block / 32) * sizeof(Node);
+}
+
+// Shared memory of the persistent kernel and of the long-machine kernel behind it.
+static cudaError_t set_persistent_smem(size_t smem) {
+  const cudaError_t e =
+      cudaFuncSetAttribute(search_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)long_smem());
 }
 
 // ------------------------------------------------------------------------
@@ -1300,7 +1791,7 @@ static int split_share(e13_ctx *c, const e13_job *job, const e13_tuning &tu, int
     t.slice = kSplitSlice;
     t.step_cap = kSplitStepCap;
     t.run_skip = 1;
-    Params S = make_params(c, t, job->nq, nwarps, nwarps * 32);
+    Params S = make_params(c, t, job->nq, nwarps, nwarps * 32, stack_n);
     S.jobs = jobs;
     S.jobcnt = jobcnt;
     S.stack = stack;
@@ -1393,10 +1884,11 @@ static int search_impl(e13_ctx *c, const e13_job *job, const e13_tuning *tuning,
   // the frontier capacity of this search: exactly what the tuning asks for,
   // else all that the context holds (a larger stack left by a serve session)
   const long long cap = tu.stack_nodes > 0 ? tu.stack_nodes : c->stack_cap;
-  if ((rc = grow(&c->out, &c->out_cap, out_nodes))) return rc;
+  if ((rc = grow(&c->out, &c->out_cap, out_nodes + (persist ? kLongOut : 0)))) return rc;
   if (persist && (rc = grow(&c->wstack, &c->wstack_nodes, nwarps * tu.warp_stack))) return rc;
   if (persist && (rc = grow(&c->pool, &c->pool_cap, kPoolNodes))) return rc;
   if (persist && (rc = grow(&c->pool_ready, &c->pool_ready_cap, kPoolNodes))) return rc;
+  if (persist && (rc = grow_long(c))) return rc;
   const long long scap = std::max<long long>(surv_cap, 1024);
   if ((rc = grow(&c->surv, &c->surv_cap, scap))) return rc;
 
@@ -1407,10 +1899,10 @@ static int search_impl(e13_ctx *c, const e13_job *job, const e13_tuning *tuning,
   jp[0].sym_hi = job->sym_hi;
   CK(h2d(c, c->d_jobs, jp, sizeof jp));
   CK(cudaMemsetAsync(c->d_jobcnt, 0, sizeof(unsigned long long) * kMaxJobs * kJobCounters, c->stream));
-  Params P = make_params(c, tu, job->nq, nwarps, dump_room);
+  Params P = make_params(c, tu, job->nq, nwarps, dump_room, cap);
 
   const size_t smem = search_smem(tu.block);
-  if (persist) CK(cudaFuncSetAttribute(search_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (persist) CK(set_persistent_smem(smem));
   else CK(cudaFuncSetAttribute(search_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 
   // the root: blank tape, every cell unread
@@ -1422,7 +1914,10 @@ static int search_impl(e13_ctx *c, const e13_job *job, const e13_tuning *tuning,
   c->ctl_host->peak = 1;
   CK(h2d(c, c->stack, &root, sizeof root));
   // pool slots carry the tag of the launch that wrote them; tags restart with every search
-  if (persist) CK(cudaMemsetAsync(c->pool_ready, 0, sizeof(int) * (size_t)c->pool_ready_cap, c->stream));
+  if (persist) {
+    CK(cudaMemsetAsync(c->pool_ready, 0, sizeof(int) * (size_t)c->pool_ready_cap, c->stream));
+    CK(cudaMemsetAsync(c->long_items, 0, sizeof(unsigned long long) * (size_t)c->long_items_cap, c->stream));
+  }
   CK(h2d(c, c->ctl, c->ctl_host, sizeof(Ctl)));
 
   // checkpoints: resume from the last complete slot, then save into the other one
@@ -1490,6 +1985,7 @@ static int search_impl(e13_ctx *c, const e13_job *job, const e13_tuning *tuning,
     CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     for (int e = 0; e < tu.epochs_per_graph; ++e) {
       search_kernel<true><<<blocks, tu.block, smem, c->stream>>>(P);
+      long_kernel<<<c->nsm * kLongPerSm, kLongBlock, long_smem(), c->stream>>>(P);
       move_outputs<<<move_blocks, 256, 0, c->stream>>>(c->ctl, c->stack, c->out, c->pool, c->pool_cap, cap);
       finish_launch<<<1, 1, 0, c->stream>>>(c->ctl, cap, batch_max, c->pool_cap);
     }
@@ -1497,7 +1993,7 @@ static int search_impl(e13_ctx *c, const e13_job *job, const e13_tuning *tuning,
     CK(cudaGraphInstantiate(&exec, graph, 0));
     for (;;) {
       CK(cudaGraphLaunch(exec, c->stream));
-      launches += 3LL * tu.epochs_per_graph;
+      launches += 4LL * tu.epochs_per_graph;
       search_launches += tu.epochs_per_graph;
       CK(d2h(c, c->ctl_host, c->ctl, sizeof(Ctl)));
       CK(cudaStreamSynchronize(c->stream));
@@ -1638,12 +2134,13 @@ extern "C" int e13_selftest_pool_wait(e13_ctx *c, int32_t wait_us) {
   const long long nwarps = (long long)c->nsm * tu.block / 32;
   const long long dump_room = nwarps * (32 + tu.warp_stack);
   if ((rc = grow(&c->stack, &c->stack_cap, 1024))) return rc;
-  if ((rc = grow(&c->out, &c->out_cap, 2 * dump_room + 65536))) return rc;
+  if ((rc = grow(&c->out, &c->out_cap, 2 * dump_room + 65536 + kLongOut))) return rc;
   if ((rc = grow(&c->wstack, &c->wstack_nodes, nwarps * tu.warp_stack))) return rc;
   if ((rc = grow(&c->pool, &c->pool_cap, kPoolNodes))) return rc;
   if ((rc = grow(&c->pool_ready, &c->pool_ready_cap, kPoolNodes))) return rc;
+  if ((rc = grow_long(c))) return rc;
   if ((rc = grow(&c->surv, &c->surv_cap, 1024))) return rc;
-  Params P = make_params(c, tu, 16, nwarps, dump_room);
+  Params P = make_params(c, tu, 16, nwarps, dump_room, c->stack_cap);
   P.wait_ns = (long long)wait_us * 1000LL;
   const size_t smem = search_smem(tu.block);
   CK(cudaFuncSetAttribute(search_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1653,8 +2150,10 @@ extern "C" int e13_selftest_pool_wait(e13_ctx *c, int32_t wait_us) {
   CK(cudaMemsetAsync(c->d_jobcnt, 0, sizeof(unsigned long long) * kMaxJobs * kJobCounters, c->stream));
   // ready tags 0; the launch's tag is launches + 1 = 1, so slot 0 never looks published
   CK(cudaMemsetAsync(c->pool_ready, 0, sizeof(int) * (size_t)c->pool_ready_cap, c->stream));
+  CK(cudaMemsetAsync(c->long_items, 0, sizeof(unsigned long long) * (size_t)c->long_items_cap, c->stream));
   memset(c->ctl_host, 0, sizeof(Ctl));
   c->ctl_host->pool_tail = 1;  // slot 0 donated (claimable), its data never written
+  c->ctl_host->pool_avail = 1;
   CK(h2d(c, c->ctl, c->ctl_host, sizeof(Ctl)));
   search_kernel<true><<<c->nsm, tu.block, smem, c->stream>>>(P);
   move_outputs<<<c->nsm * 4, 256, 0, c->stream>>>(c->ctl, c->stack, c->out, c->pool, c->pool_cap, c->stack_cap);
@@ -1861,18 +2360,20 @@ extern "C" int e13_serve_create(e13_ctx *c, const e13_tuning *tuning, int64_t re
   const long long stack_nodes = tu.stack_nodes > 0 ? tu.stack_nodes : (16LL << 20);
   if ((rc = grow(&c->stack, &c->stack_cap, stack_nodes))) return rc;
   s->cap = tu.stack_nodes > 0 ? tu.stack_nodes : c->stack_cap;
-  if ((rc = grow(&c->out, &c->out_cap, s->out_nodes))) return rc;
+  if ((rc = grow(&c->out, &c->out_cap, s->out_nodes + kLongOut))) return rc;
   if ((rc = grow(&c->wstack, &c->wstack_nodes, nwarps * tu.warp_stack))) return rc;
   if ((rc = grow(&c->pool, &c->pool_cap, kPoolNodes))) return rc;
   if ((rc = grow(&c->pool_ready, &c->pool_ready_cap, kPoolNodes))) return rc;
+  if ((rc = grow_long(c))) return rc;
   if ((rc = grow(&c->surv, &c->surv_cap, 1LL << 20))) return rc;
   memset(s->jp, 0, sizeof s->jp);
-  s->P = make_params(c, tu, 16, nwarps, dump_room);
+  s->P = make_params(c, tu, 16, nwarps, dump_room, s->cap);
   s->smem = search_smem(tu.block);
-  CK(cudaFuncSetAttribute(search_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s->smem));
+  CK(set_persistent_smem(s->smem));
   memset(c->ctl_host, 0, sizeof(Ctl));
   CK(h2d(c, c->ctl, c->ctl_host, sizeof(Ctl)));
   CK(cudaMemsetAsync(c->pool_ready, 0, sizeof(int) * (size_t)c->pool_ready_cap, c->stream));
+  CK(cudaMemsetAsync(c->long_items, 0, sizeof(unsigned long long) * (size_t)c->long_items_cap, c->stream));
   CK(cudaMemsetAsync(c->d_jobcnt, 0, sizeof(unsigned long long) * kMaxJobs * kJobCounters, c->stream));
   CK(h2d(c, c->d_jobs, s->jp, sizeof s->jp));
   CK(cudaMalloc(&s->alt, sizeof(Node) * (size_t)c->stack_cap));
@@ -2136,8 +2637,9 @@ extern "C" int e13_serve_step(e13_serve *s, e13_serve_result *done, int cap, int
   }
   if (running == 0) return E13_OK;
   // 2. one epoch of the persistent kernel, then the live nodes of every job
-  launches += 4;
+  launches += 5;
   search_kernel<true><<<c->nsm, s->tu.block, s->smem, c->stream>>>(s->P);
+  long_kernel<<<c->nsm * kLongPerSm, kLongBlock, long_smem(), c->stream>>>(s->P);
   move_outputs<<<c->nsm * 4, 256, 0, c->stream>>>(c->ctl, c->stack, c->out, c->pool, c->pool_cap, s->cap);
   finish_launch<<<1, 1, 0, c->stream>>>(c->ctl, s->cap, s->batch_max, c->pool_cap);
   CK(cudaMemsetAsync(c->d_jobnodes, 0, sizeof(unsigned long long) * kMaxJobs, c->stream));

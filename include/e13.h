@@ -98,11 +98,12 @@ typedef struct e13_tuning {
   int32_t epoch_us;          /* persistent: wall-clock bound of one epoch, microseconds */
   int32_t epochs_per_graph;  /* persistent: epochs captured in one CUDA graph */
   int32_t pool_low_pct;      /* persistent: warps donate stack nodes while the pool holds fewer than this % of warps */
-  int32_t run_skip;          /* advance whole tape words across runs of a self-loop (exact in every form):
-                                0 never, 1 always, N >= 2 in the slices of warps where some running
-                                machine has made N steps or more (younger machines' runs are short;
-                                persistent kernel only: the plain kernel takes N >= 2 as 1, since
-                                each of its launches waits for its oldest machine) */
+  int32_t run_skip;          /* old machines advance by more than a step at a time (exact in every form):
+                                0 never, 1 as early as possible, N >= 2: the persistent kernel hands a
+                                machine over to the long-machine kernel once it has run 2 N steps since it
+                                was loaded (sooner while warps wait for work).  The plain kernel crosses runs
+                                of a self-loop a tape word at a time for every N >= 1, since each of its
+                                launches waits for its oldest machine */
   int64_t stack_nodes;       /* frontier stack capacity in nodes (0 = auto) */
 } e13_tuning;
 

@@ -10,11 +10,9 @@
 //   E13_CHECK_DEEP     deep.c: limit t + 64*4^n + 1e5, tape -4096 .. 2^nmax+4096,
 //                      off tape below -4094 or past 2^n + 2000 (src/deep.c:56-64)
 //
-// One machine per lane.  The tape is bit-packed; cells -4096 .. 2^nmax + 4096
-// (all of deep's tape, the busy part of recheck's) sit in a shared-memory
-// window interleaved by lane, the rest of recheck's +-4M cells in HBM.  The
-// word under the head stays in a register; runs of a self-loop are crossed a
-// word at a time.
+// One machine per warp (e13_walk.cuh), one warp per CTA.  The tape is
+// bit-packed; cells -4096 .. 2^nmax + 4096 (all of deep's tape, the busy part
+// of recheck's) sit in shared memory, the rest of recheck's +-4M cells in HBM.
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -25,15 +23,16 @@
 #include <vector>
 
 #include "e13.h"
+#include "e13_walk.cuh"
+
+using namespace e13dev;
 
 namespace {
 
 typedef unsigned int u32;
 typedef long long i64;
 
-constexpr i64 kWinLeft = 4096;        // the shared-memory window starts at cell -4096
 constexpr i64 kRecheckSide = 4000000;  // recheck's tape: cells -4e6 .. 4e6 (src/recheck.c:16-17)
-constexpr int kSmemBudget = 200 * 1024;
 
 struct CheckParams {
   int n, nmax, deep;
@@ -47,222 +46,121 @@ struct CheckParams {
 
 __device__ __forceinline__ int first_of_class(int n) { return n <= 2 ? 1 : (n <= 8 ? 3 : 9); }
 
-// A lane's tape: a window of W words in shared memory (interleaved by lane,
-// so a warp never has bank conflicts), the rest in HBM (recheck only).
-struct Tape {
-  u32 *win;
-  int nl, W;
-  u32 *g;
-  i64 gshift;
-  __device__ __forceinline__ bool in_win(i64 ww) const { return ww >= 0 && ww < W; }
-  __device__ __forceinline__ u32 ld(i64 ww) const { return in_win(ww) ? win[ww * nl] : g[ww + gshift]; }
-  __device__ __forceinline__ void st(i64 ww, u32 v) const {
-    if (in_win(ww)) win[ww * nl] = v;
-    else g[ww + gshift] = v;
-  }
-};
+// Shared memory of one machine: the remembered visits, the table, the window.
+size_t check_smem(int W) { return sizeof(uint4) * kMemoSize + sizeof(uint2) * 16 + sizeof(u32) * (size_t)W; }
+
+// Words of the window for stage nmax: cells -4096 .. 2^nmax + 4096.
+int window_words(int nmax) { return (int)((kWalkLeft + (1LL << nmax) + 4096 + 31) / 32 + 2); }
+
+// Cell entry of a machine: bit 0 write, bit 1 right, bits 2..5 next, bit 7 not
+// a move.
+__device__ u32 check_code(const e13_check_in &in, int s, int a) {
+  const int i = 2 * s + a;
+  if (s >= in.nq || in.kind[i] != 0) return 0x80u;
+  return (u32)(in.write[i] & 1) | (in.move[i] > 0 ? 2u : 0u) | ((u32)(in.next[i] & 15) << 2);
+}
 
 __global__ void __launch_bounds__(32) check_kernel(const CheckParams P) {
-  extern __shared__ __align__(16) u32 s_win[];
-  __shared__ unsigned short s_rows[16 * 32];
-  const int nl = blockDim.x;
-  const int m = blockIdx.x * nl + threadIdx.x;
-  Tape tp;
-  tp.win = s_win + threadIdx.x;
-  tp.nl = nl;
-  tp.W = P.W;
-  tp.g = P.deep ? nullptr : P.gtapes + (i64)(m < P.n ? m : 0) * P.gwords;
-  tp.gshift = P.gshift;
-  if (m >= P.n) return;
-  for (int w = 0; w < P.W; ++w) tp.win[w * nl] = 0;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  uint4 *memo = reinterpret_cast<uint4 *>(smem_raw);
+  uint2 *act = reinterpret_cast<uint2 *>(memo + kMemoSize);
+  const int m = blockIdx.x, lane = threadIdx.x;
+  WalkTape T;
+  T.win = reinterpret_cast<u32 *>(act + 16);
+  T.W = P.W;
+  T.g = P.deep ? nullptr : P.gtapes + (i64)m * P.gwords;
+  T.gshift = P.gshift;
   const e13_check_in &in = P.in[m];
   e13_check_out &o = P.out[m];
-  unsigned short *rows = s_rows + threadIdx.x;  // row s at rows[s * 32]: two 8-bit cells
-  // cell entry: bit 0 write, bit 1 right, bits 2..5 next, bit 6 self-loop, bit 7 not a move
-  for (int s = 0; s < 16; ++s) {
-    unsigned short r = 0;
-    for (int a = 0; a < 2; ++a) {
-      const int i = 2 * s + a;
-      unsigned e = 0x80u;
-      if (s < in.nq && in.kind[i] == 0) {
-        e = (unsigned)(in.write[i] & 1) | (in.move[i] > 0 ? 2u : 0u) | ((unsigned)(in.next[i] & 15) << 2);
-        if (in.next[i] == s && in.write[i] == a) e |= 0x40u;  // reads a, writes a, stays: sweeps a run of a
-      }
-      r |= (unsigned short)(e << (8 * a));
-    }
-    rows[s * 32] = r;
-  }
+  for (int i = lane; i < kMemoSize; i += 32) memo[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (int w = lane; w < P.W; w += 32) T.win[w] = 0;
+  reinterpret_cast<u32 *>(act)[lane] = act_word(check_code(in, lane >> 1, lane & 1), (u32)lane & 1u);
+  __syncwarp();
   const bool deep = P.deep != 0;
-
-  o.status = E13_CHK_OK;
-  o.fail_stage = 0;
-  o.stages_done = 0;
-  o.fail_t = 0;
-  o.fail_head = 0;
-  i64 head = 0, t = 0, minhead = 0, ones = 0;
-  int st = 0;
-  i64 ww = kWinLeft >> 5;  // word of cell 0
-  int bit = 0;
-  u32 word = tp.ld(ww);
-  const int st0 = in.st0;
-  const i64 head0 = in.head0;
-  const int rel = in.rel;
-
+  const i64 side = deep ? 0 : kRecheckSide;
+  if (lane == 0) {
+    o.status = E13_CHK_OK;
+    o.fail_stage = 0;
+    o.stages_done = 0;
+    o.fail_t = 0;
+    o.fail_head = 0;
+  }
+  Walker M{0, 0, 0, 0, 0};
+  i64 t = 0;
   for (int n = 1; n <= P.nmax; ++n) {
-    const i64 blk = 1LL << n;
+    const int blk = 1 << n;
     const i64 limit = t + (deep ? 64LL : 8LL) * (1LL << (2 * n)) + 100000;
-    const i64 want = rel ? head0 + blk - 2 : head0;
-    int fail = 0;
-    for (;;) {
-      if (st == st0 && head == want && ones == blk) {
-        // all of -1 .. blk-2 set?  (the cached word goes back first)
-        tp.st(ww, word);
-        bool ok = true;
-        for (i64 c = -1; c < blk - 1 && ok;) {
-          const i64 b = c + kWinLeft;
-          const int sh = (int)(b & 31);
-          const int take = (int)min((i64)(32 - sh), blk - 1 - c);
-          const u32 mask = take == 32 ? 0xFFFFFFFFu : (((1u << take) - 1u) << sh);
-          if ((tp.ld(b >> 5) & mask) != mask) ok = false;
-          c += take;
+    const i64 at = in.rel ? in.head0 + blk - 2 : in.head0;
+    // a head position that no allowed tape has stands for every one out of reach
+    const int want = at > (1 << 29) || at < -(1 << 29) ? 1 << 29 : (int)at;
+    const WalkStop S{blk, in.st0, want, want, false};
+    M.left = limit - t;
+    int sym = 0;
+    const int ev = walk_run<false>(T, memo, act, lane, M, S, deep ? -4096 + 2 : (int)(-side + 3),
+                                   deep ? blk + 2000 : (int)(side - 3), &sym);
+    t = limit - M.left;
+    if (ev != kWalkStop) {
+      if (lane == 0) {
+        int fail = ev == kWalkLimit ? E13_CHK_LIMIT : E13_CHK_OFFTAPE;
+        if (ev == kWalkCell) {
+          fail = in.kind[2 * M.st + sym] == 2 ? E13_CHK_FREE_READ : E13_CHK_HALT;
+          o.free_state = M.st;
+          o.free_sym = sym;
         }
-        if (ok) break;
+        o.status = fail;
+        o.fail_stage = n;
+        o.fail_t = t;
+        o.fail_head = M.head;
       }
-      if (t >= limit) { fail = E13_CHK_LIMIT; break; }
-      if (deep ? (head < -4096 + 2 || head > blk + 2000) : (head <= -kRecheckSide + 2 || head >= kRecheckSide - 2)) {
-        fail = E13_CHK_OFFTAPE;
-        break;
-      }
-      const u32 s = (word >> bit) & 1u;
-      const unsigned e = (rows[st * 32] >> (8 * s)) & 0xFFu;
-      if (e & 0x80u) {
-        const int i = 2 * st + (int)s;
-        fail = in.kind[i] == 2 ? E13_CHK_FREE_READ : E13_CHK_HALT;
-        o.free_state = st;
-        o.free_sym = (int)s;
-        break;
-      }
-      const bool right = (e & 2u) != 0;
-      if (e & 0x40u) {
-        // Run skip: the next k steps read s, write nothing, keep the state and
-        // the ones count.  k stops before the step limit, before the tape ends,
-        // at the window edge, and at `want` when a stage start could happen
-        // there, so every test the single-step loop makes is still made.
-        i64 lim = limit - t;
-        if (deep) lim = min(lim, right ? blk + 2001 - head : head + 4095);
-        else lim = min(lim, right ? kRecheckSide - 2 - head : head + kRecheckSide - 2);
-        if (st == st0 && ones == blk) {
-          const i64 dd = right ? want - head : head - want;
-          if (dd > 0) lim = min(lim, dd);
-        }
-        if (lim > 1 && tp.in_win(ww)) {
-          const u32 flip = s ? 0xFFFFFFFFu : 0u;
-          i64 k = 0;
-          i64 w = ww;
-          if (right) {
-            u32 x = (word ^ flip) >> bit;
-            int b0 = bit;
-            for (;;) {
-              k += x ? (__ffs(x) - 1) : (32 - b0);
-              if (x || k >= lim || !tp.in_win(w + 1)) break;
-              ++w;
-              b0 = 0;
-              x = tp.ld(w) ^ flip;
-            }
-          } else {
-            u32 x = (word ^ flip) << (31 - bit);
-            int b0 = bit;
-            for (;;) {
-              k += x ? __clz(x) : (b0 + 1);
-              if (x || k >= lim || !tp.in_win(w - 1)) break;
-              --w;
-              b0 = 31;
-              x = tp.ld(w) ^ flip;
-            }
-          }
-          if (k > lim) k = lim;
-          if (k > 1) {
-            const i64 pos = (i64)bit + (right ? k : -k);
-            head += right ? k : -k;
-            t += k;
-            if (pos < 0 || pos > 31) {
-              tp.st(ww, word);
-              ww += pos >> 5;  // arithmetic shift: floor division by 32
-              word = tp.ld(ww);
-            }
-            bit = (int)(pos & 31);
-            if (head < minhead) minhead = head;
-            continue;
-          }
-        }
-      }
-      const u32 wr = e & 1u;
-      if (wr != s) {
-        word ^= 1u << bit;
-        if (head >= -2) ones += wr ? 1 : -1;
-      }
-      if (right) {
-        ++head;
-        if (++bit == 32) {
-          tp.st(ww, word);
-          word = tp.ld(++ww);
-          bit = 0;
-        }
-      } else {
-        --head;
-        if (--bit < 0) {
-          tp.st(ww, word);
-          word = tp.ld(--ww);
-          bit = 31;
-        }
-        if (head < minhead) minhead = head;
-      }
-      st = (int)((e >> 2) & 15u);
-      ++t;
-    }
-    if (fail) {
-      o.status = fail;
-      o.fail_stage = n;
-      o.fail_t = t;
-      o.fail_head = head;
       return;
     }
-    // stage start n: record the counter (all ones at cells <= -3)
-    tp.st(ww, word);
-    o.stages_done = n;
-    if (n <= E13_CHECK_MAX_NMAX) {
-      o.stage_t[n] = t;
-      o.minhead[n] = minhead;
-      int cnt = 0;
-      i64 leftmost = 0;
-      const i64 lowest = deep ? -4096 + 1 : minhead - 1;
-      for (i64 c = -3; c >= lowest;) {
-        const i64 b = c + kWinLeft;
-        const int sh = (int)(b & 31);
-        // bits sh down to 0 of this word hold cells c .. c - sh
-        u32 x = tp.ld(b >> 5) & (sh == 31 ? 0xFFFFFFFFu : ((2u << sh) - 1u));
-        const i64 wlow = c - sh;  // cell of bit 0
-        while (x) {
-          const int hb = 31 - __clz(x);
-          const i64 cell = wlow + hb;
-          if (cell < lowest) break;
-          if (cnt < E13_CHECK_MAX_ONES) o.ones_cells[n][cnt] = (int)cell;
-          ++cnt;
-          leftmost = cell;
-          x &= ~(1u << hb);
-        }
-        c = wlow - 1;
+    // stage start n: record the counter (all ones at cells <= -3, from -3
+    // down), a lane per word
+    int cnt = 0, leftmost = 0;
+    const int lowest = deep ? -4096 + 1 : M.minhead - 1;
+    for (int top = kWalkZero - 1; top >= walk_word(lowest); top -= 32) {
+      const int w = top - lane;
+      u32 x = w >= walk_word(lowest) ? T.ld(w) : 0u;
+      if (w == kWalkZero - 1) x &= ~kBlockBits;
+      const int first = 32 * w - kWalkLeft;
+      if (first < lowest) x &= 0xFFFFFFFFu << (lowest - first > 31 ? 31 : lowest - first);
+      int before = __popc(x);
+      const int own = before;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int v = __shfl_up_sync(kAll, before, d);
+        if (lane >= d) before += v;
       }
+      const int all = __shfl_sync(kAll, before, 31);
+      int k = cnt + before - own;
+      for (u32 y = x; y; ++k) {
+        const int hb = 31 - __clz(y);
+        y &= ~(1u << hb);
+        if (k < E13_CHECK_MAX_ONES) o.ones_cells[n][k] = first + hb;
+      }
+      const u32 has = __ballot_sync(kAll, x != 0);
+      if (has) {
+        const int last = 31 - __clz(has);
+        leftmost = __shfl_sync(kAll, x ? first + __ffs(x) - 1 : 0, last);
+      }
+      cnt += all;
+    }
+    __syncwarp();
+    if (lane == 0) {
+      o.stages_done = n;
+      o.stage_t[n] = t;
+      o.minhead[n] = M.minhead;
       o.nones[n] = cnt;
       o.leftmost[n] = leftmost;
-      if (!deep) {
-        const int f = first_of_class(n);
-        if (n != f) {
-          bool same = o.nones[n] == o.nones[f];
-          const int k = min(cnt, E13_CHECK_MAX_ONES);
-          for (int j = 0; j < k && same; ++j) same = o.ones_cells[n][j] == o.ones_cells[f][j];
-          if (!same) return;  // recheck stops at the first counter change
-        }
+    }
+    if (!deep) {
+      const int f = first_of_class(n);
+      __syncwarp();
+      if (n != f) {
+        bool same = cnt == o.nones[f];
+        const int k = min(cnt, E13_CHECK_MAX_ONES);
+        for (int j = lane; j < k && same; j += 32) same = o.ones_cells[n][j] == o.ones_cells[f][j];
+        if (!__all_sync(kAll, same)) return;  // recheck stops at the first counter change
       }
     }
   }
@@ -280,11 +178,8 @@ extern "C" int e13_check(e13_ctx *ctx, const e13_check_in *in, int n, int nmax, 
   if (n == 0) return E13_OK;
   if (cudaSetDevice(e13_ctx_device(ctx)) != cudaSuccess) return E13_ERR_CUDA;
   const bool deep = mode == E13_CHECK_DEEP;
-  // window: cells -4096 .. 2^nmax + 4096 (deep's whole tape; recheck's busy part)
-  const int W = (int)((kWinLeft + (1LL << nmax) + 4096 + 31) / 32 + 2);
-  int nl = (int)std::min<i64>(32, kSmemBudget / ((i64)W * 4));
-  if (nl < 1) return E13_ERR_ARG;
-  const size_t smem = (size_t)W * nl * 4;
+  const int W = window_words(nmax);
+  const size_t smem = check_smem(W);
   const i64 gwords = deep ? 0 : (2 * kRecheckSide + 1 + 31) / 32 + 2;
   const int chunk = deep ? n : (int)std::min<i64>(n, std::max<i64>(1, (4LL << 30) / (gwords * 4)));
   u32 *d_tapes = nullptr;
@@ -306,7 +201,7 @@ extern "C" int e13_check(e13_ctx *ctx, const e13_check_in *in, int n, int nmax, 
     P.deep = deep ? 1 : 0;
     P.W = W;
     P.gwords = gwords;
-    P.gshift = (kRecheckSide - kWinLeft) / 32;
+    P.gshift = (kRecheckSide - kWalkLeft) / 32;
     P.gtapes = d_tapes;
     P.in = d_in;
     P.out = d_out;
@@ -316,7 +211,7 @@ extern "C" int e13_check(e13_ctx *ctx, const e13_check_in *in, int n, int nmax, 
       rc = E13_ERR_CUDA;
       break;
     }
-    check_kernel<<<(k + nl - 1) / nl, nl, smem>>>(P);
+    check_kernel<<<k, 32, smem>>>(P);
     if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess ||
         cudaMemcpy(out + b, d_out, sizeof(e13_check_out) * (size_t)k, cudaMemcpyDeviceToHost) != cudaSuccess) {
       rc = E13_ERR_CUDA;
@@ -392,10 +287,8 @@ extern "C" int e13_check_noalloc(int device, const e13_check_in *in, int n, int 
   if (rc) return rc;
   const cudaStream_t st = a->stream;
   const bool deep = mode == E13_CHECK_DEEP;
-  const int W = (int)((kWinLeft + (1LL << nmax) + 4096 + 31) / 32 + 2);
-  const int nl = (int)std::min<i64>(32, kSmemBudget / ((i64)W * 4));
-  if (nl < 1) return E13_ERR_NOALLOC_SIZE;
-  const size_t smem = (size_t)W * nl * 4;
+  const int W = window_words(nmax);
+  const size_t smem = check_smem(W);
   if (cudaFuncSetAttribute(check_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return E13_ERR_CUDA;
   // the arrays keep the previous call's contents: clear the tapes and outputs
@@ -409,11 +302,11 @@ extern "C" int e13_check_noalloc(int device, const e13_check_in *in, int n, int 
   P.deep = deep ? 1 : 0;
   P.W = W;
   P.gwords = deep ? 0 : kNoAllocWords;
-  P.gshift = (kRecheckSide - kWinLeft) / 32;
+  P.gshift = (kRecheckSide - kWalkLeft) / 32;
   P.gtapes = a->tapes;
   P.in = a->in;
   P.out = a->out;
-  check_kernel<<<(n + nl - 1) / nl, nl, smem, st>>>(P);
+  check_kernel<<<n, 32, smem, st>>>(P);
   if (cudaGetLastError() != cudaSuccess ||
       cudaMemcpyAsync(out, a->out, sizeof(e13_check_out) * (size_t)n, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
       cudaStreamSynchronize(st) != cudaSuccess)

@@ -15,14 +15,14 @@
 //      reach the start with block 2m and the counter of c or c + 1, within
 //      40 m^2 + 5000 steps.
 //
-// Device work: one lane per stage walk (about 3.3e6 steps for erdos_14), one
-// lane per crafted run (at most 117 per placement).  Each lane's tape is a bit
-// array in HBM with the word under the head kept in a register.  check.py's
-// tape is unbounded; here it is cells -2^22 .. 2^22 for the walk and -2^18 ..
-// 2^18 for a crafted run (|head - start| <= 69,000 there).  A head that leaves
-// it ends the run as "off tape", which check.py cannot print; the verdict line
-// then says so.  The host applies check.py's rules to the recorded starts and
-// run outcomes and prints its text.
+// Device work: one warp per stage walk (about 3.3e6 steps for erdos_14), one
+// warp per crafted run (at most 117 per placement), a tape word at a time
+// (e13_walk.cuh).  Cells -4096 .. 8191 of a tape are in shared memory, the
+// rest in HBM.  check.py's tape is unbounded; here it is cells -2^22 .. 2^22
+// for the walk and -2^18 .. 2^18 for a crafted run (|head - start| <= 69,000
+// there).  A head that leaves it ends the run as "off tape", which check.py
+// cannot print; the verdict line then says so.  The host applies check.py's
+// rules to the recorded starts and run outcomes and prints its text.
 #include <cuda_runtime.h>
 #include <stdio.h>
 #include <string.h>
@@ -33,6 +33,9 @@
 #include <vector>
 
 #include "e13.h"
+#include "e13_walk.cuh"
+
+using namespace e13dev;
 
 namespace {
 
@@ -42,7 +45,7 @@ typedef long long i64;
 constexpr int kNmax = 11;   // src/check.py:20
 constexpr int kMmax = 40;   // src/check.py:21
 constexpr int kCells = E13_CRAFTED_MAX_CELLS;  // counter cells recorded per start
-constexpr int kBlock = 64;
+constexpr int kWindow = (kWalkLeft + 8192) / 32;  // tape words in shared memory
 constexpr i64 kWalkSide = 1LL << 22;   // stage walk: cells -2^22 .. 2^22 - 1
 constexpr i64 kRunSide = 1LL << 18;    // crafted run: cells -2^18 .. 2^18 - 1
 constexpr int kWalkBatch = 2048;       // walks per launch (1 MiB of tape each)
@@ -81,107 +84,26 @@ struct RunOut {
   int32_t cnt[kCells];
 };
 
-struct Stop {
-  i64 size, h0, hh;
-  int s0;
-  int stage_one, crafted;
+// One warp's shared memory.
+struct WarpMem {
+  uint4 memo[kMemoSize];
+  uint2 act[16];
+  u32 win[kWindow];
 };
 
-// cells -1 .. size - 2 all ones?  (the rest of the stop test is in run())
-__device__ bool block_ok(const u32 *tape, i64 side, i64 size) {
-  const i64 a = side - 1, b = side + size - 2;
-  for (i64 w = a >> 5; w <= (b >> 5); ++w) {
-    u32 mask = ~0u;
-    if (w == (a >> 5)) mask &= ~0u << (a & 31);
-    if (w == (b >> 5)) mask &= ~0u >> (31 - (b & 31));
-    if ((tape[w] & mask) != mask) return false;
-  }
-  return true;
-}
-
-struct Machine {
-  i64 head, ones_ge, minhead;
-  int st;
-};
-
-// run_tracked (src/check.py:55-77): before each of at most `limit` steps,
-// the stop test; then a halt cell ends the run, else write, move, next state.
-__device__ int run(const u32 *rows, int stride, u32 *tape, i64 side, Machine &M, const Stop &S, i64 limit,
-                   i64 &steps) {
-  const i64 nwords = (2 * side) >> 5;
-  i64 pos = M.head + side;
-  i64 ww = pos >> 5;
-  int bit = (int)(pos & 31);
-  u32 word = tape[ww];
-  int res = kLimit;
-  i64 k = 0;
-  for (;; ++k) {
-    if (k == limit) break;
-    if (M.ones_ge == S.size &&
-        (S.stage_one ||
-         (M.st == S.s0 && (S.crafted ? M.head == S.hh : (M.head == S.h0 || M.head - S.size == S.h0 - 2))))) {
-      tape[ww] = word;
-      if (block_ok(tape, side, S.size)) {
-        res = kStop;
-        break;
-      }
-    }
-    const u32 sym = (word >> bit) & 1u;
-    const u32 e = (rows[M.st * stride] >> (8 * sym)) & 0xFFu;
-    if (e & 0x80u) {
-      res = kHalt;
-      break;
-    }
-    const u32 w = e & 1u;
-    if (w != sym) {
-      word ^= 1u << bit;
-      if (M.head >= -2) M.ones_ge += w ? 1 : -1;
-    }
-    M.st = (int)((e >> 2) & 15u);
-    if (e & 2u) {
-      ++M.head;
-      if (++bit == 32) {
-        tape[ww] = word;
-        bit = 0;
-        if (++ww >= nwords) {
-          res = kOff;
-          ++k;
-          break;
-        }
-        word = tape[ww];
-      }
-    } else {
-      --M.head;
-      if (M.head < M.minhead) M.minhead = M.head;
-      if (--bit < 0) {
-        tape[ww] = word;
-        bit = 31;
-        if (--ww < 0) {
-          res = kOff;
-          ++k;
-          break;
-        }
-        word = tape[ww];
-      }
-    }
-  }
-  if (res != kOff) tape[ww] = word;
-  steps = k;
-  return res;
-}
-
-// the ones at cells minhead .. -3, ascending (check.py:51-52)
-__device__ int counter_cells(const u32 *tape, i64 side, i64 minhead, int32_t *cells, int32_t &overflow) {
+// The ones at cells minhead .. -3, ascending (check.py:51-52), by lane 0.
+__device__ int counter_cells(const WalkTape &T, i64 side, int minhead, int32_t *cells, int32_t &overflow) {
   int n = 0;
-  const i64 a = (minhead > -side ? minhead : -side) + side, b = side - 3;
-  for (i64 w = a >> 5; w <= (b >> 5) && a <= b; ++w) {
-    u32 x = tape[w];
-    if (w == (a >> 5)) x &= ~0u << (a & 31);
-    if (w == (b >> 5)) x &= ~0u >> (31 - (b & 31));
+  const int lo = minhead > -(int)side ? minhead : -(int)side;
+  for (int w = walk_word(lo); w < kWalkZero && lo <= -3; ++w) {
+    const int first = 32 * w - kWalkLeft;
+    u32 x = T.ld(w);
+    if (first < lo) x &= ~0u << (lo - first);
+    if (w == kWalkZero - 1) x &= ~kBlockBits;
     while (x) {
       const int bpos = __ffs(x) - 1;
       x &= x - 1;
-      if (n < kCells) cells[n] = (int32_t)((w << 5) + bpos - side);
+      if (n < kCells) cells[n] = first + bpos;
       else overflow = 1;
       ++n;
     }
@@ -189,80 +111,109 @@ __device__ int counter_cells(const u32 *tape, i64 side, i64 minhead, int32_t *ce
   return n < kCells ? n : kCells;
 }
 
-__device__ void load_rows(u32 *rows, int stride, const unsigned char *code) {
-  for (int s = 0; s < 16; ++s) rows[s * stride] = (u32)code[2 * s] | ((u32)code[2 * s + 1] << 8);
+// A blank tape with its HBM words at `tape`, and the table.
+__device__ WalkTape start(WarpMem &M, u32 *tape, i64 side, const unsigned char *code, int lane) {
+  for (int i = lane; i < kMemoSize; i += 32) M.memo[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (int i = lane; i < kWindow; i += 32) M.win[i] = 0;
+  reinterpret_cast<u32 *>(M.act)[lane] = act_word(code[lane], (u32)lane & 1u);
+  __syncwarp();
+  return WalkTape{M.win, kWindow, tape, (side - kWalkLeft) / 32};
 }
 
-__global__ void __launch_bounds__(kBlock) walk_kernel(const WalkIn *in, int n, u32 *tapes, WalkOut *out) {
-  __shared__ u32 s_rows[16 * kBlock];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  u32 *rows = s_rows + threadIdx.x;
-  load_rows(rows, blockDim.x, in[i].code);
-  u32 *tape = tapes + (i64)i * ((2 * kWalkSide) >> 5);
+__device__ __forceinline__ int result_of(int ev) {
+  return ev == kWalkStop ? kStop : ev == kWalkLimit ? kLimit : ev == kWalkCell ? kHalt : kOff;
+}
+
+__global__ void __launch_bounds__(32) walk_kernel(const WalkIn *in, u32 *tapes, WalkOut *out) {
+  __shared__ WarpMem mem;
+  const int i = blockIdx.x, lane = threadIdx.x;
+  const WalkTape T = start(mem, tapes + (i64)i * ((2 * kWalkSide) >> 5), kWalkSide, in[i].code, lane);
   WalkOut &o = out[i];
-  o.nstarts = 0;
-  o.res = kStop;
-  o.fail_n = 0;
-  o.overflow = 0;
-  o.fail_total = 0;
-  Machine M{0, 0, 0, 0};
+  if (lane == 0) {
+    o.nstarts = 0;
+    o.res = kStop;
+    o.fail_n = 0;
+    o.overflow = 0;
+    o.fail_total = 0;
+  }
+  Walker M{0, 0, 0, 0, 0};
   i64 total = 0;
+  int h0 = 0, s0 = 0;
   for (int k = 1; k <= kNmax; ++k) {
-    Stop S{1LL << k, k > 1 ? o.head[0] : 0, 0, k > 1 ? o.st[0] : 0, k == 1, 0};
-    i64 t = 0;
-    const int res = run(rows, blockDim.x, tape, kWalkSide, M, S, 40LL * (1LL << (2 * k)) + 1000, t);
-    total += t;
+    const WalkStop S{1 << k, s0, h0, h0 - 2 + (1 << k), k == 1};
+    const i64 limit = 40LL * (1LL << (2 * k)) + 1000;
+    M.left = limit;
+    int sym = 0;
+    const int res = result_of(walk_run<true>(T, mem.memo, mem.act, lane, M, S, -(int)kWalkSide, (int)kWalkSide - 1, &sym));
+    total += limit - M.left;
     if (res != kStop) {
-      o.res = res;
-      o.fail_n = k;
-      o.fail_total = total;
+      if (lane == 0) {
+        o.res = res;
+        o.fail_n = k;
+        o.fail_total = total;
+      }
       return;
     }
-    const int j = o.nstarts++;
-    o.st[j] = M.st;
-    o.head[j] = M.head;
-    o.total[j] = total;
-    o.ncnt[j] = counter_cells(tape, kWalkSide, M.minhead, o.cnt[j], o.overflow);
+    if (k == 1) {
+      h0 = M.head;
+      s0 = M.st;
+    }
+    if (lane == 0) {
+      const int j = o.nstarts++;
+      o.st[j] = M.st;
+      o.head[j] = M.head;
+      o.total[j] = total;
+      o.ncnt[j] = counter_cells(T, kWalkSide, M.minhead, o.cnt[j], o.overflow);
+    }
+    __syncwarp();
   }
 }
 
-__global__ void __launch_bounds__(kBlock) run_kernel(const RunIn *in, int n, const WalkIn *tables,
-                                                     const int32_t *cells, u32 *tapes, RunOut *out) {
-  __shared__ u32 s_rows[16 * kBlock];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+__global__ void __launch_bounds__(32) run_kernel(const RunIn *in, const WalkIn *tables, const int32_t *cells,
+                                                 u32 *tapes, RunOut *out) {
+  __shared__ WarpMem mem;
+  const int i = blockIdx.x, lane = threadIdx.x;
   const RunIn &r = in[i];
-  u32 *rows = s_rows + threadIdx.x;
-  load_rows(rows, blockDim.x, tables[r.walk].code);
-  u32 *tape = tapes + (i64)i * ((2 * kRunSide) >> 5);
+  const WalkTape T = start(mem, tapes + (i64)i * ((2 * kRunSide) >> 5), kRunSide, tables[r.walk].code, lane);
   RunOut &o = out[i];
-  o.overflow = 0;
-  o.ncnt = 0;
   // the crafted start (src/check.py:131-135): counter of c, block -1 .. m - 2
-  Machine M{r.absolute ? r.h0 : r.h0 - 2 + r.m, r.m, 0, r.s0};
+  const int h0 = (int)r.h0;
+  Walker M;
+  M.head = r.absolute ? h0 : h0 - 2 + r.m;
+  M.ones = r.m;
   M.minhead = M.head;
+  M.st = r.s0;
+  bool beyond = false;
   for (int k = 0; k < r.ncnt; ++k) {
-    const i64 c = cells[r.cnt_off + k];
-    if (c < -kRunSide) {  // a counter cell beyond this tape: cannot run exactly
-      o.res = kOff;
-      o.t = 0;
-      return;
+    const int c = cells[r.cnt_off + k];
+    if (c < -(int)kRunSide) {  // a counter cell beyond this tape: cannot run exactly
+      beyond = true;
+      break;
     }
-    const i64 pos = c + kRunSide;
-    tape[pos >> 5] |= 1u << (pos & 31);
+    if (lane == 0) T.st(walk_word(c), T.ld(walk_word(c)) | 1u << (c & 31));
     if (c < M.minhead) M.minhead = c;
   }
-  for (i64 c = -1; c < r.m - 1; ++c) {
-    const i64 pos = c + kRunSide;
-    tape[pos >> 5] |= 1u << (pos & 31);
+  for (int c = -1; c < r.m - 1 && lane == 0; ++c) T.st(walk_word(c), T.ld(walk_word(c)) | 1u << (c & 31));
+  __syncwarp();
+  if (lane == 0) {
+    o.overflow = 0;
+    o.ncnt = 0;
+    o.res = kOff;
+    o.t = 0;
   }
-  const i64 nxt = 2LL * r.m;
-  Stop S{nxt, r.h0, r.absolute ? r.h0 : r.h0 - 2 + nxt, r.s0, 0, 1};
-  i64 t = 0;
-  o.res = run(rows, blockDim.x, tape, kRunSide, M, S, 40LL * r.m * r.m + 5000, t);
-  o.t = t;
-  if (o.res == kStop) o.ncnt = counter_cells(tape, kRunSide, M.minhead, o.cnt, o.overflow);
+  if (beyond) return;
+  const int nxt = 2 * r.m;
+  const int want = r.absolute ? h0 : h0 - 2 + nxt;
+  const WalkStop S{nxt, r.s0, want, want, false};
+  const i64 limit = 40LL * r.m * r.m + 5000;
+  M.left = limit;
+  int sym = 0;
+  const int res = result_of(walk_run<true>(T, mem.memo, mem.act, lane, M, S, -(int)kRunSide, (int)kRunSide - 1, &sym));
+  if (lane == 0) {
+    o.res = res;
+    o.t = limit - M.left;
+    if (res == kStop) o.ncnt = counter_cells(T, kRunSide, M.minhead, o.cnt, o.overflow);
+  }
 }
 
 // ---- host
@@ -416,7 +367,7 @@ extern "C" int e13_check_crafted(e13_ctx *ctx, const char *const *lines, int n, 
     for (int b0 = 0; b0 < np; b0 += kWalkBatch) {
       const int nb = std::min(kWalkBatch, np - b0);
       CKC(cudaMemsetAsync(d_tape, 0, (size_t)nb * ((2 * kWalkSide) >> 5) * sizeof(u32), stream));
-      walk_kernel<<<(nb + kBlock - 1) / kBlock, kBlock, 0, stream>>>(d_tables + b0, nb, d_tape, d_walk);
+      walk_kernel<<<nb, 32, 0, stream>>>(d_tables + b0, d_tape, d_walk);
       CKC(cudaGetLastError());
       CKC(cudaMemcpyAsync(walks.data() + b0, d_walk, sizeof(WalkOut) * nb, cudaMemcpyDeviceToHost, stream));
       CKC(cudaStreamSynchronize(stream));
@@ -492,7 +443,7 @@ extern "C" int e13_check_crafted(e13_ctx *ctx, const char *const *lines, int n, 
     for (int b0 = 0; b0 < nr; b0 += kRunBatch) {
       const int nb = std::min(kRunBatch, nr - b0);
       CKC(cudaMemsetAsync(d_tape, 0, (size_t)nb * ((2 * kRunSide) >> 5) * sizeof(u32), stream));
-      run_kernel<<<(nb + kBlock - 1) / kBlock, kBlock, 0, stream>>>(d_runs + b0, nb, d_tables, d_cells, d_tape, d_rout);
+      run_kernel<<<nb, 32, 0, stream>>>(d_runs + b0, d_tables, d_cells, d_tape, d_rout);
       CKC(cudaGetLastError());
       CKC(cudaMemcpyAsync(runouts.data() + b0, d_rout, sizeof(RunOut) * nb, cudaMemcpyDeviceToHost, stream));
       CKC(cudaStreamSynchronize(stream));

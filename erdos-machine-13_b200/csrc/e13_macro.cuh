@@ -31,36 +31,22 @@
 //    runs on to its deadline and dies there (src/e13search.c:161).
 #pragma once
 #include "e13_device.cuh"
+#include "e13_visit.cuh"
 
 namespace e13dev {
 
-constexpr int kMemoBits = 9;
-constexpr int kMemoSize = 1 << kMemoBits;
-constexpr int kMemoMaxSteps = 2048;  // longest remembered visit
 constexpr int kSnapEvery = 32;       // single-stepped visits between configuration snapshots
 constexpr int kLastWord = kTapeWords - 1;
 constexpr int kSpans = 32;           // functionals per word
-constexpr u32 kAll = 0xFFFFFFFFu;
 
-// What one warp needs in shared memory.  memo entry: x content on entry;
-// y bits 0..5 the key (state, side entered from: 16 = right, 32 = valid), bits
-// 6..11 the same for the word entered next, 16..31 steps (0: single-step this
-// visit); z content on exit; w table cells read (bit per cell; bare runs only).
+// What one warp needs in shared memory.
 struct MacroMem {
   uint4 memo[kMemoSize];
   u32 tape[kTapeWords + 1];
-  uint2 act[16];  // the table for macro_visit: what each state does on 0 and on 1
+  uint2 act[16];  // the table for macro_visit
   u32 rows[16];
   u32 pad[4];
 };
-
-// act words: bit 0 flip, bits 3..6 next state, bit 7 not a plain move, bits
-// 24..31 the head's move (64 for anything but a plain move: leaves the word)
-constexpr u32 kActSpecial = 0x80u;
-__device__ __forceinline__ u32 act_word(u32 code, u32 sym) {
-  if (code & kEntSpecial) return 0x40000000u | kActSpecial;
-  return ((code ^ sym) & 1u) | ((code << 1) & 0x78u) | ((code & 2u) ? 0x01000000u : 0xFF000000u);
-}
 
 // The functionals, [functional][word].
 __device__ u64 d_span[kSpans * kTapeWords];
@@ -77,26 +63,6 @@ __device__ __forceinline__ void macro_table(MacroMem &M, int lane) {
   reinterpret_cast<u32 *>(M.act)[lane] = act_word((M.rows[lane >> 1] >> ((lane & 1) << 4)) & 0xFFu, (u32)lane & 1u);
   for (int i = lane; i < kMemoSize; i += 32) M.memo[i] = make_uint4(0u, 0u, 0u, 0u);
   __syncwarp();
-}
-
-// Runs the machine inside one word of content c until it leaves it: the entry
-// to remember.  sk: the key (state and side).
-template <bool READS>
-static __device__ __noinline__ uint4 macro_visit(const uint2 *act, u32 c, u32 sk) {
-  u32 w = c, reads = 0, x = 0;
-  int st = (int)(sk & 15u), q = (sk & 16u) ? 31 : 0, n = 0;
-  do {
-    const uint2 a = act[st];
-    const u32 sym = (w >> q) & 1u;
-    x = sym ? a.y : a.x;
-    if (READS) reads |= 1u << (2 * st + (int)sym);
-    w ^= (x & 1u) << q;
-    q += (int)x >> 24;
-    st = (int)((x >> 3) & 15u);
-    ++n;
-  } while ((unsigned)q <= 31u && n < kMemoMaxSteps);
-  if ((unsigned)q <= 31u || (x & kActSpecial)) return make_uint4(c, sk, c, 0u);
-  return make_uint4(c, sk | ((u32)(st | 32 | (q < 0 ? 16 : 0)) << 6) | ((u32)n << 16), w, reads);
 }
 
 __device__ __forceinline__ u32 span_bit(u64 v, u64 f) {
@@ -139,7 +105,7 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const Ke
       bool ok, in_range, sweep;
       do {
         c = M.tape[b];
-        slot = M.memo + ((c * 0x9E3779B1u + sk * 0x85EBCA6Bu) >> (32 - kMemoBits));
+        slot = M.memo + memo_slot(c, sk);
         e = *slot;
         n = e.y >> 16;
         in_range = (unsigned)(b - 1) < (unsigned)(kLastWord - 1);
@@ -181,7 +147,7 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const Ke
           b += dir * run;
           if (noted < 32) continue;
         } else if (in_range && !known) {
-          const uint4 v = macro_visit<!HASH>(M.act, c, sk);
+          const uint4 v = macro_visit<HASH ? kNoteNothing : kNoteReads>(M.act, c, sk);
           __syncwarp();
           if (lane == 0) *slot = v;
           __syncwarp();

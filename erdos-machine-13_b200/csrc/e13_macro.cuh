@@ -35,6 +35,10 @@
 
 namespace e13dev {
 
+constexpr int kWindowSteps = 4096;   // bare runs: steps of one turn in the window
+constexpr int kYieldEvery = 4;       // ... batches of visits between looks at what they yield
+constexpr int kStepCycles = 80;      // ... cycles a step in the window
+constexpr int kLoopTries = 8;        // recurrences of a batch's first visit looked at
 constexpr int kSnapEvery = 32;       // single-stepped visits between configuration snapshots
 constexpr int kLastWord = kTapeWords - 1;
 constexpr int kSpans = 32;           // functionals per word
@@ -47,9 +51,6 @@ struct MacroMem {
   u32 rows[16];
   u32 pad[4];
 };
-
-// The functionals, [functional][word].
-__device__ u64 d_span[kSpans * kTapeWords];
 
 __device__ __forceinline__ unsigned long long macro_clock() {
   unsigned long long t;
@@ -75,10 +76,10 @@ __device__ __forceinline__ u32 span_bit(u64 v, u64 f) {
 // passes t_end (HASH only).  HASH: the filter, hb being the full 64-bit hash.
 // Otherwise the bare table runs until L.t is past L.deadline (kEvDead), and
 // kEvOff says that a step left the window (L.p is then outside it, that step
-// not counted); reads collects the table cells read.
+// not counted).  READS: reads collects the table cells read.
 enum { kEvOff = 5 };
 
-template <bool HASH>
+template <bool HASH, bool READS = false>
 __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const KeyTabs &K, const u64 *span, int lane,
                                          u32 &reads, int &cell, u32 &ecell, unsigned long long t_end) {
   int p = L.p, b = L.p >> 5;
@@ -96,6 +97,10 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const Ke
   int snap_b = 0, snap_left = 0, snaps = 0;
   u32 snap_at = 0, snap0 = 0, snap1 = 0, snap2 = 0;  // words snap_b - 1 .. snap_b + 1
   bool far = true;                  // left those words, or reached a stage, since the snapshot
+  // bare runs: batches until the next look at what visits yield, steps left and
+  // clock at the last one, steps still to take in the window
+  int visits_left = kYieldEvery, yield_left = left, window_left = 0;
+  long long yield_clock = HASH ? 0 : clock64();
   for (;;) {
     if (!single) {
       // remembered visits, one after another.  Nothing in this loop branches
@@ -116,7 +121,7 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const Ke
         v_sk = mine ? sk : v_sk;
         v_left = mine ? left : v_left;
         v_d = mine ? c ^ e.z : v_d;
-        if (!HASH && ok) reads |= e.w;
+        if (READS && ok) reads |= e.w;
         if (ok) M.tape[b] = e.z;  // every lane writes the same value
         const u32 next = (e.y >> 6) & 63u;
         left = ok ? left - (int)n : left;
@@ -147,7 +152,7 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const Ke
           b += dir * run;
           if (noted < 32) continue;
         } else if (in_range && !known) {
-          const uint4 v = macro_visit<HASH ? kNoteNothing : kNoteReads>(M.act, c, sk);
+          const uint4 v = macro_visit<READS ? kNoteReads : kNoteNothing>(M.act, c, sk);
           __syncwarp();
           if (lane == 0) *slot = v;
           __syncwarp();
@@ -213,23 +218,32 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const Ke
       const u32 sk0 = __shfl_sync(kAll, v_sk, 0);
       if (__any_sync(kAll, lane < noted && (unsigned)(v_b - snap_b + 1) > 2u)) far = true;
       m = __ballot_sync(kAll, lane > 0 && lane < noted && v_b == b0 && v_sk == sk0);
-      if (m) {
+      for (int tries = 0; m && tries < kLoopTries; ++tries, m &= m - 1) {
         const int j = __ffs(m) - 1;
         const bool in = lane < j;
-        const bool out = __any_sync(kAll, in && (unsigned)(v_b - b0 + 1) > 2u);
-        if (!out) {
-          const u32 x0 = __reduce_xor_sync(kAll, (in && v_b == b0 - 1) ? v_d : 0u);
-          const u32 x1 = __reduce_xor_sync(kAll, (in && v_b == b0) ? v_d : 0u);
-          const u32 x2 = __reduce_xor_sync(kAll, (in && v_b == b0 + 1) ? v_d : 0u);
-          if ((x0 | x1 | x2) == 0u) {
-            if (HASH) {
-              L.t = L.deadline + 1;
-              return kEvDead;
-            }
-            const int period = __shfl_sync(kAll, v_left, 0) - __shfl_sync(kAll, v_left, j);
-            left %= period;
+        if (__any_sync(kAll, in && (unsigned)(v_b - b0 + 1) > 2u)) break;
+        const u32 x0 = __reduce_xor_sync(kAll, (in && v_b == b0 - 1) ? v_d : 0u);
+        const u32 x1 = __reduce_xor_sync(kAll, (in && v_b == b0) ? v_d : 0u);
+        const u32 x2 = __reduce_xor_sync(kAll, (in && v_b == b0 + 1) ? v_d : 0u);
+        if ((x0 | x1 | x2) == 0u) {
+          if (HASH) {
+            L.t = L.deadline + 1;
+            return kEvDead;
           }
+          left %= __shfl_sync(kAll, v_left, 0) - __shfl_sync(kAll, v_left, j);
+          break;
         }
+      }
+      if (!HASH && --visits_left <= 0) {
+        // visits that cost more than the steps they take: over to the window
+        const long long now = clock64();
+        if (now - yield_clock > (long long)kStepCycles * (yield_left - left)) {
+          single = true;
+          window_left = kWindowSteps;
+        }
+        yield_left = left;
+        yield_clock = now;
+        visits_left = kYieldEvery;
       }
       noted = 0;
       rep = false;
@@ -242,9 +256,52 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const Ke
     }
     if (!single) continue;
 
-    // single steps until the head is in another word
     int st = (int)(sk & 15u);
     if (!inside) p = b * 32 + ((sk & 16u) ? 31 : 0);
+    if (!HASH && p >= 18 && p <= kTapeCells - 18) {
+      // a bare run: 32 cells around the head, all inside the window the machine
+      // may not leave, step by step
+      const int b0 = (p - 16) >> 5, sh = (p - 16) & 31;
+      const u32 w0 = M.tape[b0], w1 = M.tape[b0 + 1];
+      Window V;
+      V.w = __funnelshift_r(w0, w1, sh);
+      V.q = 16;
+      V.st = st;
+      u32 r = 0;
+      window_run<READS>(M.act, V, left < kWindowSteps ? left : kWindowSteps, r);
+      if (READS) reads |= r;
+      __syncwarp();
+      M.tape[b0] = (w0 & ~(0xFFFFFFFFu << sh)) | (V.w << sh);
+      if (sh) M.tape[b0 + 1] = (w1 & (0xFFFFFFFFu << sh)) | (V.w >> (32 - sh));
+      __syncwarp();
+      left -= V.steps;
+      if (V.loop) left %= V.loop;
+      p += V.q - 16;
+      st = V.st;
+      b = p >> 5;
+      sk = (u32)st | 32u | ((p & 31) ? 16u : 0u);
+      inside = (p & 31) != 0 && (p & 31) != 31;
+      rep = false;
+      yield_left = left;
+      yield_clock = clock64();
+      visits_left = kYieldEvery;
+      window_left -= V.steps;
+      if (V.special || left <= 0) {
+        L.p = p;
+        L.st = st;
+        L.t = L.deadline + 1 - left;
+        __syncwarp();
+        if (!V.special) return kEvDead;
+        const u32 sym = (M.tape[b] >> (p & 31)) & 1u;
+        cell = (st << 1) | (int)sym;
+        ecell = (M.rows[st] >> (sym << 4)) & 0xFFu;
+        return kEvCell;
+      }
+      // inside a word still, or not yet done: on with the window
+      single = inside || window_left > 0;
+      continue;
+    }
+    // single steps until the head is in another word
     // a loop that passes through here every turn: the same configuration
     // again, on words not left since the snapshot?
     if ((unsigned)(b - snap_b + 1) > 2u) far = true;
@@ -287,7 +344,7 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const Ke
         ev = kEvCell;
         break;
       }
-      if (!HASH) reads |= 1u << ((st << 1) | (int)sym);
+      if (READS) reads |= 1u << ((st << 1) | (int)sym);
       if (x & 1u) {
         word ^= 1u << (p & 31);
         if (HASH) hb ^= ((u64)K.hi[p] << 32) | K.lo[p];

@@ -49,6 +49,9 @@ using namespace e13dev;
 namespace {
 
 constexpr unsigned kFull = 0xFFFFFFFFu;
+
+// macro_run's functionals, [functional][word] (upload_span_functionals).
+__device__ u64 d_span[kSpans * kTapeWords];
 constexpr long long kPoolNodes = 1LL << 18;  // donation pool: 256 Ki nodes (80 MiB)
 constexpr long long kWholeFrontier = 1LL << 62;  // persistent batch when e13_tuning::batch is 0
 constexpr long long kPoolWaitNs = 200000000;     // 200 ms: a donor publishes a claimed slot within microseconds
@@ -1047,7 +1050,7 @@ __global__ void __launch_bounds__(kLongBlock) long_kernel(const __grid_constant_
       R.t = 0;
       R.deadline = L.t - 1;
       reads = 0;
-      macro_run<false>(R, hb, M, K, span, lane, reads, cell, ecell, t_end);
+      macro_run<false, true>(R, hb, M, K, span, lane, reads, cell, ecell, t_end);
       if (lane == 0) {
         atomicAdd(cnt, 1ull);
         record_survivor(ctl, P.surv, P.surv_cap, L.st0, L.p0, L.flags, L.t, L.job, nullptr, M.rows, 1, reads);
@@ -1187,8 +1190,42 @@ __global__ void finish_launch(Ctl *ctl, long long cap, long long batch_max, long
   ctl->launches += 1;
 }
 
-// Whole-table runs (src/e13search.c:428-433): one machine per thread.
-__global__ void __launch_bounds__(256) run_full_kernel(const int *tabs, int n, int nq, long long *out) {
+// Whole-table runs (src/e13search.c:428-433).  Most tables die within a few
+// hundred steps: run_full_kernel runs one machine per thread for kFullSteps
+// steps and lists the ones that live longer, which full_long_kernel runs one
+// per warp from the blank tape.  In one kernel the longest machine of each
+// warp held up the other 31, and a loop to the deadline took 80 ms (20,000
+// mutants with 2 changed cells: 26-85 ms, now 5.6 ms: 0.7 ms and 3 ms for the
+// two kernels, the rest copies and allocation).
+constexpr int kFullSteps = 1024;
+
+__device__ u32 full_row(const int *tab, int nq, int s) {
+  u32 e0 = kEntHalt, e1 = kEntHalt;
+  if (s < nq) {
+    e0 = tab[2 * s] < 0 ? kEntHalt : (u32)tab[2 * s];
+    e1 = tab[2 * s + 1] < 0 ? kEntHalt : (u32)tab[2 * s + 1];
+  }
+  return cell_slot(2 * s, e0, true) | (cell_slot(2 * s + 1, e1, true) << 16);
+}
+
+__device__ void full_start(Lane &L) {
+  L.p = kLeft; L.st = 0; L.t = 0; L.deadline = s_deadline[1]; L.hb = 0; L.tgt = (u32)s_tgt[1];
+  L.nt = 1; L.stage = 0; L.st0 = -1; L.p0 = kLeft; L.flags = 3; L.ch0 = L.ch1 = L.ch2 = 0;  // head0 = 0 until stage 1
+}
+
+__device__ void full_result(const Lane &L, int ev, long long *o) {
+  o[0] = ev == kEvSurv;
+  o[1] = L.stage;
+  o[2] = L.st0;
+  o[3] = L.p0 - kLeft;
+  o[4] = L.flags & 1;
+  o[5] = (L.flags >> 1) & 1;
+  o[6] = L.t;
+}
+
+// list: [0] the number of machines listed, [1] taken by full_long_kernel, then
+// their indices.
+__global__ void __launch_bounds__(256) run_full_kernel(const int *tabs, int n, int nq, long long *out, int *list) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const KeyTabs K = key_tables(smem_raw);
   u32 *tape = reinterpret_cast<u32 *>(smem_raw + kKeySmemBytes);
@@ -1203,20 +1240,11 @@ __global__ void __launch_bounds__(256) run_full_kernel(const int *tabs, int n, i
   u32 *rcol = rows + threadIdx.x;
   for (int w = 0; w < kTapeWords; ++w) tcol[w * stride] = 0;
   const int *tab = tabs + (long long)m * E13_MAXCELLS;
-  for (int s = 0; s < 16; ++s) {
-    u32 e0 = kEntHalt, e1 = kEntHalt;
-    if (s < nq) {
-      e0 = tab[2 * s] < 0 ? kEntHalt : (u32)tab[2 * s];
-      e1 = tab[2 * s + 1] < 0 ? kEntHalt : (u32)tab[2 * s + 1];
-    }
-    rcol[s * stride] = cell_slot(2 * s, e0, true) | (cell_slot(2 * s + 1, e1, true) << 16);
-  }
+  for (int s = 0; s < 16; ++s) rcol[s * stride] = full_row(tab, nq, s);
   Lane L;
-  L.p = kLeft; L.st = 0; L.t = 0; L.deadline = s_deadline[1]; L.hb = 0; L.tgt = (u32)s_tgt[1];
-  L.nt = 1; L.stage = 0; L.st0 = -1; L.p0 = kLeft; L.flags = 3; L.ch0 = L.ch1 = L.ch2 = 0;  // head0 = 0 until stage 1
-  int ev;
+  full_start(L);
+  int ev, nn = kFullSteps, cell = 0;
   for (;;) {
-    int nn = 1 << 30, cell = 0;
     ev = step_slice(L.p, L.st, L.t, L.deadline, L.hb, L.tgt, tcol, rcol, K.lo, stride, nn, cell);
     if (ev == kEvStage) {
       ev = stage_check(L, tcol, K, stride);
@@ -1225,14 +1253,41 @@ __global__ void __launch_bounds__(256) run_full_kernel(const int *tabs, int n, i
     if (ev == kEvCell) ev = kEvDead;  // only halts are special here
     break;
   }
-  long long *o = out + 7LL * m;
-  o[0] = ev == kEvSurv;
-  o[1] = L.stage;
-  o[2] = L.st0;
-  o[3] = L.p0 - kLeft;
-  o[4] = L.flags & 1;
-  o[5] = (L.flags >> 1) & 1;
-  o[6] = L.t;
+  if (ev == kEvRun) list[2 + atomicAdd(list, 1)] = m;
+  else full_result(L, ev, out + 7LL * m);
+}
+
+__global__ void __launch_bounds__(kLongBlock) full_long_kernel(const int *tabs, int nq, long long *out, int *list) {
+  const int n = list[0];
+  if (n == 0) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const KeyTabs K = key_tables(smem_raw);
+  u64 *span = reinterpret_cast<u64 *>(smem_raw + kKeySmemBytes);
+  const int lane = threadIdx.x & 31;
+  MacroMem &M = reinterpret_cast<LongMem *>(span + kSpans * kTapeWords)[threadIdx.x >> 5].m;
+  fill_key_tables(K);
+  load_stage_tables();
+  for (int i = threadIdx.x; i < kSpans * kTapeWords; i += blockDim.x) span[i] = d_span[i];
+  __syncthreads();
+  for (;;) {
+    int k = 0;
+    if (lane == 0) k = atomicAdd(list + 1, 1);
+    k = __shfl_sync(kFull, k, 0);
+    if (k >= n) break;
+    const int m = list[2 + k];
+    if (lane < 16) M.rows[lane] = full_row(tabs + (long long)m * E13_MAXCELLS, nq, lane);
+    for (int w = lane; w < kTapeWords; w += 32) M.tape[w] = 0;
+    macro_table(M, lane);
+    Lane L;
+    full_start(L);
+    u64 hb = 0;
+    u32 reads = 0, ecell = 0;
+    int cell = 0;
+    int ev = macro_run<true>(L, hb, M, K, span, lane, reads, cell, ecell, ~0ull);
+    if (ev == kEvCell) ev = kEvDead;
+    if (lane == 0) full_result(L, ev, out + 7LL * m);
+    __syncwarp();
+  }
 }
 
 }  // namespace
@@ -2103,19 +2158,25 @@ extern "C" int e13_run_full(e13_ctx *c, const int32_t *tabs, int n, int nq, int6
   int rc = ensure_consts(c);
   if (rc) return rc;
   int *d_tabs = nullptr;
+  int *d_list = nullptr;
   long long *d_out = nullptr;
   CK(cudaMalloc(&d_tabs, sizeof(int) * E13_MAXCELLS * (size_t)n));
   CK(cudaMalloc(&d_out, sizeof(long long) * 7 * (size_t)n));
+  CK(cudaMalloc(&d_list, sizeof(int) * ((size_t)n + 2)));
+  CK(cudaMemsetAsync(d_list, 0, sizeof(int) * 2, c->stream));
   CK(h2d(c, d_tabs, tabs, sizeof(int) * E13_MAXCELLS * (size_t)n));
   const int bd = 256;
   const size_t smem = kKeySmemBytes + (size_t)(kTapeWords + 16) * bd * 4;
   CK(cudaFuncSetAttribute(run_full_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  run_full_kernel<<<(n + bd - 1) / bd, bd, smem, c->stream>>>(d_tabs, n, nq, d_out);
+  CK(cudaFuncSetAttribute(full_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)long_smem()));
+  run_full_kernel<<<(n + bd - 1) / bd, bd, smem, c->stream>>>(d_tabs, n, nq, d_out, d_list);
+  full_long_kernel<<<c->nsm * kLongPerSm, kLongBlock, long_smem(), c->stream>>>(d_tabs, nq, d_out, d_list);
   CK(cudaGetLastError());
   CK(d2h(c, out, d_out, sizeof(long long) * 7 * (size_t)n));
   CK(cudaStreamSynchronize(c->stream));
   cudaFree(d_tabs);
   cudaFree(d_out);
+  cudaFree(d_list);
   return E13_OK;
 }
 

@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "e13.h"
+#include "e13_scratch.h"
 #include "e13_walk.cuh"
 
 using namespace e13dev;
@@ -170,6 +171,7 @@ __global__ void __launch_bounds__(32) check_kernel(const CheckParams P) {
 
 struct e13_ctx;
 extern "C" int e13_ctx_device(const e13_ctx *c);
+extern "C" cudaStream_t e13_ctx_stream(const e13_ctx *c);
 
 extern "C" int e13_check(e13_ctx *ctx, const e13_check_in *in, int n, int nmax, int mode, e13_check_out *out) {
   if (!ctx || (n > 0 && (!in || !out)) || n < 0 || nmax < 1 || nmax > E13_CHECK_MAX_NMAX ||
@@ -182,15 +184,12 @@ extern "C" int e13_check(e13_ctx *ctx, const e13_check_in *in, int n, int nmax, 
   const size_t smem = check_smem(W);
   const i64 gwords = deep ? 0 : (2 * kRecheckSide + 1 + 31) / 32 + 2;
   const int chunk = deep ? n : (int)std::min<i64>(n, std::max<i64>(1, (4LL << 30) / (gwords * 4)));
-  u32 *d_tapes = nullptr;
-  e13_check_in *d_in = nullptr;
-  e13_check_out *d_out = nullptr;
   int rc = E13_OK;
-  if ((!deep && cudaMalloc(&d_tapes, (size_t)chunk * gwords * 4) != cudaSuccess) ||
-      cudaMalloc(&d_in, sizeof(e13_check_in) * (size_t)chunk) != cudaSuccess ||
-      cudaMalloc(&d_out, sizeof(e13_check_out) * (size_t)chunk) != cudaSuccess) {
-    rc = E13_ERR_CUDA;
-  }
+  const cudaStream_t st = e13_ctx_stream(ctx);
+  u32 *d_tapes = deep ? nullptr : (u32 *)e13_ctx_scratch(ctx, kScratchCheckTapes, (size_t)chunk * gwords * 4);
+  e13_check_in *d_in = (e13_check_in *)e13_ctx_scratch(ctx, kScratchCheckIn, sizeof(e13_check_in) * (size_t)chunk);
+  e13_check_out *d_out = (e13_check_out *)e13_ctx_scratch(ctx, kScratchCheckOut, sizeof(e13_check_out) * (size_t)chunk);
+  if ((!deep && !d_tapes) || !d_in || !d_out) rc = E13_ERR_CUDA;
   if (!rc && cudaFuncSetAttribute(check_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     rc = E13_ERR_CUDA;
   for (int b = 0; b < n && rc == E13_OK; b += chunk) {
@@ -205,22 +204,21 @@ extern "C" int e13_check(e13_ctx *ctx, const e13_check_in *in, int n, int nmax, 
     P.gtapes = d_tapes;
     P.in = d_in;
     P.out = d_out;
-    if ((!deep && cudaMemset(d_tapes, 0, (size_t)k * gwords * 4) != cudaSuccess) ||
-        cudaMemset(d_out, 0, sizeof(e13_check_out) * (size_t)k) != cudaSuccess ||
-        cudaMemcpy(d_in, in + b, sizeof(e13_check_in) * (size_t)k, cudaMemcpyHostToDevice) != cudaSuccess) {
+    if ((!deep && cudaMemsetAsync(d_tapes, 0, (size_t)k * gwords * 4, st) != cudaSuccess) ||
+        cudaMemsetAsync(d_out, 0, sizeof(e13_check_out) * (size_t)k, st) != cudaSuccess ||
+        cudaMemcpyAsync(d_in, in + b, sizeof(e13_check_in) * (size_t)k, cudaMemcpyHostToDevice, st) != cudaSuccess) {
       rc = E13_ERR_CUDA;
       break;
     }
-    check_kernel<<<k, 32, smem>>>(P);
-    if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess ||
-        cudaMemcpy(out + b, d_out, sizeof(e13_check_out) * (size_t)k, cudaMemcpyDeviceToHost) != cudaSuccess) {
+    check_kernel<<<k, 32, smem, st>>>(P);
+    if (cudaGetLastError() != cudaSuccess ||
+        cudaMemcpyAsync(out + b, d_out, sizeof(e13_check_out) * (size_t)k, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess) {
       rc = E13_ERR_CUDA;
       break;
     }
   }
-  cudaFree(d_tapes);
-  cudaFree(d_in);
-  cudaFree(d_out);
+  e13_ctx_scratch_done(ctx);
   return rc;
 }
 

@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "e13.h"
+#include "e13_scratch.h"
 #include "e13_walk.cuh"
 
 using namespace e13dev;
@@ -312,6 +313,16 @@ extern "C" cudaStream_t e13_ctx_stream(const e13_ctx *c);
     }                                           \
   } while (0)
 
+// A scratch buffer of the context, or the call's end.
+#define SCRATCH(p, slot, bytes)                                             \
+  do {                                                                      \
+    (p) = (decltype(p))e13_ctx_scratch(ctx, (slot), (bytes));               \
+    if (!(p)) {                                                             \
+      rc = E13_ERR_CUDA;                                                    \
+      goto done;                                                            \
+    }                                                                       \
+  } while (0)
+
 extern "C" int e13_check_crafted(e13_ctx *ctx, const char *const *lines, int n, char *out, size_t out_len,
                                  size_t *needed) {
   if (!ctx || (n > 0 && !lines) || n < 0 || (out_len > 0 && !out)) return E13_ERR_ARG;
@@ -359,11 +370,11 @@ extern "C" int e13_check_crafted(e13_ctx *ctx, const char *const *lines, int n, 
   std::string text;
 
   if (np > 0) {
-    CKC(cudaMalloc(&d_tables, sizeof(WalkIn) * np));
+    SCRATCH(d_tables, kScratchCraftTables, sizeof(WalkIn) * np);
     CKC(cudaMemcpyAsync(d_tables, tables.data(), sizeof(WalkIn) * np, cudaMemcpyHostToDevice, stream));
     const int wb = std::min(np, kWalkBatch);
-    CKC(cudaMalloc(&d_walk, sizeof(WalkOut) * wb));
-    CKC(cudaMalloc(&d_tape, (size_t)wb * ((2 * kWalkSide) >> 5) * sizeof(u32)));
+    SCRATCH(d_walk, kScratchCraftWalks, sizeof(WalkOut) * wb);
+    SCRATCH(d_tape, kScratchCraftTapes, (size_t)wb * ((2 * kWalkSide) >> 5) * sizeof(u32));
     for (int b0 = 0; b0 < np; b0 += kWalkBatch) {
       const int nb = std::min(kWalkBatch, np - b0);
       CKC(cudaMemsetAsync(d_tape, 0, (size_t)nb * ((2 * kWalkSide) >> 5) * sizeof(u32), stream));
@@ -372,8 +383,6 @@ extern "C" int e13_check_crafted(e13_ctx *ctx, const char *const *lines, int n, 
       CKC(cudaMemcpyAsync(walks.data() + b0, d_walk, sizeof(WalkOut) * nb, cudaMemcpyDeviceToHost, stream));
       CKC(cudaStreamSynchronize(stream));
     }
-    cudaFree(d_tape);
-    d_tape = nullptr;
   }
 
   // stages and counter classes (src/check.py:112-126), then the crafted runs
@@ -433,10 +442,10 @@ extern "C" int e13_check_crafted(e13_ctx *ctx, const char *const *lines, int n, 
     const int nr = (int)runs.size();
     runouts.resize(nr);
     const int rb = std::min(nr, kRunBatch);
-    CKC(cudaMalloc(&d_runs, sizeof(RunIn) * nr));
-    CKC(cudaMalloc(&d_cells, sizeof(int32_t) * std::max<size_t>(cells.size(), 1)));
-    CKC(cudaMalloc(&d_rout, sizeof(RunOut) * rb));
-    CKC(cudaMalloc(&d_tape, (size_t)rb * ((2 * kRunSide) >> 5) * sizeof(u32)));
+    SCRATCH(d_runs, kScratchCraftRuns, sizeof(RunIn) * nr);
+    SCRATCH(d_cells, kScratchCraftCells, sizeof(int32_t) * std::max<size_t>(cells.size(), 1));
+    SCRATCH(d_rout, kScratchCraftRunOuts, sizeof(RunOut) * rb);
+    SCRATCH(d_tape, kScratchCraftTapes, (size_t)rb * ((2 * kRunSide) >> 5) * sizeof(u32));
     CKC(cudaMemcpyAsync(d_runs, runs.data(), sizeof(RunIn) * nr, cudaMemcpyHostToDevice, stream));
     if (!cells.empty())
       CKC(cudaMemcpyAsync(d_cells, cells.data(), sizeof(int32_t) * cells.size(), cudaMemcpyHostToDevice, stream));
@@ -523,11 +532,7 @@ extern "C" int e13_check_crafted(e13_ctx *ctx, const char *const *lines, int n, 
     if (overflow) rc = E13_ERR_OVERFLOW;
   }
 done:
-  cudaFree(d_tables);
-  cudaFree(d_walk);
-  cudaFree(d_runs);
-  cudaFree(d_rout);
-  cudaFree(d_cells);
-  cudaFree(d_tape);
+  cudaStreamSynchronize(stream);
+  e13_ctx_scratch_done(ctx);
   return rc;
 }

@@ -27,6 +27,7 @@
 #include "e13.h"
 #include "e13_device.cuh"
 #include "e13_node.cuh"
+#include "e13_scratch.h"
 
 using namespace e13dev;
 
@@ -232,7 +233,9 @@ extern "C" int e13_estimate(e13_ctx *ctx, const e13_job *job, int64_t probes, ui
     if (job->tab[i] < E13_FREE || (job->tab[i] >= 0 && (job->tab[i] >> 2) >= job->nq)) return E13_ERR_ARG;
   if (cudaSetDevice(e13_ctx_device(ctx)) != cudaSuccess) return E13_ERR_CUDA;
   cudaStream_t s = e13_ctx_stream(ctx);
-  if (upload_filter_tables() != cudaSuccess) return E13_ERR_CUDA;
+  bool *tables = e13_ctx_filter_tables(ctx, 0);
+  if (!*tables && upload_filter_tables() != cudaSuccess) return E13_ERR_CUDA;
+  *tables = true;
   int nsm = 0;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, e13_ctx_device(ctx));
   const size_t smem = kKeySmemBytes + (size_t)(kTapeWords + 16) * kEstBlock * 4 + (size_t)(kEstBlock / 32) * sizeof(Node);
@@ -247,9 +250,10 @@ extern "C" int e13_estimate(e13_ctx *ctx, const e13_job *job, int64_t probes, ui
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   int rc = E13_ERR_CUDA;
   std::vector<double> h((size_t)probes * 4);
-  if (cudaMalloc(&d_root, sizeof(Node)) != cudaSuccess || cudaMalloc(&d_out, sizeof(double) * 4 * probes) != cudaSuccess ||
-      cudaMalloc(&d_next, sizeof(unsigned long long)) != cudaSuccess || cudaEventCreate(&e0) != cudaSuccess ||
-      cudaEventCreate(&e1) != cudaSuccess)
+  d_root = (Node *)e13_ctx_scratch(ctx, kScratchEstRoot, sizeof(Node));
+  d_out = (double *)e13_ctx_scratch(ctx, kScratchEstOut, sizeof(double) * 4 * probes);
+  d_next = (unsigned long long *)e13_ctx_scratch(ctx, kScratchEstNext, sizeof(unsigned long long));
+  if (!d_root || !d_out || !d_next || cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess)
     goto done;
   if (cudaMemcpyAsync(d_root, &root, sizeof root, cudaMemcpyHostToDevice, s) != cudaSuccess ||
       cudaMemsetAsync(d_next, 0, sizeof(unsigned long long), s) != cudaSuccess)
@@ -292,8 +296,6 @@ extern "C" int e13_estimate(e13_ctx *ctx, const e13_job *job, int64_t probes, ui
 done:
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
-  cudaFree(d_root);
-  cudaFree(d_out);
-  cudaFree(d_next);
+  e13_ctx_scratch_done(ctx);
   return rc;
 }

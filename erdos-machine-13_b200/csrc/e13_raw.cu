@@ -18,6 +18,7 @@
 #include "e13.h"
 #include "e13_device.cuh"
 #include "e13_macro.cuh"
+#include "e13_scratch.h"
 
 using namespace e13dev;
 
@@ -215,10 +216,11 @@ extern "C" int e13_raw_run(e13_ctx *ctx, const uint8_t *codes, uint64_t seed, in
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  if (codes && cudaMalloc(&d_codes, (size_t)n * 2 * nq) != cudaSuccess) rc = E13_ERR_CUDA;
-  if (!rc && out && cudaMalloc(&d_out, sizeof(long long) * 4 * (size_t)n) != cudaSuccess) rc = E13_ERR_CUDA;
-  if (!rc && cudaMalloc(&d_work, sizeof(RawWork)) != cudaSuccess) rc = E13_ERR_CUDA;
-  if (!rc && park && cudaMalloc(&d_list, sizeof(int) * (size_t)n) != cudaSuccess) rc = E13_ERR_CUDA;
+  if (codes) d_codes = (unsigned char *)e13_ctx_scratch(ctx, kScratchRawCodes, (size_t)n * 2 * nq);
+  if (out) d_out = (long long *)e13_ctx_scratch(ctx, kScratchRawOut, sizeof(long long) * 4 * (size_t)n);
+  d_work = (RawWork *)e13_ctx_scratch(ctx, kScratchRawWork, sizeof(RawWork));
+  if (park) d_list = (int *)e13_ctx_scratch(ctx, kScratchRawList, sizeof(int) * (size_t)n);
+  if ((codes && !d_codes) || (out && !d_out) || !d_work || (park && !d_list)) rc = E13_ERR_CUDA;
   if (!rc) {
     int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, e13_ctx_device(ctx));
@@ -250,9 +252,6 @@ extern "C" int e13_raw_run(e13_ctx *ctx, const uint8_t *codes, uint64_t seed, in
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  cudaFree(d_codes);
-  cudaFree(d_out);
-  cudaFree(d_work);
-  cudaFree(d_list);
+  e13_ctx_scratch_done(ctx);
   return rc;
 }

@@ -43,6 +43,7 @@
 #include "e13_device.cuh"
 #include "e13_macro.cuh"
 #include "e13_node.cuh"
+#include "e13_scratch.h"
 
 using namespace e13dev;
 
@@ -1295,6 +1296,14 @@ __global__ void __launch_bounds__(kLongBlock) full_long_kernel(const int *tabs, 
 // ------------------------------------------------------------------------
 // host side
 
+// What the graph of a search's epochs depends on.
+struct GraphKey {
+  Params P;
+  int blocks, block, epochs, pad;
+  size_t smem;
+  long long cap, batch_max, pool_cap;
+};
+
 struct e13_ctx {
   int device;
   int nsm;
@@ -1325,6 +1334,17 @@ struct e13_ctx {
   unsigned long long *d_jobnodes;  // kMaxJobs
   unsigned long long *h_jobbuf;  // pinned: counters then node counts
   e13_stats stats;
+  // working memory of the calls that need some, kept from one call to the next
+  // (e13_ctx_scratch), and the serve sessions' second frontier stack
+  void *scratch[kScratchSlots];
+  size_t scratch_cap[kScratchSlots];
+  Node *alt;
+  long long alt_cap;
+  e13_serve *sessions;             // open ones, linked by e13_serve::next
+  bool filter_tables[2];           // other files' copies of the filter tables are uploaded
+  // the epochs' graph of the last search, for the next one with the same parameters
+  cudaGraphExec_t graph;
+  unsigned char graph_key[sizeof(GraphKey)];
 };
 
 static int cuda_fail(cudaError_t e, const char *what) {
@@ -1418,6 +1438,8 @@ extern "C" int e13_ctx_create(int device, e13_ctx **out) {
   return E13_OK;
 }
 
+static void detach_sessions(e13_ctx *c);
+
 extern "C" void e13_ctx_destroy(e13_ctx *c) {
   if (!c) return;
   cudaSetDevice(c->device);
@@ -1436,6 +1458,10 @@ extern "C" void e13_ctx_destroy(e13_ctx *c) {
   cudaFree(c->d_jobcnt);
   cudaFree(c->d_jobnodes);
   cudaFreeHost(c->h_jobbuf);
+  for (int k = 0; k < kScratchSlots; ++k) cudaFree(c->scratch[k]);
+  cudaFree(c->alt);
+  if (c->graph) cudaGraphExecDestroy(c->graph);
+  detach_sessions(c);
   cudaEventDestroy(c->ev0);
   cudaEventDestroy(c->ev1);
   cudaEventDestroy(c->k0);
@@ -1457,6 +1483,40 @@ extern "C" int e13_last_stats(const e13_ctx *c, e13_stats *out) {
   if (!c || !out) return E13_ERR_ARG;
   *out = c->stats;
   return E13_OK;
+}
+
+extern "C" bool *e13_ctx_filter_tables(e13_ctx *c, int which) { return &c->filter_tables[which]; }
+
+extern "C" void *e13_ctx_scratch(e13_ctx *c, int slot, size_t bytes) {
+  if (c->scratch_cap[slot] >= bytes) return c->scratch[slot];
+  cudaFree(c->scratch[slot]);
+  c->scratch[slot] = nullptr;
+  c->scratch_cap[slot] = 0;
+  if (cudaMalloc(&c->scratch[slot], bytes) != cudaSuccess) {
+    // give back what other calls left, and try once more
+    cudaGetLastError();
+    for (int k = 0; k < kScratchSlots; ++k) {
+      if (e13_scratch_call(k) == e13_scratch_call(slot)) continue;  // this call's own
+      cudaFree(c->scratch[k]);
+      c->scratch[k] = nullptr;
+      c->scratch_cap[k] = 0;
+    }
+    if (cudaMalloc(&c->scratch[slot], bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+  }
+  c->scratch_cap[slot] = bytes;
+  return c->scratch[slot];
+}
+
+extern "C" void e13_ctx_scratch_done(e13_ctx *c) {
+  for (int k = 0; k < kScratchSlots; ++k) {
+    if (c->scratch_cap[k] <= kScratchKeep) continue;
+    cudaFree(c->scratch[k]);
+    c->scratch[k] = nullptr;
+    c->scratch_cap[k] = 0;
+  }
 }
 
 template <typename T>
@@ -1791,8 +1851,8 @@ constexpr int kSplitStepCap = 20000;
 // depends only on its nodes (the same on every rank) and shard s keeps nodes
 // s, s + nshards, ...  What the expansion itself finished (leaves, steps,
 // survivors, with their read masks) counts in shard 0 only: *cnt and *recs
-// are zero / empty for the other shards.  Runs on buffers of its own (freed
-// before it returns), so a serve session's frontier is left alone; `slot` is
+// are zero / empty for the other shards.  Runs on scratch buffers of its own,
+// so a serve session's frontier is left alone; `slot` is
 // the job slot written into the nodes.  The expansion runs with a fixed
 // slice, step cap and run skip: a lane is requeued at the first slice end
 // past the step cap, so those settings shape the frontier, and with them fixed
@@ -1809,11 +1869,14 @@ static int split_share(e13_ctx *c, const e13_job *job, const e13_tuning &tu, int
   const long long target = kSplitPerShard * nshards;
   // the last level starts below target nodes and each node has at most `fan` children
   const long long stack_n = target * fan + nwarps * 32 + 1024, out_n = stack_n, surv_n = 4096;
-  Node *stack = nullptr, *out = nullptr;
-  Ctl *ctl = nullptr;
-  JobParam *jobs = nullptr;
-  unsigned long long *jobcnt = nullptr;
-  SurvRec *surv = nullptr;
+  Node *stack = (Node *)e13_ctx_scratch(c, kScratchSplitStack, sizeof(Node) * (size_t)stack_n);
+  Node *out = (Node *)e13_ctx_scratch(c, kScratchSplitOut, sizeof(Node) * (size_t)out_n);
+  Ctl *ctl = (Ctl *)e13_ctx_scratch(c, kScratchSplitCtl, sizeof(Ctl));
+  JobParam *jobs = (JobParam *)e13_ctx_scratch(c, kScratchSplitJobs, sizeof(JobParam) * kMaxJobs);
+  unsigned long long *jobcnt = (unsigned long long *)e13_ctx_scratch(
+      c, kScratchSplitCounts, sizeof(unsigned long long) * kMaxJobs * kJobCounters);
+  SurvRec *surv = (SurvRec *)e13_ctx_scratch(c, kScratchSplitSurv, sizeof(SurvRec) * (size_t)surv_n);
+  if (!stack || !out || !ctl || !jobs || !jobcnt || !surv) return E13_ERR_CUDA;
   int rc = E13_OK;
   auto fail = [&](cudaError_t e, const char *what) {
     if (e != cudaSuccess && rc == E13_OK) rc = cuda_fail(e, what) ? E13_ERR_CUDA : E13_OK;
@@ -1832,13 +1895,7 @@ static int split_share(e13_ctx *c, const e13_job *job, const e13_tuning &tu, int
   h.batch = 1;
   h.peak = 1;
   long long top = 1;
-  if (!fail(cudaMalloc(&stack, sizeof(Node) * (size_t)stack_n), "split stack") &&
-      !fail(cudaMalloc(&out, sizeof(Node) * (size_t)out_n), "split outputs") &&
-      !fail(cudaMalloc(&ctl, sizeof(Ctl)), "split control") &&
-      !fail(cudaMalloc(&jobs, sizeof jp), "split job") &&
-      !fail(cudaMalloc(&jobcnt, sizeof(unsigned long long) * kMaxJobs * kJobCounters), "split counters") &&
-      !fail(cudaMalloc(&surv, sizeof(SurvRec) * (size_t)surv_n), "split survivors") &&
-      !fail(h2d(c, stack, &root, sizeof root), "split root") && !fail(h2d(c, ctl, &h, sizeof h), "split ctl") &&
+  if (!fail(h2d(c, stack, &root, sizeof root), "split root") && !fail(h2d(c, ctl, &h, sizeof h), "split ctl") &&
       !fail(h2d(c, jobs, jp, sizeof jp), "split job") &&
       !fail(cudaMemsetAsync(jobcnt, 0, sizeof(unsigned long long) * kMaxJobs * kJobCounters, c->stream), "memset")) {
     e13_tuning t = tu;
@@ -1894,12 +1951,7 @@ static int split_share(e13_ctx *c, const e13_job *job, const e13_tuning &tu, int
     }
   }
   cudaStreamSynchronize(c->stream);
-  cudaFree(stack);
-  cudaFree(out);
-  cudaFree(ctl);
-  cudaFree(jobs);
-  cudaFree(jobcnt);
-  cudaFree(surv);
+  e13_ctx_scratch_done(c);
   return rc;
 }
 
@@ -2035,17 +2087,35 @@ static int search_impl(e13_ctx *c, const e13_job *job, const e13_tuning *tuning,
     CK(cudaStreamSynchronize(c->stream));
   }
   if (persist) {
-    cudaGraph_t graph;
-    cudaGraphExec_t exec;
-    CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    for (int e = 0; e < tu.epochs_per_graph; ++e) {
-      search_kernel<true><<<blocks, tu.block, smem, c->stream>>>(P);
-      long_kernel<<<c->nsm * kLongPerSm, kLongBlock, long_smem(), c->stream>>>(P);
-      move_outputs<<<move_blocks, 256, 0, c->stream>>>(c->ctl, c->stack, c->out, c->pool, c->pool_cap, cap);
-      finish_launch<<<1, 1, 0, c->stream>>>(c->ctl, cap, batch_max, c->pool_cap);
+    GraphKey key;
+    memset((void *)&key, 0, sizeof key);
+    memcpy((void *)&key.P, (const void *)&P, sizeof P);
+    key.blocks = blocks;
+    key.block = tu.block;
+    key.epochs = tu.epochs_per_graph;
+    key.smem = smem;
+    key.cap = cap;
+    key.batch_max = batch_max;
+    key.pool_cap = c->pool_cap;
+    if (!c->graph || memcmp(&key, c->graph_key, sizeof key) != 0) {
+      cudaGraph_t graph;
+      if (c->graph) CK(cudaGraphExecDestroy(c->graph));
+      c->graph = nullptr;
+      CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+      for (int e = 0; e < tu.epochs_per_graph; ++e) {
+        search_kernel<true><<<blocks, tu.block, smem, c->stream>>>(P);
+        long_kernel<<<c->nsm * kLongPerSm, kLongBlock, long_smem(), c->stream>>>(P);
+        move_outputs<<<move_blocks, 256, 0, c->stream>>>(c->ctl, c->stack, c->out, c->pool, c->pool_cap, cap);
+        finish_launch<<<1, 1, 0, c->stream>>>(c->ctl, cap, batch_max, c->pool_cap);
+      }
+      CK(cudaStreamEndCapture(c->stream, &graph));
+      const cudaError_t made = cudaGraphInstantiate(&c->graph, graph, 0);
+      cudaGraphDestroy(graph);
+      if (made != cudaSuccess) c->graph = nullptr;
+      CK(made);
+      memcpy(c->graph_key, &key, sizeof key);
     }
-    CK(cudaStreamEndCapture(c->stream, &graph));
-    CK(cudaGraphInstantiate(&exec, graph, 0));
+    const cudaGraphExec_t exec = c->graph;
     for (;;) {
       CK(cudaGraphLaunch(exec, c->stream));
       launches += 4LL * tu.epochs_per_graph;
@@ -2063,8 +2133,6 @@ static int search_impl(e13_ctx *c, const e13_job *job, const e13_tuning *tuning,
       }
       if (checkpoint_step(err)) break;
     }
-    cudaGraphExecDestroy(exec);
-    cudaGraphDestroy(graph);
   } else {
     for (;;) {
       search_kernel<false><<<blocks, tu.block, smem, c->stream>>>(P);
@@ -2157,12 +2225,10 @@ extern "C" int e13_run_full(e13_ctx *c, const int32_t *tabs, int n, int nq, int6
   CK(cudaSetDevice(c->device));
   int rc = ensure_consts(c);
   if (rc) return rc;
-  int *d_tabs = nullptr;
-  int *d_list = nullptr;
-  long long *d_out = nullptr;
-  CK(cudaMalloc(&d_tabs, sizeof(int) * E13_MAXCELLS * (size_t)n));
-  CK(cudaMalloc(&d_out, sizeof(long long) * 7 * (size_t)n));
-  CK(cudaMalloc(&d_list, sizeof(int) * ((size_t)n + 2)));
+  int *d_tabs = (int *)e13_ctx_scratch(c, kScratchFullTabs, sizeof(int) * E13_MAXCELLS * (size_t)n);
+  long long *d_out = (long long *)e13_ctx_scratch(c, kScratchFullOut, sizeof(long long) * 7 * (size_t)n);
+  int *d_list = (int *)e13_ctx_scratch(c, kScratchFullList, sizeof(int) * ((size_t)n + 2));
+  if (!d_tabs || !d_out || !d_list) return E13_ERR_CUDA;
   CK(cudaMemsetAsync(d_list, 0, sizeof(int) * 2, c->stream));
   CK(h2d(c, d_tabs, tabs, sizeof(int) * E13_MAXCELLS * (size_t)n));
   const int bd = 256;
@@ -2174,9 +2240,7 @@ extern "C" int e13_run_full(e13_ctx *c, const int32_t *tabs, int n, int nq, int6
   CK(cudaGetLastError());
   CK(d2h(c, out, d_out, sizeof(long long) * 7 * (size_t)n));
   CK(cudaStreamSynchronize(c->stream));
-  cudaFree(d_tabs);
-  cudaFree(d_out);
-  cudaFree(d_list);
+  e13_ctx_scratch_done(c);
   return E13_OK;
 }
 
@@ -2392,11 +2456,29 @@ struct e13_serve {
   unsigned long long *d_fill = nullptr;
   unsigned long long fill[kMaxJobs];
   bool reorder = false;
+  e13_serve *next = nullptr;  // e13_ctx::sessions
   ~e13_serve() {
+    if (c) {
+      // the context keeps the second stack for its next session
+      for (e13_serve **p = &c->sessions; *p; p = &(*p)->next)
+        if (*p == this) {
+          *p = next;
+          break;
+        }
+      if (!c->alt) {
+        std::swap(c->alt, alt);
+        c->alt_cap = alt_cap;
+      }
+    }
     cudaFree(alt);
     cudaFree(d_fill);
   }
 };
+
+// A context that goes before its sessions: they then own what they hold.
+static void detach_sessions(e13_ctx *c) {
+  for (e13_serve *s = c->sessions; s; s = s->next) s->c = nullptr;
+}
 
 extern "C" int e13_serve_create(e13_ctx *c, const e13_tuning *tuning, int64_t reserve_nodes, e13_serve **out) {
   if (!c || !out || reserve_nodes < 0) return E13_ERR_ARG;
@@ -2437,12 +2519,22 @@ extern "C" int e13_serve_create(e13_ctx *c, const e13_tuning *tuning, int64_t re
   CK(cudaMemsetAsync(c->long_items, 0, sizeof(unsigned long long) * (size_t)c->long_items_cap, c->stream));
   CK(cudaMemsetAsync(c->d_jobcnt, 0, sizeof(unsigned long long) * kMaxJobs * kJobCounters, c->stream));
   CK(h2d(c, c->d_jobs, s->jp, sizeof s->jp));
-  CK(cudaMalloc(&s->alt, sizeof(Node) * (size_t)c->stack_cap));
-  s->alt_cap = c->stack_cap;
+  if (c->alt_cap < c->stack_cap) {
+    cudaFree(c->alt);
+    c->alt = nullptr;
+    c->alt_cap = 0;
+    CK(cudaMalloc(&c->alt, sizeof(Node) * (size_t)c->stack_cap));
+    c->alt_cap = c->stack_cap;
+  }
+  std::swap(s->alt, c->alt);
+  s->alt_cap = c->alt_cap;
+  c->alt_cap = 0;
   CK(cudaMalloc(&s->d_fill, sizeof(unsigned long long) * kMaxJobs));
   CK(cudaStreamSynchronize(c->stream));
   memset(&c->stats, 0, sizeof c->stats);
   s->t0 = wall_seconds();
+  s->next = c->sessions;
+  c->sessions = s.get();
   *out = s.release();
   return E13_OK;
 }

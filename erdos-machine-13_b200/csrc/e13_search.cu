@@ -181,6 +181,8 @@ static __device__ __noinline__ void record_survivor(Ctl *ctl, SurvRec *surv, lon
   r->job = job;
 }
 
+constexpr int kWarpWords = (kTapeWords + 16) * 32 + (int)sizeof(Node) / 4;  // shared memory of a search warp
+
 enum { kStRun = 0, kStIdle = 1, kStFork = 2, kStCap = 3, kStDead = 4, kStSurv = 5 };
 
 // A block's view of the persistent kernel's control words.  All warps of the
@@ -280,12 +282,14 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
   if (P.ctl->top == 0 && P.ctl->pool_tail == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const KeyTabs K = key_tables(smem_raw);
-  u32 *tape = reinterpret_cast<u32 *>(smem_raw + kKeySmemBytes);
-  const int stride = blockDim.x;
+  // a warp's tapes, its tables, and (persistent) a copy of its current
+  // stack-top node, so lanes taking its children read shared memory instead of
+  // HBM.  Words of a lane are 32 apart: a constant, so that addresses fold
+  constexpr int stride = 32;
+  const int nthr = blockDim.x;
+  u32 *tape = reinterpret_cast<u32 *>(smem_raw + kKeySmemBytes) + (threadIdx.x >> 5) * kWarpWords;
   u32 *rows = tape + kTapeWords * stride;
-  // persistent: a shared-memory copy of each warp's current stack-top node, so
-  // lanes taking its children read shared memory instead of HBM
-  Node *mytop = reinterpret_cast<Node *>(rows + 16 * stride) + (threadIdx.x >> 5);
+  Node *mytop = reinterpret_cast<Node *>(rows + 16 * stride);
   __shared__ int4 s_jp[kMaxJobs];                              // per-job moves and symmetry range
   __shared__ unsigned long long s_jc[kMaxJobs][kJobCounters];  // per-job leaves, steps, deaths by stage
 
@@ -309,16 +313,16 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
     const JobParam jp = P.jobs[threadIdx.x];
     s_jp[threadIdx.x] = make_int4(jp.nv, jp.sym_lo, jp.sym_hi, 0);
   }
-  for (int i = threadIdx.x; i < kMaxJobs * kJobCounters; i += stride) (&s_jc[0][0])[i] = 0ull;
+  for (int i = threadIdx.x; i < kMaxJobs * kJobCounters; i += nthr) (&s_jc[0][0])[i] = 0ull;
   load_stage_tables();
-  u32 *tcol = tape + threadIdx.x;
-  u32 *rcol = rows + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  u32 *tcol = tape + lane;
+  u32 *rcol = rows + lane;
   for (int w = 0; w < kTapeWords; ++w) tcol[w * stride] = 0;
   __syncthreads();
 
-  const int lane = threadIdx.x & 31;
   const unsigned lt_mask = (1u << lane) - 1u;
-  const long long gwarp = ((long long)blockIdx.x * stride + threadIdx.x) >> 5;
+  const long long gwarp = ((long long)blockIdx.x * nthr + threadIdx.x) >> 5;
   Ctl *ctl = P.ctl;
   const long long top0 = ctl->top;
   const long long batch = ctl->batch;
@@ -356,7 +360,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
   L.job = 0;
 
   // warp-uniform state
-  const int nwarps_all = (int)(((long long)gridDim.x * stride) >> 5);
+  const int nwarps_all = (int)(((long long)gridDim.x * nthr) >> 5);
   int sp = 0, wbot = 0;        // persistent: this warp's DFS stack, a ring of D slots from wbot
   bool have_cur = false;       // cursor registers hold the children left of the current node
   const Node *cur = nullptr;   // plain: the current input node
@@ -810,7 +814,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
     atomicAdd(&s_stat[4], (unsigned long long)st_claims);
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < kMaxJobs * kJobCounters; i += stride) {
+  for (int i = threadIdx.x; i < kMaxJobs * kJobCounters; i += nthr) {
     const unsigned long long v = (&s_jc[0][0])[i];
     if (v) atomicAdd(P.jobcnt + i, v);
   }
@@ -821,7 +825,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
   if (PERSIST) {
     // input this block claimed but did not take before the epoch ended
     const unsigned k0 = (unsigned)s_in.range, k1 = (unsigned)(s_in.range >> 32);
-    for (unsigned k = k0 + (threadIdx.x >> 5); k < k1; k += stride >> 5) {
+    for (unsigned k = k0 + (threadIdx.x >> 5); k < k1; k += nthr >> 5) {
       unsigned long long o = 0;
       if (lane == 0) o = atomicAdd(&ctl->nout, 1ull);
       o = __shfl_sync(kFull, o, 0);
@@ -1602,7 +1606,7 @@ static size_t long_smem() {
 }
 
 static size_t search_smem(int block) {
-  return kKeySmemBytes + (size_t)(kTapeWords + 16) * block * 4 + (size_t)(block / 32) * sizeof(Node);
+  return kKeySmemBytes + (size_t)(block / 32) * kWarpWords * 4;
 }
 
 // Shared memory of the persistent kernel and of the long-machine kernel behind it.

@@ -39,7 +39,10 @@ def test_random_machines_equal_oracle(nq, nmax, mode):
     for line, ci, o in zip(lines, ins, outs):
         if mode == 0:
             ok, verdict, counters = O.recheck_line(line, nmax)
-            assert E.format_recheck(o, nmax) == verdict, line
+            got = E.format_recheck(o, nmax)
+            if nmax < 9:  # recheck.c prints a counter it has not filled there, the library the empty set
+                got, verdict = (v.split(" (c2 counter")[0] for v in (got, verdict))
+            assert got == verdict, line
             for n in range(1, o.stages_done + 1):
                 got = "".join(f"{o.ones_cells[n][j]}," for j in range(min(o.nones[n], 64)))
                 assert got == counters[n - 1], (line, n)

@@ -85,15 +85,13 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const Ke
   int p = L.p, b = L.p >> 5;
   int left = L.deadline + 1 - L.t;  // steps that still pass the deadline test
   u64 tgt = HASH ? s_tgt[L.nt] : 0ull;
-  u32 sk = (u32)L.st | 32u | ((p & 31) ? 16u : 0u);
+  u32 key = make_key(L.st, (p & 31) != 0);
   bool single = (p & 31) != 0 && (p & 31) != 31;  // this visit step by step
   bool inside = single;                           // the head is inside the word (at p), not on its edge
-  bool rep = false;                 // the last visit left its word alone and goes on in the same way,
-  u32 rep_c = 0;                    // from content rep_c
   // visits not yet tested: lane j holds the j-th (its word, key, steps left
   // before it and the cells it changed)
   int noted = 0, v_b = 0, v_left = 0;
-  u32 v_sk = 0, v_d = 0;
+  u32 v_key = 0, v_d = 0;
   int snap_b = 0, snap_left = 0, snaps = 0;
   u32 snap_at = 0, snap0 = 0, snap1 = 0, snap2 = 0;  // words snap_b - 1 .. snap_b + 1
   bool far = true;                  // left those words, or reached a stage, since the snapshot
@@ -107,35 +105,33 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const Ke
       // but its end: what the visit changes is selected by `ok`
       u32 c, n;
       uint4 *slot, e;
-      bool ok, in_range, sweep;
+      bool ok, in_range;
+      bool rep;  // the visit left its word alone and goes on in the same way
       do {
         c = M.tape[b];
-        slot = M.memo + memo_slot(c, sk);
+        slot = M.memo + memo_slot(c, key);
         e = *slot;
-        n = e.y >> 16;
+        n = memo_steps(e);
         in_range = (unsigned)(b - 1) < (unsigned)(kLastWord - 1);
-        sweep = rep && c == rep_c;
-        ok = in_range && !sweep && e.x == c && (e.y & 63u) == sk && n - 1u < (u32)left;
+        ok = in_range && memo_match(e, c, key) && n - 1u < (u32)left;
         const bool mine = ok && lane == noted;
         v_b = mine ? b : v_b;
-        v_sk = mine ? sk : v_sk;
+        v_key = mine ? key : v_key;
         v_left = mine ? left : v_left;
         v_d = mine ? c ^ e.z : v_d;
-        if (READS && ok) reads |= e.w;
+        if (READS && ok) reads |= e.y;
         if (ok) M.tape[b] = e.z;  // every lane writes the same value
-        const u32 next = (e.y >> 6) & 63u;
+        const u32 next = memo_next(e);
         left = ok ? left - (int)n : left;
         noted = ok ? noted + 1 : noted;
-        rep = ok && e.z == c && next == sk;
-        rep_c = c;
-        sk = ok ? next : sk;
-        b = ok ? b + 1 - (int)((next >> 3) & 2u) : b;
-      } while (ok && noted < 32);
-      if (!ok) {
-        const bool known = e.x == c && (e.y & 63u) == sk;
-        if (in_range && sweep && known) {
-          // the i-th free lane looks at the i-th word ahead
-          const int dir = 1 - (int)((sk >> 3) & 2u), i = lane - noted;
+        rep = ok && e.z == c && next == key;
+        key = ok ? next : key;
+        b = ok ? b + memo_move(e) : b;
+      } while (ok && !rep && noted < 32);
+      if (rep) {
+        if (noted < 32) {
+          // a sweep: the i-th free lane looks at the i-th word ahead
+          const int dir = key_dir(key), i = lane - noted;
           const int w = b + dir * i;
           const bool same = i >= 0 && (unsigned)(w - 1) < (unsigned)(kLastWord - 1) && M.tape[w] == c;
           const u32 m = __ballot_sync(kAll, !same) >> noted;
@@ -143,7 +139,7 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const Ke
           if (run * (int)n > left) run = 0;
           if (i >= 0 && i < run) {
             v_b = w;
-            v_sk = sk;
+            v_key = key;
             v_left = left - i * (int)n;
             v_d = 0;
           }
@@ -151,12 +147,10 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const Ke
           left -= run * (int)n;
           b += dir * run;
           if (noted < 32) continue;
-        } else if (in_range && !known) {
-          const uint4 v = macro_visit<READS ? kNoteReads : kNoteNothing>(M.act, c, sk);
-          __syncwarp();
-          if (lane == 0) *slot = v;
-          __syncwarp();
-          if (v.y >> 16) continue;
+        }
+      } else if (!ok) {
+        if (in_range && !memo_match(e, c, key)) {
+          if (memo_steps(memo_fetch<READS, false>(slot, e, M.act, c, key, lane))) continue;
           single = true;
         } else {
           single = true;  // an end of the window, a visit to be single-stepped, or too few steps left
@@ -205,7 +199,7 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const Ke
         if (mine && lane >= j && v_d) atomicXor(&M.tape[v_b], v_d);
         __syncwarp();
         b = __shfl_sync(kAll, v_b, j);
-        sk = __shfl_sync(kAll, v_sk, j);
+        key = __shfl_sync(kAll, v_key, j);
         left = __shfl_sync(kAll, v_left, j);
         hb = start ^ (((u64)__shfl_sync(kAll, (u32)(sum >> 32), j) << 32) | __shfl_sync(kAll, (u32)sum, j));
         single = true;
@@ -215,9 +209,9 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const Ke
       // same word in the same way as visit 0, and between them only visit 0's
       // word and its neighbours were entered and ended as they were
       const int b0 = __shfl_sync(kAll, v_b, 0);
-      const u32 sk0 = __shfl_sync(kAll, v_sk, 0);
+      const u32 key0 = __shfl_sync(kAll, v_key, 0);
       if (__any_sync(kAll, lane < noted && (unsigned)(v_b - snap_b + 1) > 2u)) far = true;
-      m = __ballot_sync(kAll, lane > 0 && lane < noted && v_b == b0 && v_sk == sk0);
+      m = __ballot_sync(kAll, lane > 0 && lane < noted && v_b == b0 && v_key == key0);
       for (int tries = 0; m && tries < kLoopTries; ++tries, m &= m - 1) {
         const int j = __ffs(m) - 1;
         const bool in = lane < j;
@@ -246,18 +240,17 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const Ke
         visits_left = kYieldEvery;
       }
       noted = 0;
-      rep = false;
       if (HASH && macro_clock() > t_end) {
-        L.p = b * 32 + ((sk & 16u) ? 31 : 0);
-        L.st = (int)(sk & 15u);
+        L.p = b * 32 + key_bit(key);
+        L.st = key_state(key);
         L.t = L.deadline + 1 - left;
         return kEvRun;
       }
     }
     if (!single) continue;
 
-    int st = (int)(sk & 15u);
-    if (!inside) p = b * 32 + ((sk & 16u) ? 31 : 0);
+    int st = key_state(key);
+    if (!inside) p = b * 32 + key_bit(key);
     if (!HASH && p >= 18 && p <= kTapeCells - 18) {
       // a bare run: 32 cells around the head, all inside the window the machine
       // may not leave, step by step
@@ -279,9 +272,8 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const Ke
       p += V.q - 16;
       st = V.st;
       b = p >> 5;
-      sk = (u32)st | 32u | ((p & 31) ? 16u : 0u);
+      key = make_key(st, (p & 31) != 0);
       inside = (p & 31) != 0 && (p & 31) != 31;
-      rep = false;
       yield_left = left;
       yield_clock = clock64();
       visits_left = kYieldEvery;
@@ -405,9 +397,8 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const Ke
       return ev;
     }
     b = p >> 5;
-    sk = (u32)st | 32u | ((p & 31) ? 16u : 0u);
+    key = make_key(st, (p & 31) != 0);
     single = inside = false;
-    rep = false;
   }
 }
 

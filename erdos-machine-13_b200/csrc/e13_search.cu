@@ -843,7 +843,7 @@ struct LongMem {
 
 // A warp's machine takes a child of its first read of `cell` (entry e): -1 the
 // table's own move, now read, else move v.
-static __device__ __noinline__ void take_child(Lane &L, u32 *rows, int lane, int cell, u32 e, int v,
+static __device__ __forceinline__ void take_child(Lane &L, u32 *rows, int lane, int cell, u32 e, int v,
                                                const JobParam &jp, bool run_skip) {
   __syncwarp();
   if (v < 0) {

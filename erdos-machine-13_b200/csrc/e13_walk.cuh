@@ -92,7 +92,7 @@ __device__ __forceinline__ bool walk_block_set(const WalkTape &T, int size, int 
 // limit, edge).  The head may be at cells lo .. hi.  For kWalkCell, W.st and
 // *sym say which cell.  memo must be empty or hold this table's visits.
 template <bool CRAFT>
-__device__ __noinline__ int walk_run(const WalkTape &T, uint4 *memo, const uint2 *act, int lane, Walker &W,
+__device__ __forceinline__ int walk_run(const WalkTape &T, uint4 *memo, const uint2 *act, int lane, Walker &W,
                                      const WalkStop &S, int lo, int hi, int *sym_out) {
   int head = W.head, ones = W.ones, minhead = W.minhead;
   wi64 left = W.left;
@@ -104,60 +104,54 @@ __device__ __noinline__ int walk_run(const WalkTape &T, uint4 *memo, const uint2
   const int q0 = (head + kWalkLeft) & 31;
   bool inside = q0 != 0 && q0 != 31;  // the head is inside its word, not on an edge
   bool single = inside || S.any;
-  unsigned sk = (unsigned)W.st | 32u | (q0 ? 16u : 0u);
-  bool rep = false;     // the last visit left its word alone and goes on in the same way,
-  unsigned rep_c = 0;   // from content rep_c
+  unsigned key = make_key(W.st, q0 != 0);
   int count = kWalkWatch, watch = 0;
   int snap_b = 0;
   wi64 snap_left = 0;
-  unsigned snap_sk = 0, snap0 = 0, snap1 = 0, snap2 = 0;
+  unsigned snap_key = 0, snap0 = 0, snap1 = 0, snap2 = 0;
   bool far = true;      // left the words snap_b - 1 .. snap_b + 1 since the snapshot
   for (;;) {
     if (!single) {
       unsigned c, n;
       uint4 *slot, e;
-      bool ok, in_range, sweep, clear;
+      bool ok, in_range, clear;
+      bool rep;  // the visit left its word alone and goes on in the same way
       do {
         in_range = b >= b_lo && b <= b_hi;
         c = T.win[in_range ? b : 0];
-        slot = memo + memo_slot(c, sk);
+        slot = memo + memo_slot(c, key);
         e = *slot;
-        n = e.y >> 16;
+        n = memo_steps(e);
         const unsigned mask = walk_mask(b);
         const int was = __popc(c & mask);
-        sweep = rep && c == rep_c;
         clear = (b != w1 || ones - was != S.size - t1) && (b != w2 || ones - was != S.size - t2);
-        ok = in_range && !sweep && clear && e.x == c && (e.y & 63u) == sk && n != 0 && (wi64)n <= left;
+        ok = in_range && clear && memo_match(e, c, key) && n != 0 && (wi64)n <= left;
         if (ok) T.win[b] = e.z;  // every lane writes the same value
-        const unsigned next = (e.y >> 6) & 63u;
+        const unsigned next = memo_next(e);
         ones = ok ? ones + __popc(e.z & mask) - was : ones;
-        minhead = ok ? min(minhead, 32 * b - kWalkLeft + (int)e.w) : minhead;
+        minhead = ok ? min(minhead, 32 * b - kWalkLeft + memo_lowest(e)) : minhead;
         left = ok ? left - (wi64)n : left;
-        rep = ok && e.z == c && next == sk;
-        rep_c = c;
-        sk = ok ? next : sk;
-        b = ok ? b + 1 - (int)((next >> 3) & 2u) : b;
-      } while (ok && --count > 0);
-      if (!ok) {
-        const bool known = e.x == c && (e.y & 63u) == sk;
-        if (in_range && clear && sweep && known) {
-          // lane i looks at the i-th word ahead
-          const int dir = 1 - (int)((sk >> 3) & 2u);
-          const int w = b + dir * lane;
-          const bool same = w >= b_lo && w <= b_hi && (lane == 0 || (w != w1 && w != w2)) && T.win[w] == c;
-          const unsigned m = __ballot_sync(kAll, !same);
-          int run = m ? __ffs(m) - 1 : 32;
-          if ((wi64)run * n > left) run = 0;
-          left -= (wi64)run * n;
-          b += dir * run;
-          // each visit went down to its lowest bit (and one past the word when going left)
-          if (run > 0) minhead = min(minhead, 32 * (dir < 0 ? b + 1 : b - run) - kWalkLeft + (int)e.w);
-        } else if (in_range && clear && !known) {
-          const uint4 v = macro_visit<kNoteLowest>(act, c, sk);
-          __syncwarp();
-          if (lane == 0) *slot = v;
-          __syncwarp();
-          single = (v.y >> 16) == 0;
+        rep = ok && e.z == c && next == key;
+        key = ok ? next : key;
+        b = ok ? b + memo_move(e) : b;
+      } while (ok && !rep && --count > 0);
+      if (rep) {
+        // a sweep: lane i looks at the i-th word ahead (a word that a stage may
+        // start in is left to the loop above)
+        --count;
+        const int dir = key_dir(key);
+        const int w = b + dir * lane;
+        const bool same = w >= b_lo && w <= b_hi && w != w1 && w != w2 && T.win[w] == c;
+        const unsigned m = __ballot_sync(kAll, !same);
+        int run = m ? __ffs(m) - 1 : 32;
+        if ((wi64)run * n > left) run = 0;
+        left -= (wi64)run * n;
+        b += dir * run;
+        // each visit went down to its lowest bit (and one past the word when going left)
+        if (run > 0) minhead = min(minhead, 32 * (dir < 0 ? b + 1 : b - run) - kWalkLeft + memo_lowest(e));
+      } else if (!ok) {
+        if (in_range && clear && !memo_match(e, c, key)) {
+          single = memo_steps(memo_fetch<false, true>(slot, e, act, c, key, lane)) == 0;
         } else {
           single = true;
         }
@@ -168,7 +162,7 @@ __device__ __noinline__ int walk_run(const WalkTape &T, uint4 *memo, const uint2
           if (watch == 0) {  // a snapshot, and a look after each of the next visits
             if (b > b_lo && b < b_hi) {
               snap_b = b;
-              snap_sk = sk;
+              snap_key = key;
               snap_left = left;
               snap0 = T.win[b - 1];
               snap1 = T.win[b];
@@ -177,7 +171,7 @@ __device__ __noinline__ int walk_run(const WalkTape &T, uint4 *memo, const uint2
             }
             watch = kWalkWatchFor;
           } else {
-            if (!far && b == snap_b && sk == snap_sk && T.win[b] == snap1 && T.win[b - 1] == snap0 &&
+            if (!far && b == snap_b && key == snap_key && T.win[b] == snap1 && T.win[b - 1] == snap0 &&
                 T.win[b + 1] == snap2) {
               left %= snap_left - left;
               far = true;
@@ -197,8 +191,8 @@ __device__ __noinline__ int walk_run(const WalkTape &T, uint4 *memo, const uint2
 
     // single steps until the head is in another word
     far = true;
-    int st = (int)(sk & 15u);
-    if (!inside) head = 32 * b - kWalkLeft + ((sk & 16u) ? 31 : 0);
+    int st = key_state(key);
+    if (!inside) head = 32 * b - kWalkLeft + key_bit(key);
     unsigned word = T.ld(b);
     const int first = 32 * b - kWalkLeft;
     unsigned lw = 0;  // a configuration inside this word seen earlier
@@ -273,10 +267,9 @@ __device__ __noinline__ int walk_run(const WalkTape &T, uint4 *memo, const uint2
       return ev;
     }
     b = walk_word(head);
-    sk = (unsigned)st | 32u | ((head - first) < 0 ? 16u : 0u);
+    key = make_key(st, head < first);
     inside = false;
     single = S.any;
-    rep = false;
   }
 }
 

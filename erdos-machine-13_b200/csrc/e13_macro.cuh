@@ -166,31 +166,33 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const Ke
       u64 sum = 0;
       const u64 start = hb;
       if (HASH) {
-        u32 lo = 0, hi = 0;
-        for (u32 d = mine ? v_d : 0u; d; d &= d - 1) {
-          const int i = 32 * v_b + __ffs(d) - 1;
-          lo ^= K.lo[i];
-          hi ^= K.hi[i];
-        }
-        const u32 lo0 = lo, hi0 = hi;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {  // running hash changes
-          const u32 a = __shfl_up_sync(kAll, lo, o), c = __shfl_up_sync(kAll, hi, o);
-          if (lane >= o) {
-            lo ^= a;
-            hi ^= c;
+        if (__any_sync(kAll, mine && v_d)) {  // (sweeps change nothing)
+          u32 lo = 0, hi = 0;
+          for (u32 d = mine ? v_d : 0u; d; d &= d - 1) {
+            const int i = 32 * v_b + __ffs(d) - 1;
+            lo ^= K.lo[i];
+            hi ^= K.hi[i];
           }
+          const u32 lo0 = lo, hi0 = hi;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {  // running hash changes
+            const u32 a = __shfl_up_sync(kAll, lo, o), c = __shfl_up_sync(kAll, hi, o);
+            if (lane >= o) {
+              lo ^= a;
+              hi ^= c;
+            }
+          }
+          sum = ((u64)(hi ^ hi0) << 32) | (lo ^ lo0);  // before this lane's visit
+          hb ^= ((u64)__shfl_sync(kAll, hi, 31) << 32) | __shfl_sync(kAll, lo, 31);
         }
-        sum = ((u64)(hi ^ hi0) << 32) | (lo ^ lo0);  // before this lane's visit
-        const u64 v = hb ^ sum ^ tgt;
+        const u64 v = start ^ sum ^ tgt;
         bad = mine;
-        for (int j = 0; j < kSpans && __any_sync(kAll, bad); j += 4) {
+        for (int j = 0; j < kSpans && __any_sync(kAll, bad); j += 8) {
           u32 any = 0;
 #pragma unroll
-          for (int k = 0; k < 4; ++k) any |= span_bit(v, span[(j + k) * kTapeWords + v_b]);
+          for (int k = 0; k < 8; ++k) any |= span_bit(v, span[(j + k) * kTapeWords + v_b]);
           if (any) bad = false;
         }
-        hb ^= ((u64)__shfl_sync(kAll, hi, 31) << 32) | __shfl_sync(kAll, lo, 31);
       }
       u32 m = __ballot_sync(kAll, bad);
       if (m) {

@@ -85,6 +85,7 @@ constexpr int kLongPerSm = 2;            // 96 KB of shared memory a block
 constexpr long long kLongMinNs = 1000000;  // shortest time bound of long_kernel: 1 ms (else a tenth of the epoch)
 constexpr int kIdlePark = 8;             // many warps wait: an eighth
 constexpr int kParkMin = 1536;
+constexpr int kNeverPark = 0x7FFFFFFF;
 // Taking input and pool nodes.  One word of L2 takes an atomic or a polling
 // read at a time, so blocks claim input in chunks (at most kInputChunk nodes,
 // at least kInputChunks claims a block) and a warp donates up to kGive stack
@@ -1573,8 +1574,8 @@ static Params make_params(const e13_ctx *c, const e13_tuning &tu, int nq, long l
   P.nq = nq;
   P.slice = tu.slice;
   P.run_skip = tu.run_skip ? 1 : 0;
-  P.park_after = tu.run_skip ? std::max(kParkMin, 2 * std::min(tu.run_skip, 1 << 29)) : 0x7FFFFFFF;
-  P.park_idle = tu.run_skip ? kParkMin : 0x7FFFFFFF;
+  P.park_after = tu.run_skip ? std::max(kParkMin, 2 * std::min(tu.run_skip, 1 << 29)) : kNeverPark;
+  P.park_idle = tu.run_skip ? kParkMin : kNeverPark;
   P.longq = c->longq;
   P.long_items = c->long_items;
   P.long_ns = std::max(kLongMinNs, (long long)tu.epoch_us * 1000LL / 10);

@@ -336,6 +336,42 @@ __device__ __forceinline__ int lane_act(Lane &L, u32 *__restrict__ tcol, const u
   return 0;
 }
 
+// N steps of a running lane whose table and tape columns are 32 words apart:
+// the persistent search's hot loop.  left: steps that still pass the deadline
+// test (deadline + 1 - t).  Two branches a step: one before it for what keeps
+// it from being taken (the deadline, a cell that is no plain move), one after
+// it for what it led to (out of the window, a match of the low hash halves).
+// Returns 0 (all N taken), or as lane_act.
+template <int N>
+__device__ __forceinline__ int lane_steps(Lane &L, int &left, u32 *__restrict__ tcol, const u32 *__restrict__ rcol,
+                                          const u32 *__restrict__ keyb, int &cell, u32 &ecell) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int p = L.p;
+    u32 *const wp = tcol + ((p >> 5) << 5);
+    const u32 word = *wp;
+    const u32 row = rcol[L.st << 5];
+    const u32 kk = keyb[p];
+    const u32 sym = (word >> (p & 31)) & 1u;
+    const u32 e = row >> (sym << 4);
+    if (((e & kEntSpecial) != 0u) | (left <= 0)) {
+      if (left <= 0) return kEvDead;
+      cell = (L.st << 1) | (int)sym;
+      ecell = e & 0xFFu;
+      return kEvCell;
+    }
+    const u32 flip = (e ^ sym) & 1u;
+    *wp = word ^ (flip << (p & 31));
+    L.hb ^= kk & (0u - flip);
+    L.p = p + (int)(e & 2u) - 1;
+    const bool in = (unsigned)(L.p - 1) < (unsigned)(kTapeCells - 2);
+    L.st = (int)((e >> 2) & 15u);
+    left -= in ? 1 : 0;
+    if (!in | (L.hb == L.tgt)) return in ? kEvStage : kEvDead;  // head <= -64 or >= 1299
+  }
+  return 0;
+}
+
 // Counter hash from the tape: XOR of the keys of the ones at cells < -2
 // (exactly what the reference accumulates in hc, src/e13search.c:170).
 __device__ __forceinline__ u64 counter_hash(const u32 *tcol, const u64 *keyc, int stride) {

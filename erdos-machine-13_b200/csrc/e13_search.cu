@@ -57,14 +57,20 @@ constexpr long long kPoolNodes = 1LL << 18;  // donation pool: 256 Ki nodes (80 
 constexpr long long kWholeFrontier = 1LL << 62;  // persistent batch when e13_tuning::batch is 0
 constexpr long long kPoolWaitNs = 200000000;     // 200 ms: a donor publishes a claimed slot within microseconds
 constexpr long long kMinEpochNs = 200000;        // 200 us: the shortest epoch a starvation dump may end
-// A warp with at most kLoneLanes running machines runs each of them in the
-// tight single-machine loop step_slice, up to kLoneSteps steps per iteration
-// (kLoneStepsShort in the persistent kernel): its speed is then bound by one
-// machine's dependent chain, not by issue slots, and the lock-step loop's
-// control would only lengthen it.
+// Plain kernel: a warp with at most kLoneLanes running machines runs each of
+// them in the tight single-machine loop step_slice, up to kLoneSteps steps per
+// iteration: its speed is then bound by one machine's dependent chain, not by
+// issue slots, and the lock-step loop's control would only lengthen it.  (In
+// the persistent kernel long machines leave for long_kernel; without that loop
+// the counter search takes 706 ms instead of 731.)
 constexpr int kLoneLanes = 2;
 constexpr int kLoneSteps = 512;
-constexpr int kLoneStepsShort = 64;  // persistent: its long machines are handed over between slices
+// Persistent kernel: steps of a slice iteration.  With the default slice of 24
+// iterations a warp refills every 72 steps, and most machines die at a deadline,
+// after 73 or 153 steps.  Counter search / FMAX = 4 search of 1.8e8 machines:
+// 2 steps 749 / 53.4 ms, 3 steps 706 / 51.1, 4 steps 787 / 56.3 (739 / 51.8 with a
+// slice of 20).
+constexpr int kSteps = 3;
 
 // Long machines.  In lock-step a long machine costs a lane 0.3 us a step; alone
 // in a warp of long_kernel (e13_macro.cuh) one of 835,000 steps takes 1.5-3 ms,
@@ -694,7 +700,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
       }
     }
 
-    // ---- (D) run a slice: every running lane takes up to two actions per iteration
+    // ---- (D) run a slice
     ++rounds;
     {
       const unsigned rm = __ballot_sync(kFull, status == kStRun);
@@ -703,25 +709,28 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
       // most kLoneLanes machines runs each in the single-machine loop.  The
       // persistent kernel hands old machines over instead (below), and on
       // young ones the skip arithmetic costs more than it saves.
-      const bool lone_w = __popc(rm) <= kLoneLanes;
+      const bool lone_w = !PERSIST && __popc(rm) <= kLoneLanes;
       st_lane_rounds += __popc(rm);
       if (rm) {
+        int left = L.deadline + 1 - L.t;
 #pragma unroll 1
         for (int it = 0; it < P.slice; ++it) {
           if (status == kStRun) {
             int cell = 0;
             u32 e = 0;
-            // two actions per iteration: the loop control and the event
-            // dispatch below are paid once for both
+            // several steps or two actions per iteration: the loop control and
+            // the event dispatch below are paid once for all
             int ev;
-            if (lone_w) {
+            if (PERSIST) {
+              ev = lane_steps<kSteps>(L, left, tcol, rcol, K.lo, cell, e);
+            } else if (lone_w) {
               // the same steps and events as lane_act (step_slice follows
               // src/e13search.c:134-177 too); a hash match ends the iteration
               // and goes to the one stage test below
-              int n = PERSIST ? kLoneStepsShort : kLoneSteps;
+              int n = kLoneSteps;
               ev = step_slice(L.p, L.st, L.t, L.deadline, L.hb, L.tgt, tcol, rcol, K.lo, stride, n, cell);
               if (ev == kEvCell) e = get_entry(rcol, stride, cell);
-            } else if (!PERSIST && P.run_skip) {
+            } else if (P.run_skip) {
               ev = lane_act<true>(L, tcol, rcol, K, stride, cell, e);
               if (!ev) ev = lane_act<true>(L, tcol, rcol, K, stride, cell, e);
             } else {
@@ -731,7 +740,11 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
             // the stage test of a hash match, once per iteration outside
             // lane_act: one copy of it in the loop instead of one per
             // inlined action (the second action waits for it)
-            if (ev == kEvStage) ev = stage_check(L, tcol, K, stride);
+            if (ev == kEvStage) {
+              if (PERSIST) L.t = L.deadline + 1 - left;
+              ev = stage_check(L, tcol, K, stride);
+              left = L.deadline + 1 - L.t;
+            }
             if (ev == kEvCell) {
               if (e == kEntHalt) {
                 ev = kEvDead;
@@ -762,6 +775,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
           // of the if-blocks above, so the next action issues once for the
           // whole warp
         }
+        if (PERSIST) L.t = L.deadline + 1 - left;
         if (__any_sync(kFull, status >= kStDead)) {
           if (status >= kStDead) {
             acc_steps += (u32)(L.t - L.tseg);

@@ -35,6 +35,7 @@ namespace {
 
 constexpr unsigned kFull = 0xFFFFFFFFu;
 constexpr int kEstBlock = 256;
+constexpr int kYoungIterations = 56;  // iterations of three steps: 168 steps
 
 enum { kPrIdle = 0, kPrRun = 1, kPrFork = 2, kPrDead = 3, kPrSurv = 4 };
 
@@ -51,13 +52,21 @@ __device__ __forceinline__ u64 mix_next(u64 &s) {
 // per-step semantics as the search (lane_act, src/e13search.c:134-177); here
 // every first read is a fork, as in run() with fixed[i] == 0.
 __device__ __forceinline__ void run_to_event(Lane &L, int &status, int &fork_cell, u32 &fork_e, u32 *tcol,
-                                             const u32 *rcol, const KeyTabs &K, int stride) {
-  while (__any_sync(kFull, status == kPrRun)) {
+                                             const u32 *rcol, const KeyTabs &K) {
+  // most children stop within two deadlines (153 steps): single steps, three
+  // an iteration; the ones that go on cross runs a tape word at a time
+  for (int it = 0; __any_sync(kFull, status == kPrRun); ++it) {
     if (status == kPrRun) {
-      int cell = 0;
+      int cell = 0, ev;
       u32 e = 0;
-      int ev = lane_act<true>(L, tcol, rcol, K, stride, cell, e);
-      if (ev == kEvStage) ev = stage_check(L, tcol, K, stride);
+      if (it < kYoungIterations) {
+        int left = L.deadline + 1 - L.t;
+        ev = lane_steps<3>(L, left, tcol, rcol, K.lo, cell, e);
+        L.t = L.deadline + 1 - left;
+      } else {
+        ev = lane_act<true>(L, tcol, rcol, K, 32, cell, e);
+      }
+      if (ev == kEvStage) ev = stage_check(L, tcol, K, 32);
       if (ev == kEvCell) {
         if (e == kEntHalt) {
           status = kPrDead;  // a fixed halt cell
@@ -82,17 +91,19 @@ __global__ void __launch_bounds__(kEstBlock) estimate_kernel(const Node *root, i
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const KeyTabs K = key_tables(smem_raw);
   u32 *tape = reinterpret_cast<u32 *>(smem_raw + kKeySmemBytes);
-  const int stride = blockDim.x;
+  // a warp's tapes, tables and path node; words of a lane are 32 apart
+  constexpr int stride = 32;
+  const int lane = threadIdx.x & 31;
+  tape += (threadIdx.x >> 5) * ((kTapeWords + 16) * 32 + (int)sizeof(Node) / 4);
   u32 *rows = tape + kTapeWords * stride;
-  Node *node = reinterpret_cast<Node *>(rows + 16 * stride) + (threadIdx.x >> 5);  // this warp's path node
+  Node *node = reinterpret_cast<Node *>(rows + 16 * stride);
   fill_key_tables(K);
   load_stage_tables();
-  u32 *tcol = tape + threadIdx.x;
-  u32 *rcol = rows + threadIdx.x;
+  u32 *tcol = tape + lane;
+  u32 *rcol = rows + lane;
   for (int w = 0; w < kTapeWords; ++w) tcol[w * stride] = 0;
   __syncthreads();
 
-  const int lane = threadIdx.x & 31;
   Lane L;
   L.t = 0;
   L.tseg = 0;
@@ -116,7 +127,7 @@ __global__ void __launch_bounds__(kEstBlock) estimate_kernel(const Node *root, i
       lane_load(L, root, tcol, rcol, stride, 0);
       status = kPrRun;
     }
-    run_to_event(L, status, fork_cell, fork_e, tcol, rcol, K, stride);
+    run_to_event(L, status, fork_cell, fork_e, tcol, rcol, K);
     if (lane == 0) {
       o_nodes += 1.0;
       o_steps += (double)L.t;
@@ -151,17 +162,29 @@ __global__ void __launch_bounds__(kEstBlock) estimate_kernel(const Node *root, i
           t0 = L.t;
           status = kPrRun;
         }
-        run_to_event(L, status, fork_cell, fork_e, tcol, rcol, K, stride);
-        // weighted counts, added in child order as the reference does
+        run_to_event(L, status, fork_cell, fork_e, tcol, rcol, K);
+        // weighted counts, added in child order as the reference does: whole
+        // numbers, so in one go while all of them stay below 2^53
         const int nb = min(32, k - 32 * b);
-        for (int j = 0; j < nb; ++j) {
-          const int sj = __shfl_sync(kFull, status, j);
-          const int dj = __shfl_sync(kFull, L.t - t0, j);
-          if (lane == 0) {
-            o_nodes += w;
-            o_steps += w * (double)dj;
-            if (sj != kPrFork) o_leaves += w;
-            if (sj == kPrSurv) o_surv += w;
+        const int sum = __reduce_add_sync(kFull, c < k ? L.t - t0 : 0);
+        const int leaves = __popc(__ballot_sync(kFull, c < k && status != kPrFork));
+        const int surv = __popc(__ballot_sync(kFull, c < k && status == kPrSurv));
+        const double most = o_nodes + o_steps + w * ((double)sum + nb);  // o_leaves, o_surv <= o_nodes
+        if (__shfl_sync(kFull, most < 9007199254740992.0, 0)) {
+          o_nodes += w * nb;
+          o_steps += w * (double)sum;
+          o_leaves += w * leaves;
+          o_surv += w * surv;
+        } else {
+          for (int j = 0; j < nb; ++j) {
+            const int sj = __shfl_sync(kFull, status, j);
+            const int dj = __shfl_sync(kFull, L.t - t0, j);
+            if (lane == 0) {
+              o_nodes += w;
+              o_steps += w * (double)dj;
+              if (sj != kPrFork) o_leaves += w;
+              if (sj == kPrSurv) o_surv += w;
+            }
           }
         }
         livem[b] = __ballot_sync(kFull, status == kPrFork);
@@ -193,7 +216,7 @@ __global__ void __launch_bounds__(kEstBlock) estimate_kernel(const Node *root, i
           apply_child(L, node, ch, rcol, stride, sym_lo, sym_hi, true);
           status = kPrRun;
         }
-        run_to_event(L, status, fork_cell, fork_e, tcol, rcol, K, stride);
+        run_to_event(L, status, fork_cell, fork_e, tcol, rcol, K);
       }
       __syncwarp();  // every lane is done reading the old path node
       if (lane == holder) {

@@ -10,6 +10,7 @@ The function names follow the reference's program structure
 from __future__ import annotations
 
 import ctypes
+import mmap
 import os
 import subprocess
 
@@ -245,6 +246,17 @@ def resolve_tuning(tune: Tuning | None, serve: bool = False):
     return r, out
 
 
+def _room(ctype, n: int):
+    """A zeroed array of n ctype for a call to fill.  ctypes clears its arrays by
+    writing to them, 0.4 ms for the 65,536 records a search may return, as much
+    as a small search takes; fresh pages are zero already and cost nothing until
+    something is written to them."""
+    size = ctypes.sizeof(ctype) * n
+    if size < 1 << 16:
+        return (ctype * n)()
+    return (ctype * n).from_buffer(mmap.mmap(-1, size))
+
+
 class Context:
     """A device context (one CUDA device, one stream, reusable buffers)."""
 
@@ -267,7 +279,7 @@ class Context:
 
     def search(self, job: Job, tune: Tuning | None = None, surv_cap: int = 1 << 16):
         counts = Counts()
-        surv = (Survivor * max(surv_cap, 1))()
+        surv = _room(Survivor, max(surv_cap, 1))
         ns = ctypes.c_int()
         r = lib().e13_search(self.h, ctypes.byref(job), ctypes.byref(tune) if tune else None, ctypes.byref(counts),
                              surv, surv_cap, ctypes.byref(ns))
@@ -283,7 +295,7 @@ class Context:
     def search_shard(self, job: Job, shard: int, nshards: int, tune: Tuning | None = None, surv_cap: int = 1 << 16):
         """Shard `shard` of `nshards` of the search for `job` (e13_search_shard)."""
         counts = Counts()
-        surv = (Survivor * max(surv_cap, 1))()
+        surv = _room(Survivor, max(surv_cap, 1))
         ns = ctypes.c_int()
         r = lib().e13_search_shard(self.h, ctypes.byref(job), ctypes.byref(tune) if tune else None, shard, nshards,
                                    ctypes.byref(counts), surv, surv_cap, ctypes.byref(ns))
@@ -298,7 +310,7 @@ class Context:
         0 when the search finished, STOPPED when it stopped with a checkpoint."""
         ck = Checkpoint(path.encode(), config.encode(), interval_s, stop_after_s)
         counts = Counts()
-        surv = (Survivor * max(surv_cap, 1))()
+        surv = _room(Survivor, max(surv_cap, 1))
         ns = ctypes.c_int()
         wall = ctypes.c_double()
         left = ctypes.c_int64()
@@ -496,7 +508,7 @@ class Server:
         return lib().e13_serve_pending(self.h)
 
     def survivors(self, job_id: int, cap: int = 1 << 16):
-        out = (Survivor * cap)()
+        out = _room(Survivor, cap)
         n = ctypes.c_int()
         r = lib().e13_serve_survivors(self.h, job_id, out, cap, ctypes.byref(n))
         if r and r != -7:

@@ -48,7 +48,7 @@ struct CheckParams {
 __device__ __forceinline__ int first_of_class(int n) { return n <= 2 ? 1 : (n <= 8 ? 3 : 9); }
 
 // Shared memory of one machine: the remembered visits, the table, the window.
-size_t check_smem(int W) { return sizeof(uint4) * kMemoSize + sizeof(uint2) * 16 + sizeof(u32) * (size_t)W; }
+size_t check_smem(int W) { return (sizeof(uint4) << kWalkMemoBits) + sizeof(uint2) * 16 + sizeof(u32) * (size_t)W; }
 
 // Words of the window for stage nmax: cells -4096 .. 2^nmax + 4096.
 int window_words(int nmax) { return (int)((kWalkLeft + (1LL << nmax) + 4096 + 31) / 32 + 2); }
@@ -64,7 +64,7 @@ __device__ u32 check_code(const e13_check_in &in, int s, int a) {
 __global__ void __launch_bounds__(32) check_kernel(const CheckParams P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint4 *memo = reinterpret_cast<uint4 *>(smem_raw);
-  uint2 *act = reinterpret_cast<uint2 *>(memo + kMemoSize);
+  uint2 *act = reinterpret_cast<uint2 *>(memo + (1 << kWalkMemoBits));
   const int m = blockIdx.x, lane = threadIdx.x;
   WalkTape T;
   T.win = reinterpret_cast<u32 *>(act + 16);
@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(32) check_kernel(const CheckParams P) {
   T.gshift = P.gshift;
   const e13_check_in &in = P.in[m];
   e13_check_out &o = P.out[m];
-  for (int i = lane; i < kMemoSize; i += 32) memo[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (int i = lane; i < (1 << kWalkMemoBits); i += 32) memo[i] = make_uint4(0u, 0u, 0u, 0u);
   for (int w = lane; w < P.W; w += 32) T.win[w] = 0;
   reinterpret_cast<u32 *>(act)[lane] = act_word(check_code(in, lane >> 1, lane & 1), (u32)lane & 1u);
   __syncwarp();

@@ -87,7 +87,7 @@ struct RunOut {
 
 // One warp's shared memory.
 struct WarpMem {
-  uint4 memo[kMemoSize];
+  uint4 memo[1 << kWalkMemoBits];
   uint2 act[16];
   u32 win[kWindow];
 };
@@ -114,7 +114,7 @@ __device__ int counter_cells(const WalkTape &T, i64 side, int minhead, int32_t *
 
 // A blank tape with its HBM words at `tape`, and the table.
 __device__ WalkTape start(WarpMem &M, u32 *tape, i64 side, const unsigned char *code, int lane) {
-  for (int i = lane; i < kMemoSize; i += 32) M.memo[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (int i = lane; i < 1 << kWalkMemoBits; i += 32) M.memo[i] = make_uint4(0u, 0u, 0u, 0u);
   for (int i = lane; i < kWindow; i += 32) M.win[i] = 0;
   reinterpret_cast<u32 *>(M.act)[lane] = act_word(code[lane], (u32)lane & 1u);
   __syncwarp();

@@ -6,7 +6,7 @@
 // What a machine does inside one 32-cell word depends only on its state, the
 // side it enters from and the word's content, so the warp remembers the
 // outcome of each such visit (new content, exit side and state, steps) in a
-// small direct-mapped table in shared memory and applies it in one go the next
+// small table in shared memory and applies it in one go the next
 // time.  An entry is made when it is first needed by running the machine
 // inside the word.  A visit that leaves the word as it was and goes on into an
 // equal word in the same state is a sweep: the lanes look at the next words
@@ -44,8 +44,9 @@ constexpr int kLastWord = kTapeWords - 1;
 constexpr int kSpans = 32;           // functionals per word
 
 // What one warp needs in shared memory.
+template <int BITS>
 struct MacroMem {
-  uint4 memo[kMemoSize];
+  uint4 memo[1 << BITS];
   u32 tape[kTapeWords + 1];
   uint2 act[16];  // the table for macro_visit
   u32 rows[16];
@@ -59,10 +60,11 @@ __device__ __forceinline__ unsigned long long macro_clock() {
 }
 
 // After a change of M.rows: the expanded table, and an empty memory of visits.
-__device__ __forceinline__ void macro_table(MacroMem &M, int lane) {
+template <int BITS>
+__device__ __forceinline__ void macro_table(MacroMem<BITS> &M, int lane) {
   __syncwarp();
   reinterpret_cast<u32 *>(M.act)[lane] = act_word((M.rows[lane >> 1] >> ((lane & 1) << 4)) & 0xFFu, (u32)lane & 1u);
-  for (int i = lane; i < kMemoSize; i += 32) M.memo[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (int i = lane; i < 1 << BITS; i += 32) M.memo[i] = make_uint4(0u, 0u, 0u, 0u);
   __syncwarp();
 }
 
@@ -79,9 +81,9 @@ __device__ __forceinline__ u32 span_bit(u64 v, u64 f) {
 // not counted).  READS: reads collects the table cells read.
 enum { kEvOff = 5 };
 
-template <bool HASH, bool READS = false>
-__device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const KeyTabs &K, const u64 *span, int lane,
-                                         u32 &reads, int &cell, u32 &ecell, unsigned long long t_end) {
+template <bool HASH, bool READS = false, int BITS>
+__device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem<BITS> &M, const KeyTabs &K, const u64 *span,
+                                         int lane, u32 &reads, int &cell, u32 &ecell, unsigned long long t_end) {
   int p = L.p, b = L.p >> 5;
   int left = L.deadline + 1 - L.t;  // steps that still pass the deadline test
   u64 tgt = HASH ? s_tgt[L.nt] : 0ull;
@@ -109,7 +111,7 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem &M, const Ke
       bool rep;  // the visit left its word alone and goes on in the same way
       do {
         c = M.tape[b];
-        slot = M.memo + memo_slot(c, key);
+        slot = M.memo + memo_slot<BITS>(c, key);
         e = *slot;
         n = memo_steps(e);
         in_range = (unsigned)(b - 1) < (unsigned)(kLastWord - 1);

@@ -29,6 +29,10 @@ constexpr int kRawSteps = 1024;           // steps before a machine is listed
 constexpr long long kRawIntMax = 1 << 30; // longer limits are run in raw_kernel alone (its step counts are 64-bit)
 constexpr int kRawLongBlock = 256;
 constexpr int kRawLongPerSm = 3;          // 68 KB of shared memory a block
+// 24 warps an SM with 512 visits each: the listed machines are many and short
+// lived, so warps count for more than visits (a million draws: 38 ms; 12 warps
+// with 1024 visits 38-41, 6 with 2048 45).
+typedef MacroMem<9> RawMem;
 
 __device__ __forceinline__ u64 splitmix_at(u64 seed, u64 k) {
   // draw k (1-based) of splitmix64 started at `seed`
@@ -161,7 +165,7 @@ __global__ void __launch_bounds__(kRawLongBlock) raw_long_kernel(const unsigned 
                                                                  const int *__restrict__ list) {
   extern __shared__ __align__(16) unsigned char raw_long_smem[];
   const int lane = threadIdx.x & 31;
-  MacroMem &M = reinterpret_cast<MacroMem *>(raw_long_smem)[threadIdx.x >> 5];
+  RawMem &M = reinterpret_cast<RawMem *>(raw_long_smem)[threadIdx.x >> 5];
   const unsigned long long n = work->listed;
   unsigned long long steps = 0;
   for (;;) {
@@ -234,7 +238,7 @@ extern "C" int e13_raw_run(e13_ctx *ctx, const uint8_t *codes, uint64_t seed, in
     raw_kernel<<<grid, kRawBlock, smem, s>>>(d_codes, seed, n, nq, max_steps, park ? kRawSteps : max_steps, d_out, d_work,
                                              d_list);
     if (park) {
-      const size_t lsmem = sizeof(MacroMem) * (kRawLongBlock / 32);
+      const size_t lsmem = sizeof(RawMem) * (kRawLongBlock / 32);
       cudaFuncSetAttribute(raw_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsmem);
       raw_long_kernel<<<nsm * kRawLongPerSm, kRawLongBlock, lsmem, s>>>(d_codes, seed, nq, (int)max_steps, d_out, d_work,
                                                                         d_list);

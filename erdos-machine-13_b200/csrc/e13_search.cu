@@ -86,8 +86,14 @@ constexpr int kLongCap = 1 << 14;        // machines handed over per epoch, at m
 constexpr int kLongNodes = 1 << 14;      // fork nodes long_kernel keeps for its own queue
 constexpr int kLongItems = 1 << 15;      // children it queues
 constexpr int kLongOut = kLongCap + kLongItems;  // most nodes it puts on the outputs
-constexpr int kLongBlock = 256;
-constexpr int kLongPerSm = 2;            // 96 KB of shared memory a block
+// Six warps an SM that remember 2048 visits each (223 KB of shared memory): a
+// visit made again costs its steps, and that counts for more than warps.
+// FMAX = 3 searches of three machine families, with 512 visits and 16 warps
+// 8.3, 2.9, 6.8 ms, with 1024 and 8 warps 7.2, 2.3, 6.3, with 2048 and 6 warps
+// 6.7, 2.2, 5.8; tables of 20,000 machines 3.9, 3.5, 3.1.
+constexpr int kLongMemoBits = 11;
+constexpr int kLongBlock = 192;
+constexpr int kLongPerSm = 1;
 constexpr long long kLongMinNs = 1000000;  // shortest time bound of long_kernel: 1 ms (else a tenth of the epoch)
 constexpr int kIdlePark = 8;             // many warps wait: an eighth
 constexpr int kParkMin = 1536;
@@ -852,7 +858,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
 
 // One warp's shared memory in long_kernel.
 struct LongMem {
-  MacroMem m;
+  MacroMem<kLongMemoBits> m;
   Node node;
 };
 
@@ -894,7 +900,7 @@ __global__ void __launch_bounds__(kLongBlock) long_kernel(const __grid_constant_
   u64 *span = reinterpret_cast<u64 *>(smem_raw + kKeySmemBytes);
   const int lane = threadIdx.x & 31;
   LongMem &W = reinterpret_cast<LongMem *>(span + kSpans * kTapeWords)[threadIdx.x >> 5];
-  MacroMem &M = W.m;
+  MacroMem<kLongMemoBits> &M = W.m;
   const Node *N = &W.node;
   fill_key_tables(K);
   load_stage_tables();
@@ -1284,7 +1290,7 @@ __global__ void __launch_bounds__(kLongBlock) full_long_kernel(const int *tabs, 
   const KeyTabs K = key_tables(smem_raw);
   u64 *span = reinterpret_cast<u64 *>(smem_raw + kKeySmemBytes);
   const int lane = threadIdx.x & 31;
-  MacroMem &M = reinterpret_cast<LongMem *>(span + kSpans * kTapeWords)[threadIdx.x >> 5].m;
+  MacroMem<kLongMemoBits> &M = reinterpret_cast<LongMem *>(span + kSpans * kTapeWords)[threadIdx.x >> 5].m;
   fill_key_tables(K);
   load_stage_tables();
   for (int i = threadIdx.x; i < kSpans * kTapeWords; i += blockDim.x) span[i] = d_span[i];

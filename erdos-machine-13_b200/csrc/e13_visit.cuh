@@ -20,8 +20,6 @@
 namespace e13dev {
 
 constexpr unsigned kAll = 0xFFFFFFFFu;
-constexpr int kMemoBits = 9;
-constexpr int kMemoSize = 1 << kMemoBits;
 constexpr int kMemoMaxSteps = 2048;  // longest remembered visit
 
 // A key: state and side, in place for a memo entry's w.
@@ -35,9 +33,11 @@ __device__ __forceinline__ int key_dir(unsigned key) { return (key & kKeyRight) 
 
 // The first of the two slots a visit may be in: the last one used comes first,
 // the other second.  (With one slot each, two visits of a machine's sweep
-// often shared it and each evicted the other 2000 times.)
+// often shared it and each evicted the other 2000 times.)  BITS: the memory
+// has 2^BITS entries.
+template <int BITS>
 __device__ __forceinline__ unsigned memo_slot(unsigned c, unsigned key) {
-  return ((c * 0x9E3779B1u + key * 0x85EBCA6Bu) >> (33 - kMemoBits)) << 1;
+  return ((c * 0x9E3779B1u + key * 0x85EBCA6Bu) >> (33 - BITS)) << 1;
 }
 __device__ __forceinline__ bool memo_match(const uint4 &e, unsigned c, unsigned key) {
   return e.x == c && ((e.w ^ key) & kKeyMask) == 0u;

@@ -10,13 +10,15 @@
 // the lanes look at together.  What is single-stepped instead: visits during
 // which a stage start could fall (the ones outside the word must then number
 // exactly the block's cells outside it), visits that the step limit would cut,
-// words outside the window or past an allowed cell.
+// words with a cell that is not allowed.
 //
-// Bound by the latency of one chain, about 200 cycles a visit; a survivor's
-// 13 million steps to stage 12 are about 60,000 visits and sweeps.  One B200,
-// one lane per machine before, one warp now: recheck of 61 survivors to stage
-// 12 364 -> 11 ms, of 2868 to stage 15 66 -> 17 s, check.py on 8 survivors 524
-// -> 9.5 ms.  A machine
+// Bound by the number of instructions of one chain, 200-250 cycles a visit; a
+// survivor's 13 million steps to stage 12 are about 60,000 visits and sweeps.
+// One B200, one lane per machine before, one warp now: recheck of 61 survivors
+// to stage 12 357 -> 6.8 ms, check.py on 8 survivors 580 -> 4.1 ms.  Words in
+// device memory have a path of their own, some 600 cycles a visit: a survivor
+// that zigzags 16,000 cells beyond the window for 1.3e8 steps took 31 s with a
+// lane, 13.9 with a warp that single-steps there, 1.7 with this path.  A machine
 // whose configuration repeats (inside one word, or inside three words that it
 // has not left since) turns until its limit: whole turns are left out.
 #pragma once
@@ -29,6 +31,10 @@ typedef long long wi64;
 constexpr int kWalkLeft = 4096;                       // the window starts at cell -4096
 constexpr int kWalkZero = kWalkLeft >> 5;             // its word of cell 0
 constexpr unsigned kBlockBits = 0xC0000000u;          // cells -2, -1 in the word before it
+// Visits remembered.  More of them cost nothing where every machine has an SM
+// to itself, and fewer are made again: 512 -> 1024 took recheck of 61 survivors
+// from 7.6 to 6.6 ms and check.py on 8 from 4.2 to 3.6; 2048 gave 6.5 and 3.6.
+constexpr int kWalkMemoBits = 10;
 constexpr int kWalkWatch = 512;                       // visits between looks for a repeated configuration,
 constexpr int kWalkWatchFor = 64;                     // each of this many visits
 
@@ -97,8 +103,8 @@ __device__ __forceinline__ int walk_run(const WalkTape &T, uint4 *memo, const ui
   int head = W.head, ones = W.ones, minhead = W.minhead;
   wi64 left = W.left;
   int b = walk_word(head);
-  const int b_lo = max((lo + kWalkLeft + 31) >> 5, 0);
-  const int b_hi = min(((hi + 1 + kWalkLeft) >> 5) - 1, T.W - 1);
+  const int a_lo = (lo + kWalkLeft + 31) >> 5, a_hi = ((hi + 1 + kWalkLeft) >> 5) - 1;  // words of allowed cells
+  const int b_lo = max(a_lo, 0), b_hi = min(a_hi, T.W - 1);                             // ... in the window
   const int w1 = walk_word(S.want1), w2 = walk_word(S.want2);
   const int t1 = __popc(walk_block(w1, S.size)), t2 = __popc(walk_block(w2, S.size));
   const int q0 = (head + kWalkLeft) & 31;
@@ -119,7 +125,7 @@ __device__ __forceinline__ int walk_run(const WalkTape &T, uint4 *memo, const ui
       do {
         in_range = b >= b_lo && b <= b_hi;
         c = T.win[in_range ? b : 0];
-        slot = memo + memo_slot(c, key);
+        slot = memo + memo_slot<kWalkMemoBits>(c, key);
         e = *slot;
         n = memo_steps(e);
         const unsigned mask = walk_mask(b);
@@ -152,6 +158,37 @@ __device__ __forceinline__ int walk_run(const WalkTape &T, uint4 *memo, const ui
       } else if (!ok) {
         if (in_range && clear && !memo_match(e, c, key)) {
           single = memo_steps(memo_fetch<false, true>(slot, e, act, c, key, lane)) == 0;
+        } else if (!in_range && b >= a_lo && b <= a_hi) {
+          // a word in device memory: the same rules, one visit or sweep
+          --count;
+          c = T.ld(b);
+          slot = memo + memo_slot<kWalkMemoBits>(c, key);
+          e = *slot;
+          if (!memo_match(e, c, key)) e = memo_fetch<false, true>(slot, e, act, c, key, lane);
+          n = memo_steps(e);
+          const unsigned mask = walk_mask(b);
+          const int was = __popc(c & mask);
+          single = n == 0 || (wi64)n > left || (b == w1 && ones - was == S.size - t1) ||
+                   (b == w2 && ones - was == S.size - t2);
+          if (!single) {
+            const int dir = key_dir(key);
+            int run = 1;
+            if (e.z == c && memo_next(e) == key) {
+              const int w = b + dir * lane;
+              const bool same = w >= a_lo && w <= a_hi && (unsigned)w >= (unsigned)T.W &&
+                                (w == b || (w != w1 && w != w2)) && T.ld(w) == c;
+              const unsigned m = __ballot_sync(kAll, !same);
+              run = m ? __ffs(m) - 1 : 32;
+              if ((wi64)run * n > left) run = 1;
+            } else {
+              T.st(b, e.z);
+              ones += __popc(e.z & mask) - was;
+            }
+            left -= (wi64)run * n;
+            minhead = min(minhead, 32 * (dir < 0 ? b - run + 1 : b) - kWalkLeft + memo_lowest(e));
+            b += run > 1 ? dir * run : memo_move(e);
+            key = memo_next(e);
+          }
         } else {
           single = true;
         }
@@ -160,19 +197,19 @@ __device__ __forceinline__ int walk_run(const WalkTape &T, uint4 *memo, const ui
         if ((unsigned)(b - snap_b + 1) > 2u) far = true;
         if (count <= 0) {
           if (watch == 0) {  // a snapshot, and a look after each of the next visits
-            if (b > b_lo && b < b_hi) {
+            if (b > a_lo && b < a_hi) {
               snap_b = b;
               snap_key = key;
               snap_left = left;
-              snap0 = T.win[b - 1];
-              snap1 = T.win[b];
-              snap2 = T.win[b + 1];
+              snap0 = T.ld(b - 1);
+              snap1 = T.ld(b);
+              snap2 = T.ld(b + 1);
               far = false;
             }
             watch = kWalkWatchFor;
           } else {
-            if (!far && b == snap_b && key == snap_key && T.win[b] == snap1 && T.win[b - 1] == snap0 &&
-                T.win[b + 1] == snap2) {
+            if (!far && b == snap_b && key == snap_key && T.ld(b) == snap1 && T.ld(b - 1) == snap0 &&
+                T.ld(b + 1) == snap2) {
               left %= snap_left - left;
               far = true;
             }

@@ -48,3 +48,27 @@ def test_random_machines_equal_oracle(nq, nmax, mode):
                 assert got == counters[n - 1], (line, n)
         else:
             assert E.format_deep(ci, o, nmax) == O.deep_line(line, nmax), line
+
+
+@pytest.mark.parametrize("nq,nmax", [(3, 1), (4, 2), (5, 3)])
+def test_words_beyond_the_window_equal_oracle(nq, nmax):
+    """Stage 1 may take 100,000 steps: many of these machines sweep, zigzag or
+    shift past the window's ends (cells -4096 and 2^nmax + 4096)."""
+    lines = random_lines(600, nq, 7 * nq)
+    outs = ctx().check([E.parse_survivor_line(l) for l in lines], nmax, 0)
+    assert sum(abs(o.fail_head) > 4096 + (1 << nmax) for o in outs) >= 30
+    for line, o in zip(lines, outs):
+        got, verdict = (v.split(" (c2 counter")[0] for v in (E.format_recheck(o, nmax), O.recheck_line(line, nmax)[1]))
+        assert got == verdict, line
+
+
+def test_runaway_survivor_equals_oracle():
+    """A survivor that leaves the block at stage 12 and zigzags 16,000 cells
+    beyond the window until its limit, 1.3e8 steps."""
+    line = ("SURVIVOR X=9 st0=2 head0=-2 abs=1 rel=0 steps=271500 table=1L1 1R0|1L2 1L1|1R3 0R0|0L6 0R4|0L3 1R5|0R1 1R4|"
+            "1R3 1L7|1L6 0L8|1L3 0L7|?0L10 ?1R9|?1R12 ?0L2|?0L12 ?---|?0R9 ?0L11")
+    (o,) = ctx().check([E.parse_survivor_line(line)], 12, 0)
+    ok, verdict, counters = O.recheck_line(line, 12)
+    assert E.format_recheck(o, 12) == verdict
+    for n in range(1, o.stages_done + 1):
+        assert "".join(f"{o.ones_cells[n][j]}," for j in range(min(o.nones[n], 64))) == counters[n - 1]

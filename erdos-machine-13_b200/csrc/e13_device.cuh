@@ -33,6 +33,9 @@ constexpr u32 kEntSpecial = 0xC0; // any of the above: leaves the fast path
 // state = this state, writes the symbol it reads), so the head sweeps a run of
 // that symbol; the step loop then advances over the run a word at a time.
 constexpr u32 kEntSelf = 0x100;
+// Bits 14 and 15: the head's move (01 right, 11 left), so that the sign-extended
+// slot shifted right by 14 is +-1.  Set for every entry; not in saved files.
+constexpr u32 kSlotRight = 0x4000, kSlotLeft = 0xC000, kSlotSaved = 0x1FF;
 
 // Node flags byte.
 constexpr int kFlagAbs = 1, kFlagRel = 2, kFlagCs0 = 4, kFlagKeep = 32;
@@ -49,7 +52,7 @@ struct __align__(16) Node {
   short p0, pend;
   unsigned char nintro, budget, job, pad1;  // job: the slot of the search this machine belongs to
   u32 pad2[3];
-  unsigned short cellv[32];  // cell entries with the self-loop bit; row s = cellv[2s] | cellv[2s+1] << 16
+  unsigned short cellv[32];  // cell slots (cell_slot); row s = cellv[2s] | cellv[2s+1] << 16
   u32 tape[kTapeWords];
   u32 pad3;
 };
@@ -336,40 +339,73 @@ __device__ __forceinline__ int lane_act(Lane &L, u32 *__restrict__ tcol, const u
   return 0;
 }
 
+// The slot of symbol sym in a row of two, sign extended: its move is then
+// slot >> 14.
+__device__ __forceinline__ int row_slot(u32 row, u32 sym) {
+  int e;
+  asm("prmt.b32 %0, %1, 0, %2;" : "=r"(e) : "r"(row), "r"(sym * 0x2222u + 0x9910u));
+  return e;
+}
+
 // N steps of a running lane whose table and tape columns are 32 words apart:
 // the persistent search's hot loop.  left: steps that still pass the deadline
-// test (deadline + 1 - t).  Two branches a step: one before it for what keeps
-// it from being taken (the deadline, a cell that is no plain move), one after
-// it for what it led to (out of the window, a match of the low hash halves).
-// Returns 0 (all N taken), or as lane_act.
+// test (deadline + 1 - t); row: 4 times the state.  Returns 0 (all N taken), or
+// as lane_act.
+//
+// Bound by issue slots (five in six are used, for 22 of 32 lanes), so what
+// counts is the instructions of a step:
+//  * the slot holds what a step needs as it is used: the head's move
+//    (kSlotRight), the next state as 4 times its number;
+//  * two branches a step: before it a cell that is no plain move, after it
+//    what it led to (out of the window, a match of the low hash halves);
+//  * the deadline is tested once for all N: a machine that met it on the way
+//    died there, whatever it did after.
+// Counter search / FMAX = 4 search of 1.8e8 machines, against the move made of
+// bit 1 and the deadline tested in every step: 703 -> 685 / 35.3 -> 33.8 ms.
+// Loading the one slot once the symbol is known, which saves the selection but
+// lengthens the chain, took 717 / 34.9.
 template <int N>
-__device__ __forceinline__ int lane_steps(Lane &L, int &left, u32 *__restrict__ tcol, const u32 *__restrict__ rcol,
-                                          const u32 *__restrict__ keyb, int &cell, u32 &ecell) {
+__device__ __forceinline__ int lane_steps(Lane &L, int &left, u32 &row, u32 *__restrict__ tcol,
+                                          const u32 *__restrict__ rcol, const u32 *__restrict__ keyb, int &cell,
+                                          u32 &ecell) {
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     const int p = L.p;
     u32 *const wp = tcol + ((p >> 5) << 5);
     const u32 word = *wp;
-    const u32 row = rcol[L.st << 5];
     const u32 kk = keyb[p];
+    const u32 r2 = rcol[row << 3];
     const u32 sym = (word >> (p & 31)) & 1u;
-    const u32 e = row >> (sym << 4);
-    if (((e & kEntSpecial) != 0u) | (left <= 0)) {
-      if (left <= 0) return kEvDead;
-      cell = (L.st << 1) | (int)sym;
-      ecell = e & 0xFFu;
+    const int e = row_slot(r2, sym);
+    if (e & (int)kEntSpecial) {
+      if (i >= left) {
+        left = 0;
+        return kEvDead;
+      }
+      left -= i;
+      cell = (int)((row >> 1) | sym);
+      ecell = (u32)e & 0xFFu;
       return kEvCell;
     }
-    const u32 flip = (e ^ sym) & 1u;
+    const u32 flip = ((u32)e ^ sym) & 1u;
     *wp = word ^ (flip << (p & 31));
     L.hb ^= kk & (0u - flip);
-    L.p = p + (int)(e & 2u) - 1;
+    L.p = p + (e >> 14);
+    row = (u32)e & 0x3Cu;
     const bool in = (unsigned)(L.p - 1) < (unsigned)(kTapeCells - 2);
-    L.st = (int)((e >> 2) & 15u);
-    left -= in ? 1 : 0;
-    if (!in | (L.hb == L.tgt)) return in ? kEvStage : kEvDead;  // head <= -64 or >= 1299
+    if (!in | (L.hb == L.tgt)) {  // head <= -64 or >= 1299
+      if (i >= left) {
+        left = 0;
+        return kEvDead;
+      }
+      left -= in ? i + 1 : i;
+      return in ? kEvStage : kEvDead;
+    }
   }
-  return 0;
+  left -= N;
+  if (left >= 0) return 0;
+  left = 0;
+  return kEvDead;
 }
 
 // Counter hash from the tape: XOR of the keys of the ones at cells < -2
@@ -448,11 +484,12 @@ __device__ __forceinline__ u32 get_entry(const u32 *rcol, int stride, int cell) 
   return (rcol[(cell >> 1) * stride] >> ((cell & 1) << 4)) & 0xFFu;
 }
 
-// The 16-bit slot of a cell holding entry v, with the self-loop bit when
-// run_skip is on and v is a read move that keeps the state and the symbol.
+// The 16-bit slot of a cell holding entry v, with its move and with the
+// self-loop bit when run_skip is on and v is a read move that keeps the state
+// and the symbol.
 __host__ __device__ __forceinline__ u32 cell_slot(int cell, u32 v, bool run_skip) {
   const bool self = run_skip && v < 64u && (int)(v >> 2) == (cell >> 1) && (int)(v & 1u) == (cell & 1);
-  return v | (self ? kEntSelf : 0u);
+  return v | (self ? kEntSelf : 0u) | ((v & 2u) ? kSlotRight : kSlotLeft);
 }
 
 __device__ __forceinline__ void set_entry(u32 *rcol, int stride, int cell, u32 v, bool run_skip) {

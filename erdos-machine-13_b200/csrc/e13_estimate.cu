@@ -35,7 +35,7 @@ namespace {
 
 constexpr unsigned kFull = 0xFFFFFFFFu;
 constexpr int kEstBlock = 256;
-constexpr int kYoungIterations = 56;  // iterations of three steps: 168 steps
+constexpr int kYoungIterations = 28;  // iterations of six steps: 168 steps
 
 enum { kPrIdle = 0, kPrRun = 1, kPrFork = 2, kPrDead = 3, kPrSurv = 4 };
 
@@ -53,7 +53,7 @@ __device__ __forceinline__ u64 mix_next(u64 &s) {
 // every first read is a fork, as in run() with fixed[i] == 0.
 __device__ __forceinline__ void run_to_event(Lane &L, int &status, int &fork_cell, u32 &fork_e, u32 *tcol,
                                              const u32 *rcol, const KeyTabs &K) {
-  // most children stop within two deadlines (153 steps): single steps, three
+  // most children stop within two deadlines (153 steps): single steps, six
   // an iteration; the ones that go on cross runs a tape word at a time
   for (int it = 0; __any_sync(kFull, status == kPrRun); ++it) {
     if (status == kPrRun) {
@@ -61,8 +61,10 @@ __device__ __forceinline__ void run_to_event(Lane &L, int &status, int &fork_cel
       u32 e = 0;
       if (it < kYoungIterations) {
         int left = L.deadline + 1 - L.t;
-        ev = lane_steps<3>(L, left, tcol, rcol, K.lo, cell, e);
+        u32 row = (u32)L.st << 2;
+        ev = lane_steps<6>(L, left, row, tcol, rcol, K.lo, cell, e);
         L.t = L.deadline + 1 - left;
+        L.st = (int)(row >> 2);
       } else {
         ev = lane_act<true>(L, tcol, rcol, K, 32, cell, e);
       }

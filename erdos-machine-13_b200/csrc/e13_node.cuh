@@ -127,7 +127,8 @@ static inline void build_root(const e13_job *job, int slot, Node *root, bool run
       else if (c < 0) e = (unsigned char)(kEntUnread | kEntHalt);
       else e = (unsigned char)(((clear && job->budget <= 0) ? 0u : kEntUnread) | (unsigned)c);
     }
-    root->cellv[i] = (unsigned short)(e < 64u || (e & 0xC0u) == kEntUnread ? cell_slot(i, e & 0x3Fu, run_skip) | (e & kEntUnread) : e);
+    root->cellv[i] = (unsigned short)(e < 64u || (e & 0xC0u) == kEntUnread ? cell_slot(i, e & 0x3Fu, run_skip) | (e & kEntUnread)
+                                                                                   : cell_slot(i, e, false));
   }
 }
 

@@ -65,12 +65,20 @@ constexpr long long kMinEpochNs = 200000;        // 200 us: the shortest epoch a
 // the counter search takes 706 ms instead of 731.)
 constexpr int kLoneLanes = 2;
 constexpr int kLoneSteps = 512;
-// Persistent kernel: steps of a slice iteration.  With the default slice of 24
-// iterations a warp refills every 72 steps, and most machines die at a deadline,
-// after 73 or 153 steps.  Counter search / FMAX = 4 search of 1.8e8 machines:
-// 2 steps 749 / 53.4 ms, 3 steps 706 / 51.1, 4 steps 787 / 56.3 (739 / 51.8 with a
-// slice of 20).
-constexpr int kSteps = 3;
+// Persistent kernel: steps of a slice iteration, and the running lanes below
+// which a slice ends (or the first lane to stop ends it, if fewer ran at its
+// start).  A lane that stops waits for the iteration's end, and the loop and
+// the event dispatch are paid per iteration.  Counter search / FMAX = 4 search of
+// 1.8e8 machines / a quarter of the FMAX = 4 job: slices of 72 steps (most
+// machines die after 73 or 153), 2 steps an iteration 729 / 35.8 / 169 ms,
+// 3 steps 685 / 33.6 / 160, 6 steps 648 / 31.8 / 149, 9 steps 645 / 31.1 / 148,
+// 12 steps 652 / 31.4 / 147, 24 steps 748 / 35.4 / 163.  With 9 steps and slices
+// that go on, to 216 steps at most, while 16 lanes run: 589 / 31.5 / 142 (20
+// lanes 593 / 30.6 / 146, 24 lanes 616 / 32.7 / 152).
+// While warps wait for work slices stay at 72 steps: with 216 some counter
+// neighbourhoods took a second epoch, 4.8 instead of 3.2 ms.
+constexpr int kSteps = 9;
+constexpr int kLeastLanes = 16;
 
 // Long machines.  In lock-step a long machine costs a lane 0.3 us a step; alone
 // in a warp of long_kernel (e13_macro.cuh) one of 835,000 steps takes 1.5-3 ms,
@@ -719,8 +727,13 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
       st_lane_rounds += __popc(rm);
       if (rm) {
         int left = L.deadline + 1 - L.t;
+        u32 row = (u32)L.st << 2;
+        // (a warp with idle lanes takes up new machines; a starving one has
+        // forks that others wait for)
+        const int least = min(kLeastLanes, __popc(rm)), most = PERSIST && starving ? (P.slice + 2) / 3 : P.slice;
 #pragma unroll 1
-        for (int it = 0; it < P.slice; ++it) {
+        for (int it = 0; it < most; ++it) {
+          if (PERSIST && it > 0 && __popc(__ballot_sync(kFull, status == kStRun)) < least) break;
           if (status == kStRun) {
             int cell = 0;
             u32 e = 0;
@@ -728,7 +741,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
             // the event dispatch below are paid once for all
             int ev;
             if (PERSIST) {
-              ev = lane_steps<kSteps>(L, left, tcol, rcol, K.lo, cell, e);
+              ev = lane_steps<kSteps>(L, left, row, tcol, rcol, K.lo, cell, e);
             } else if (lone_w) {
               // the same steps and events as lane_act (step_slice follows
               // src/e13search.c:134-177 too); a hash match ends the iteration
@@ -747,7 +760,10 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
             // lane_act: one copy of it in the loop instead of one per
             // inlined action (the second action waits for it)
             if (ev == kEvStage) {
-              if (PERSIST) L.t = L.deadline + 1 - left;
+              if (PERSIST) {
+                L.t = L.deadline + 1 - left;
+                L.st = (int)(row >> 2);
+              }
               ev = stage_check(L, tcol, K, stride);
               left = L.deadline + 1 - L.t;
             }
@@ -781,7 +797,10 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
           // of the if-blocks above, so the next action issues once for the
           // whole warp
         }
-        if (PERSIST) L.t = L.deadline + 1 - left;
+        if (PERSIST) {
+          L.t = L.deadline + 1 - left;
+          L.st = (int)(row >> 2);
+        }
         if (__any_sync(kFull, status >= kStDead)) {
           if (status >= kStDead) {
             acc_steps += (u32)(L.t - L.tseg);
@@ -1698,6 +1717,8 @@ int ckpt_save(e13_ctx *c, const e13_job *job, const e13_checkpoint *ck, int slot
       fclose(f);
       return E13_ERR_CUDA;
     }
+    for (long long k = 0; k < n; ++k)
+      for (unsigned short &v : buf[(size_t)k].cellv) v &= kSlotSaved;
     if (!write_all(f, buf.data(), sizeof(Node) * (size_t)n)) {
       fclose(f);
       return E13_ERR_IO;
@@ -1786,6 +1807,9 @@ int ckpt_load(e13_ctx *c, const e13_job *job, const e13_checkpoint *ck, long lon
       fclose(f);
       return E13_ERR_CKPT;
     }
+    for (long long k = 0; k < n; ++k)
+      for (unsigned short &v : buf[(size_t)k].cellv)
+        v = (unsigned short)((v & kSlotSaved) | ((v & 2u) ? kSlotRight : kSlotLeft));
     if (h2d(c, c->stack + o, buf.data(), sizeof(Node) * n) !=
             cudaSuccess ||
         cudaStreamSynchronize(c->stream) != cudaSuccess) {
@@ -1851,7 +1875,7 @@ struct ShardKey {
 static ShardKey shard_key(const Node &n) {
   ShardKey k;
   memset(&k, 0, sizeof k);
-  memcpy(k.cellv, n.cellv, sizeof k.cellv);
+  for (int i = 0; i < 32; ++i) k.cellv[i] = n.cellv[i] & kSlotSaved;  // the order that saved searches were dealt in
   k.t = n.t;
   k.p = n.p;
   k.st = n.st;

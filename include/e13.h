@@ -89,9 +89,10 @@ enum {
 typedef struct e13_tuning {
   int32_t kernel;            /* E13_KERNEL_* */
   int32_t block;             /* lanes (threads) per CTA: 64..768, multiple of 32 */
-  int32_t slice;             /* iterations per round between warp-level refills; each iteration takes up
-                                to three steps (persistent) or two actions (plain: a step or a run skip)
-                                per lane */
+  int32_t slice;             /* most iterations per round between warp-level refills; each iteration takes
+                                up to nine steps (persistent: a round ends earlier when many lanes have
+                                stopped, and at a third of the iterations while warps wait for work) or
+                                two actions (plain: a step or a run skip) per lane */
   int32_t warp_stack;        /* nodes in each warp's private DFS stack (persistent) */
   int32_t step_cap;          /* plain kernel: steps per work item before it is requeued */
   int32_t batch;             /* nodes taken from the frontier per launch / epoch (0 = auto: the whole

@@ -35,3 +35,18 @@ def test_long_machines_equal_oracle(searches, name, X, tune):
     c, surv = ctx().search(job, E.tuning(**tune))
     assert c.as_dict() == exp
     assert sorted(E.survivor_line(job, s) for s in surv) == sorted(O.survivor_line(X, r, jo.nq) for r in recs)
+
+
+@pytest.mark.parametrize("block,slice_", [(768, 1), (768, 2), (768, 8), (64, 17), (32 * 21, 4096)])
+@pytest.mark.parametrize("name,X", [("local_edits_f2", 11), ("counters_f2_base_11", -1)])
+def test_slices_equal_oracle(searches, name, X, block, slice_):
+    """Slices of one iteration of several steps, of the shortest one that
+    starving warps shorten, and ones that end because lanes have stopped: every
+    deadline and event falls on some step of an iteration."""
+    e = searches[name]
+    job = make_job(e, X)
+    _, jo = O.setup(O.load_machine(e["machine"]), X, fmax=e["fmax"], free_cells=None)
+    exp, recs = O.search(jo)
+    c, surv = ctx().search(job, E.tuning(block=block, slice=slice_))
+    assert c.as_dict() == exp
+    assert sorted(E.survivor_line(job, s) for s in surv) == sorted(O.survivor_line(X, r, jo.nq) for r in recs)

@@ -89,7 +89,7 @@ constexpr int kLeastLanes = 16;
 // never worth it: with 512 the FMAX = 3 search of X = 8 took 28 ms, with 1536
 // 18 ms, everything else equal).
 // The counter neighbourhoods (FMAX = 2, 61 machines) went from 20-240 ms to
-// 8-12 ms, their tails being in-place loops and zigzag sweeps to the deadline.
+// 3-5 ms, their tails being in-place loops and zigzag sweeps to the deadline.
 constexpr int kLongCap = 1 << 14;        // machines handed over per epoch, at most
 constexpr int kLongNodes = 1 << 14;      // fork nodes long_kernel keeps for its own queue
 constexpr int kLongItems = 1 << 15;      // children it queues
@@ -98,12 +98,12 @@ constexpr int kLongOut = kLongCap + kLongItems;  // most nodes it puts on the ou
 // visit made again costs its steps, and that counts for more than warps.
 // FMAX = 3 searches of three machine families, with 512 visits and 16 warps
 // 8.3, 2.9, 6.8 ms, with 1024 and 8 warps 7.2, 2.3, 6.3, with 2048 and 6 warps
-// 6.7, 2.2, 5.8; tables of 20,000 machines 3.9, 3.5, 3.1.
+// 6.7, 2.2, 5.8; tables of 20,000 machines 3.9, 3.5, 3.1 ms.
 constexpr int kLongMemoBits = 11;
 constexpr int kLongBlock = 192;
 constexpr int kLongPerSm = 1;
 constexpr long long kLongMinNs = 1000000;  // shortest time bound of long_kernel: 1 ms (else a tenth of the epoch)
-constexpr int kIdlePark = 8;             // many warps wait: an eighth
+constexpr int kIdlePark = 8;             // many warps wait: more than an eighth
 constexpr int kParkMin = 1536;
 constexpr int kNeverPark = 0x7FFFFFFF;
 // Taking input and pool nodes.  One word of L2 takes an atomic or a polling

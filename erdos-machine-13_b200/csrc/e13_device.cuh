@@ -34,8 +34,12 @@ constexpr u32 kEntSpecial = 0xC0; // any of the above: leaves the fast path
 // that symbol; the step loop then advances over the run a word at a time.
 constexpr u32 kEntSelf = 0x100;
 // Bits 14 and 15: the head's move (01 right, 11 left), so that the sign-extended
-// slot shifted right by 14 is +-1.  Set for every entry; not in saved files.
-constexpr u32 kSlotRight = 0x4000, kSlotLeft = 0xC000, kSlotSaved = 0x1FF;
+// slot shifted right by 14 is +-1; bit 13: the symbol is flipped.  Of use in the
+// slots of moves only, and not in saved files (kSlotSaved).
+constexpr u32 kSlotRight = 0x4000, kSlotLeft = 0xC000, kSlotFlip = 0x2000, kSlotSaved = 0x1FF;
+__host__ __device__ __forceinline__ u32 slot_move(int cell, u32 v) {
+  return ((v & 2u) ? kSlotRight : kSlotLeft) | (((v ^ (u32)cell) & 1u) ? kSlotFlip : 0u);
+}
 
 // Node flags byte.
 constexpr int kFlagAbs = 1, kFlagRel = 2, kFlagCs0 = 4, kFlagKeep = 32;
@@ -339,11 +343,11 @@ __device__ __forceinline__ int lane_act(Lane &L, u32 *__restrict__ tcol, const u
   return 0;
 }
 
-// The slot of symbol sym in a row of two, sign extended: its move is then
-// slot >> 14.
-__device__ __forceinline__ int row_slot(u32 row, u32 sym) {
+// The slot of the symbol read (one: it is 1) in a row of two, sign extended:
+// its move is then slot >> 14.
+__device__ __forceinline__ int row_slot(u32 row, bool one) {
   int e;
-  asm("prmt.b32 %0, %1, 0, %2;" : "=r"(e) : "r"(row), "r"(sym * 0x2222u + 0x9910u));
+  asm("prmt.b32 %0, %1, 0, %2;" : "=r"(e) : "r"(row), "r"(one ? 0xBB32u : 0x9910u));
   return e;
 }
 
@@ -353,58 +357,65 @@ __device__ __forceinline__ int row_slot(u32 row, u32 sym) {
 // as lane_act.
 //
 // Bound by issue slots (five in six are used, for 22 of 32 lanes), so what
-// counts is the instructions of a step:
-//  * the slot holds what a step needs as it is used: the head's move
-//    (kSlotRight), the next state as 4 times its number;
-//  * two branches a step: before it a cell that is no plain move, after it
-//    what it led to (out of the window, a match of the low hash halves);
+// counts is the instructions of a step, about 24:
+//  * the slot holds what a step needs as it is used: the head's move and
+//    whether it writes (kSlotRight, kSlotFlip), the next state as 4 times its
+//    number;
+//  * one branch a step, for what the last step led to (out of the window, a
+//    match of the low hash halves) and for a cell that is no plain move: the
+//    loads of the step go out before it;
 //  * the deadline is tested once for all N: a machine that met it on the way
 //    died there, whatever it did after.
-// Counter search / FMAX = 4 search of 1.8e8 machines, against the move made of
-// bit 1 and the deadline tested in every step: 703 -> 685 / 35.3 -> 33.8 ms.
+// Counter search / FMAX = 4 search of 1.8e8 machines: the move made of bit 1 and
+// the deadline tested in every step 703 / 35.3 ms, the move in the slot and one
+// deadline test 685 / 33.8; with 9 steps an iteration 588 / 31.8, and with one
+// branch and the flip in the slot 539 / 29.4.
 // Loading the one slot once the symbol is known, which saves the selection but
-// lengthens the chain, took 717 / 34.9.
+// lengthens the chain, took 717 / 34.9 where this took 685 / 33.8.
 template <int N>
 __device__ __forceinline__ int lane_steps(Lane &L, int &left, u32 &row, u32 *__restrict__ tcol,
                                           const u32 *__restrict__ rcol, const u32 *__restrict__ keyb, int &cell,
                                           u32 &ecell) {
+  bool stop = false;  // the last step left the window or led to a match
 #pragma unroll
-  for (int i = 0; i < N; ++i) {
+  for (int i = 0; i <= N; ++i) {
     const int p = L.p;
     u32 *const wp = tcol + ((p >> 5) << 5);
-    const u32 word = *wp;
-    const u32 kk = keyb[p];
-    const u32 r2 = rcol[row << 3];
-    const u32 sym = (word >> (p & 31)) & 1u;
-    const int e = row_slot(r2, sym);
-    if (e & (int)kEntSpecial) {
-      if (i >= left) {
-        left = 0;
-        return kEvDead;
+    u32 word = 0, kk = 0, m = 0;
+    int e = 0;
+    if (i < N) {
+      word = *wp;  // (a head outside the window is on its first or last cell)
+      kk = keyb[p];
+      m = 1u << (p & 31);
+      e = row_slot(rcol[row << 3], (word & m) != 0u);
+    }
+    if (stop | ((e & (int)kEntSpecial) != 0)) {
+      const int taken = stop ? i - 1 : i;
+      if (taken >= left) break;
+      left -= taken;
+      if (stop) {
+        const bool in = (unsigned)(p - 1) < (unsigned)(kTapeCells - 2);  // not: head <= -64 or >= 1299
+        left -= in ? 1 : 0;
+        return in ? kEvStage : kEvDead;
       }
-      left -= i;
-      cell = (int)((row >> 1) | sym);
+      cell = (int)(row >> 1) | ((word & m) != 0u ? 1 : 0);
       ecell = (u32)e & 0xFFu;
       return kEvCell;
     }
-    const u32 flip = ((u32)e ^ sym) & 1u;
-    *wp = word ^ (flip << (p & 31));
-    L.hb ^= kk & (0u - flip);
+    if (i == N) {
+      left -= N;
+      if (left >= 0) return 0;
+      break;
+    }
+    if (e & (int)kSlotFlip) {
+      *wp = word ^ m;
+      L.hb ^= kk;
+    }
     L.p = p + (e >> 14);
     row = (u32)e & 0x3Cu;
-    const bool in = (unsigned)(L.p - 1) < (unsigned)(kTapeCells - 2);
-    if (!in | (L.hb == L.tgt)) {  // head <= -64 or >= 1299
-      if (i >= left) {
-        left = 0;
-        return kEvDead;
-      }
-      left -= in ? i + 1 : i;
-      return in ? kEvStage : kEvDead;
-    }
+    stop = ((unsigned)(L.p - 1) >= (unsigned)(kTapeCells - 2)) | (L.hb == L.tgt);
   }
-  left -= N;
-  if (left >= 0) return 0;
-  left = 0;
+  left = 0;  // it met its deadline on the way
   return kEvDead;
 }
 
@@ -489,7 +500,7 @@ __device__ __forceinline__ u32 get_entry(const u32 *rcol, int stride, int cell) 
 // and the symbol.
 __host__ __device__ __forceinline__ u32 cell_slot(int cell, u32 v, bool run_skip) {
   const bool self = run_skip && v < 64u && (int)(v >> 2) == (cell >> 1) && (int)(v & 1u) == (cell & 1);
-  return v | (self ? kEntSelf : 0u) | ((v & 2u) ? kSlotRight : kSlotLeft);
+  return v | (self ? kEntSelf : 0u) | slot_move(cell, v);
 }
 
 __device__ __forceinline__ void set_entry(u32 *rcol, int stride, int cell, u32 v, bool run_skip) {

@@ -56,7 +56,7 @@ __device__ u64 d_span[kSpans * kTapeWords];
 constexpr long long kPoolNodes = 1LL << 18;  // donation pool: 256 Ki nodes (80 MiB)
 constexpr long long kWholeFrontier = 1LL << 62;  // persistent batch when e13_tuning::batch is 0
 constexpr long long kPoolWaitNs = 200000000;     // 200 ms: a donor publishes a claimed slot within microseconds
-constexpr long long kMinEpochNs = 200000;        // 200 us: the shortest epoch a starvation dump may end
+constexpr long long kMinEpochNs = 150000;        // 150 us: the shortest epoch a starvation dump may end
 // Plain kernel: a warp with at most kLoneLanes running machines runs each of
 // them in the tight single-machine loop step_slice, up to kLoneSteps steps per
 // iteration: its speed is then bound by one machine's dependent chain, not by
@@ -87,7 +87,11 @@ constexpr int kLeastLanes = 16;
 // steps since its load, and while an eighth of the warps wait for work after
 // kParkMin (machines that die at the deadline of stage 4, 1137 steps, are
 // never worth it: with 512 the FMAX = 3 search of X = 8 took 28 ms, with 1536
-// 18 ms, everything else equal).
+// 18 ms, everything else equal).  A small search's first epoch ends after
+// kMinEpochNs to deal its work out; were a few machines handed over before
+// that, the kernel would run for their sake alone and again for the others:
+// counter neighbourhoods with 1536 steps and 200 us 3.0-7.0 ms, with 2048 or
+// with 150 us 2.9-5.2.
 // The counter neighbourhoods (FMAX = 2, 61 machines) went from 20-240 ms to
 // 3-5 ms, their tails being in-place loops and zigzag sweeps to the deadline.
 constexpr int kLongCap = 1 << 14;        // machines handed over per epoch, at most
@@ -104,7 +108,7 @@ constexpr int kLongBlock = 192;
 constexpr int kLongPerSm = 1;
 constexpr long long kLongMinNs = 1000000;  // shortest time bound of long_kernel: 1 ms (else a tenth of the epoch)
 constexpr int kIdlePark = 8;             // many warps wait: more than an eighth
-constexpr int kParkMin = 1536;
+constexpr int kParkMin = 2048;
 constexpr int kNeverPark = 0x7FFFFFFF;
 // Taking input and pool nodes.  One word of L2 takes an atomic or a polling
 // read at a time, so blocks claim input in chunks (at most kInputChunk nodes,
@@ -1808,8 +1812,10 @@ int ckpt_load(e13_ctx *c, const e13_job *job, const e13_checkpoint *ck, long lon
       return E13_ERR_CKPT;
     }
     for (long long k = 0; k < n; ++k)
-      for (unsigned short &v : buf[(size_t)k].cellv)
-        v = (unsigned short)((v & kSlotSaved) | ((v & 2u) ? kSlotRight : kSlotLeft));
+      for (int i = 0; i < 32; ++i) {
+        unsigned short &v = buf[(size_t)k].cellv[i];
+        v = (unsigned short)((v & kSlotSaved) | slot_move(i, v));
+      }
     if (h2d(c, c->stack + o, buf.data(), sizeof(Node) * n) !=
             cudaSuccess ||
         cudaStreamSynchronize(c->stream) != cudaSuccess) {
@@ -1848,9 +1854,12 @@ void ckpt_remove(const e13_checkpoint *ck) {
 struct CkptClock {
   const e13_checkpoint *ck;
   std::string stop_file;
-  double t_call, last_save, last_look;
+  double t_call, last_save, last_look, last_step;
   int due(double now) {
-    if (ck->stop_after_s > 0 && now - t_call >= ck->stop_after_s) return 2;
+    // the launch that would end past the limit is not started
+    const double step = now - last_step;
+    last_step = now;
+    if (ck->stop_after_s > 0 && now - t_call + step >= ck->stop_after_s) return 2;
     if (now - last_look >= 1.0) {
       last_look = now;
       if (file_exists(stop_file)) return 2;
@@ -2080,7 +2089,7 @@ static int search_impl(e13_ctx *c, const e13_job *job, const e13_tuning *tuning,
   double prior_wall = 0.0;
   int slot = 0;
   bool stopped = false;
-  CkptClock clk{ck, ck ? std::string(ck->path) + ".stop" : std::string(), t_call, t_call, t_call};
+  CkptClock clk{ck, ck ? std::string(ck->path) + ".stop" : std::string(), t_call, t_call, t_call, t_call};
   if (ck) {
     if (file_exists(clk.stop_file)) remove(clk.stop_file.c_str());  // left from the last clean stop
     if (file_exists(ck->path)) {
@@ -2088,6 +2097,7 @@ static int search_impl(e13_ctx *c, const e13_job *job, const e13_tuning *tuning,
       if ((rc = ckpt_load(c, job, ck, batch_max, cap - out_nodes, &loaded, &prior_wall))) return rc;
       slot = loaded ^ 1;
     }
+    clk.last_step = host_seconds();
   }
   auto checkpoint_step = [&](int &status) -> bool {  // true: leave the launch loop
     if (!ck || c->ctl_host->top == 0) return false;

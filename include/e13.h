@@ -217,7 +217,8 @@ typedef struct e13_checkpoint {
   const char *config;   /* identity of the run (the CLI passes its arguments); a checkpoint written
                            under another config, job or node format is refused: E13_ERR_CKPT */
   double interval_s;    /* seconds between checkpoints; <= 0: 1800 (the reference's E13_CKPT_SEC) */
-  double stop_after_s;  /* > 0: checkpoint and stop after this many seconds of this call */
+  double stop_after_s;  /* > 0: checkpoint and stop after this many seconds of this call: a launch that
+                           would end later, going by the last one, is not started (one always is) */
 } e13_checkpoint;
 
 /* e13_search that survives being stopped (replaces E13_CKPT / E13_CKPT_SEC /

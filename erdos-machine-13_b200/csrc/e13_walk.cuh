@@ -230,6 +230,25 @@ __device__ __forceinline__ int walk_run(const WalkTape &T, uint4 *memo, const ui
     far = true;
     int st = key_state(key);
     if (!inside) head = 32 * b - kWalkLeft + key_bit(key);
+    if (head < lo || head > hi) {
+      // beyond the allowed cells, and perhaps beyond the tape: its word is not
+      // touched (check.py's allowed cells fill its tape exactly)
+      int ev = kWalkRange;
+      if (!CRAFT) {
+        if (ones == S.size && (S.any || (st == S.st && (head == S.want1 || head == S.want2))) &&
+            walk_block_set(T, S.size, lane))
+          ev = kWalkStop;
+        else if (left <= 0)
+          ev = kWalkLimit;
+      }
+      __syncwarp();
+      W.head = head;
+      W.st = st;
+      W.ones = ones;
+      W.minhead = minhead;
+      W.left = left;
+      return ev;
+    }
     unsigned word = T.ld(b);
     const int first = 32 * b - kWalkLeft;
     unsigned lw = 0;  // a configuration inside this word seen earlier

@@ -59,6 +59,13 @@ __device__ __forceinline__ unsigned long long macro_clock() {
   return t;
 }
 
+// By the whole warp: has the clock passed t_end?  Lanes read clocks of their
+// own, which may differ, and all take the way that follows from the answer: it
+// is lane 0's.
+__device__ __forceinline__ bool macro_late(unsigned long long t_end) {
+  return __shfl_sync(kAll, macro_clock() > t_end ? 1 : 0, 0) != 0;
+}
+
 // After a change of M.rows: the expanded table, and an empty memory of visits.
 template <int BITS>
 __device__ __forceinline__ void macro_table(MacroMem<BITS> &M, int lane) {
@@ -235,7 +242,8 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem<BITS> &M, co
       if (!HASH && --visits_left <= 0) {
         // visits that cost more than the steps they take: over to the window
         const long long now = clock64();
-        if (now - yield_clock > (long long)kStepCycles * (yield_left - left)) {
+        // (lane 0's clock decides, as in macro_late)
+        if (__shfl_sync(kAll, now - yield_clock > (long long)kStepCycles * (yield_left - left) ? 1 : 0, 0)) {
           single = true;
           window_left = kWindowSteps;
         }
@@ -244,7 +252,7 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem<BITS> &M, co
         visits_left = kYieldEvery;
       }
       noted = 0;
-      if (HASH && macro_clock() > t_end) {
+      if (HASH && macro_late(t_end)) {
         L.p = b * 32 + key_bit(key);
         L.st = key_state(key);
         L.t = L.deadline + 1 - left;
@@ -316,7 +324,7 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem<BITS> &M, co
       snap1 = M.tape[b];
       snap2 = M.tape[b + 1];
       far = false;
-      if (HASH && macro_clock() > t_end) {
+      if (HASH && macro_late(t_end)) {
         L.p = p;
         L.st = st;
         L.t = L.deadline + 1 - left;

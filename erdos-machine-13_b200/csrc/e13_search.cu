@@ -1020,7 +1020,7 @@ __global__ void __launch_bounds__(kLongBlock) long_kernel(const __grid_constant_
     // ---- run it
     int ev = kEvRun, cell = 0;
     u32 ecell = 0, reads = 0;
-    while (macro_clock() <= t_end) {
+    while (!macro_late(t_end)) {
       ev = macro_run<true>(L, hb, M, K, span, lane, reads, cell, ecell, t_end);
       if (ev != kEvCell) break;
       if (ecell == kEntHalt) {

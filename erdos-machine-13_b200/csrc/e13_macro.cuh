@@ -120,6 +120,7 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem<BITS> &M, co
         c = M.tape[b];
         slot = M.memo + memo_slot<BITS>(c, key);
         e = *slot;
+        __syncwarp();  // every lane has read the word (here: while the loads are under way)
         n = memo_steps(e);
         in_range = (unsigned)(b - 1) < (unsigned)(kLastWord - 1);
         ok = in_range && memo_match(e, c, key) && n - 1u < (u32)left;
@@ -332,7 +333,8 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem<BITS> &M, co
       }
     }
     u32 word = M.tape[b];
-    u32 lw = 0;  // a configuration inside this word seen earlier
+    __syncwarp();  // every lane has read the word (and its neighbours, above) before one writes it
+    u32 lw = 0;    // a configuration inside this word seen earlier
     int lat = -1, lleft = 0, lk = 0, lnext = 32, ev = -1;
     do {
       if (left <= 0) {
@@ -373,6 +375,7 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem<BITS> &M, co
         L.t = L.deadline + 1 - left;
         const int nt = L.nt;
         ev = stage_check(L, M.tape, K, 1);
+        __syncwarp();  // every lane has read the tape
         if (ev) break;
         ev = -1;
         if (L.nt != nt) {

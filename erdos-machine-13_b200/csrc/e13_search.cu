@@ -562,6 +562,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
             }
             h = __shfl_sync(kFull, h, 0);
             if (__shfl_sync(kFull, inc, 0)) busy = true;
+            __syncwarp();  // the slot's mark, which lane 0 read, before the node
             if (h >= 0) {
               src = P.pool + h;
               from_pool = true;
@@ -969,6 +970,7 @@ __global__ void __launch_bounds__(kLongBlock) long_kernel(const __grid_constant_
     if (stop) break;
     k = __shfl_sync(kFull, k, 0);
     child = __shfl_sync(kFull, child, 0);
+    __syncwarp();  // the item, which lane 0 read, before the node
     if (k < 0) {
       __nanosleep(backoff);
       backoff = backoff < 2048 ? 2 * backoff : 2048;
@@ -1064,6 +1066,8 @@ __global__ void __launch_bounds__(kLongBlock) long_kernel(const __grid_constant_
           slot = __shfl_sync(kFull, slot, 0);
           at = __shfl_sync(kFull, at, 0);
           if (slot < 0) break;  // no room or no time: the whole fork goes to the frontier
+          __syncwarp();
+          __threadfence();  // the node, which lane 0 wrote, before the items that name it
           for (int i = lane; i < rest; i += 32) {
             *((volatile unsigned long long *)&P.long_items[at + i]) =
                 ((unsigned long long)tag << 32) | ((unsigned long long)slot << 8) | (unsigned)nth_bit64(vm, i);

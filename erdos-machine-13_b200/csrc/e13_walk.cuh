@@ -127,6 +127,7 @@ __device__ __forceinline__ int walk_run(const WalkTape &T, uint4 *memo, const ui
         c = T.win[in_range ? b : 0];
         slot = memo + memo_slot<kWalkMemoBits>(c, key);
         e = *slot;
+        __syncwarp();  // every lane has read the word (here: while the loads are under way)
         n = memo_steps(e);
         const unsigned mask = walk_mask(b);
         const int was = __popc(c & mask);
@@ -181,6 +182,7 @@ __device__ __forceinline__ int walk_run(const WalkTape &T, uint4 *memo, const ui
               run = m ? __ffs(m) - 1 : 32;
               if ((wi64)run * n > left) run = 1;
             } else {
+              __syncwarp();
               T.st(b, e.z);
               ones += __popc(e.z & mask) - was;
             }
@@ -250,6 +252,7 @@ __device__ __forceinline__ int walk_run(const WalkTape &T, uint4 *memo, const ui
       return ev;
     }
     unsigned word = T.ld(b);
+    __syncwarp();  // every lane has read the word
     const int first = 32 * b - kWalkLeft;
     unsigned lw = 0;  // a configuration inside this word seen earlier
     int lat = -1, lk = 0, lnext = 64, ev = -1;

@@ -331,6 +331,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
     s_view.time = (unsigned)clock64() - kViewCycles;
     s_view.dump = 0;
     s_view.more = 1;
+    s_view.tokens = 0;
     s_view.starving = kIdlePark * P.ctl->batch < ((long long)gridDim.x * blockDim.x >> 5);
   }
   fill_key_tables(K);
@@ -396,6 +397,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
   bool top_dirty = false;      // persistent: the stack top lives only in the shared copy (its HBM slot is stale)
   bool counted_idle = false;   // persistent, lane 0: this warp is counted in ctl->idle
   bool counted_deep = false;   // persistent, lane 0: this warp is counted in ctl->deep
+  bool outputs_full = false;   // persistent: this warp put a node on the outputs beyond Params::out_soft
   bool starving = PERSIST && kIdlePark * batch < nwarps_all;  // persistent: many warps wait for work
   int rounds = 0;              // slices run: a warp dumps only after one (progress every epoch)
   unsigned long long st_lane_rounds = 0, st_polls = 0;
@@ -439,6 +441,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
             }
           }
           __syncwarp();
+          bool spilled_past = false;
           if (more) {
             Node *dst = nullptr;
             if (rank < npush - 1) {
@@ -449,6 +452,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
               const unsigned long long k = atomicAdd(&ctl->nout, 1ull);
               if ((long long)k < P.out_cap) dst = P.out + k;
               else atomicOr(&ctl->error, kErrOutFull);
+              spilled_past = (long long)k >= P.out_soft;
             }
             if (dst) lane_store(L, dst, tcol, rcol, stride, P.nq, fork_cell, keep, vm);
           }
@@ -462,7 +466,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
             sp += npush;
             have_cur = true;
           }
-          __syncwarp();
+          if (__any_sync(kFull, spilled_past)) outputs_full = true;
         }
         if (status == kStFork) {
           if (first < 0) {
@@ -661,6 +665,10 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
       d = __shfl_sync(kFull, d, 0);
       starving = d & 2;
       d &= 1;
+      if (outputs_full) {
+        if (lane == 0) *((volatile int *)&ctl->dump) = 1;
+        d = 1;
+      }
       if (d && rounds > 0) {
         // dump: live lanes as resume nodes, then this warp's stack
         if (status == kStRun) {
@@ -1610,6 +1618,15 @@ static void decode_survivor(const SurvRec &r, int nq, e13_survivor *s) {
   s->steps = r.t;
 }
 
+// Outputs of an epoch's end beside the dump of lanes and stacks: the nodes that
+// each warp's stack has no room for in the round in which the warp learns that
+// the epoch ends (a warp that passes out_soft itself knows at once), and the
+// input that a block claimed but did not take.  Without room for them, searches
+// with small stacks ended with E13_ERR_OVERFLOW.
+static long long end_room(const e13_ctx *c, long long nwarps) {
+  return nwarps * 32 + (long long)c->nsm * kInputChunk;
+}
+
 // Kernel parameters of a search or serve session over the context's buffers.
 // dump_room: frontier nodes the warps may write when an epoch ends.
 static Params make_params(const e13_ctx *c, const e13_tuning &tu, int nq, long long nwarps, long long dump_room,
@@ -1632,9 +1649,11 @@ static Params make_params(const e13_ctx *c, const e13_tuning &tu, int nq, long l
   P.pool_cap = c->pool_cap;
   P.pool = c->pool;
   P.pool_ready = c->pool_ready;
-  // the persistent kernel's outputs leave kLongOut slots to long_kernel
+  // the persistent kernel's outputs leave kLongOut slots to long_kernel, and
+  // what an epoch may still write once out_soft nodes are out: dump_room and
+  // end_room
   P.out_cap = c->out_cap - (tu.kernel == E13_KERNEL_PERSISTENT ? kLongOut : 0);
-  P.out_soft = P.out_cap - dump_room - 1024;
+  P.out_soft = P.out_cap - dump_room - end_room(c, nwarps) - 1024;
   P.out_nodes = 2 * dump_room + 65536;
   P.stack_cap = stack_cap;
   P.surv_cap = c->surv_cap;
@@ -2053,7 +2072,7 @@ static int search_impl(e13_ctx *c, const e13_job *job, const e13_tuning *tuning,
   // the frontier capacity of this search: exactly what the tuning asks for,
   // else all that the context holds (a larger stack left by a serve session)
   const long long cap = tu.stack_nodes > 0 ? tu.stack_nodes : c->stack_cap;
-  if ((rc = grow(&c->out, &c->out_cap, out_nodes + (persist ? kLongOut : 0)))) return rc;
+  if ((rc = grow(&c->out, &c->out_cap, out_nodes + (persist ? end_room(c, nwarps) + kLongOut : 0)))) return rc;
   if (persist && (rc = grow(&c->wstack, &c->wstack_nodes, nwarps * tu.warp_stack))) return rc;
   if (persist && (rc = grow(&c->pool, &c->pool_cap, kPoolNodes))) return rc;
   if (persist && (rc = grow(&c->pool_ready, &c->pool_ready_cap, kPoolNodes))) return rc;
@@ -2322,7 +2341,7 @@ extern "C" int e13_selftest_pool_wait(e13_ctx *c, int32_t wait_us) {
   const long long nwarps = (long long)c->nsm * tu.block / 32;
   const long long dump_room = nwarps * (32 + tu.warp_stack);
   if ((rc = grow(&c->stack, &c->stack_cap, 1024))) return rc;
-  if ((rc = grow(&c->out, &c->out_cap, 2 * dump_room + 65536 + kLongOut))) return rc;
+  if ((rc = grow(&c->out, &c->out_cap, 2 * dump_room + 65536 + end_room(c, nwarps) + kLongOut))) return rc;
   if ((rc = grow(&c->wstack, &c->wstack_nodes, nwarps * tu.warp_stack))) return rc;
   if ((rc = grow(&c->pool, &c->pool_cap, kPoolNodes))) return rc;
   if ((rc = grow(&c->pool_ready, &c->pool_ready_cap, kPoolNodes))) return rc;
@@ -2566,7 +2585,7 @@ extern "C" int e13_serve_create(e13_ctx *c, const e13_tuning *tuning, int64_t re
   const long long stack_nodes = tu.stack_nodes > 0 ? tu.stack_nodes : (16LL << 20);
   if ((rc = grow(&c->stack, &c->stack_cap, stack_nodes))) return rc;
   s->cap = tu.stack_nodes > 0 ? tu.stack_nodes : c->stack_cap;
-  if ((rc = grow(&c->out, &c->out_cap, s->out_nodes + kLongOut))) return rc;
+  if ((rc = grow(&c->out, &c->out_cap, s->out_nodes + end_room(c, nwarps) + kLongOut))) return rc;
   if ((rc = grow(&c->wstack, &c->wstack_nodes, nwarps * tu.warp_stack))) return rc;
   if ((rc = grow(&c->pool, &c->pool_cap, kPoolNodes))) return rc;
   if ((rc = grow(&c->pool_ready, &c->pool_ready_cap, kPoolNodes))) return rc;

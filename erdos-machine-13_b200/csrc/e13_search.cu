@@ -210,6 +210,19 @@ constexpr int kWarpWords = (kTapeWords + 16) * 32 + (int)sizeof(Node) / 4;  // s
 
 enum { kStRun = 0, kStIdle = 1, kStFork = 2, kStCap = 3, kStDead = 4, kStSurv = 5 };
 
+// Handed-over machines and their queued children may come back to the frontier
+// as one node each, beside an epoch's own outputs.  Where it has no room for
+// kLongOut such nodes more, the epoch ends that much earlier (long_taken off
+// out_soft): without hand-over a long machine is single-stepped, 41 ms instead
+// of 1 for the FMAX = 2 search of X = 8.
+static __device__ __forceinline__ long long long_taken(const Params &P, long long top) {
+  return max(0ll, min((long long)kLongOut, kLongOut - (P.stack_cap - top - P.out_nodes)));
+}
+// Frontier nodes that they may take in all.
+static __device__ __forceinline__ long long long_room(const Params &P, long long top) {
+  return max(0ll, P.stack_cap - top - P.out_nodes + long_taken(P, top));
+}
+
 // A block's view of the persistent kernel's control words.  All warps of the
 // GPU polling the same few words of L2 held up the warps at work (the first
 // epoch of a search of 1000 machines took 408 us, with one poller per block
@@ -227,7 +240,8 @@ constexpr unsigned kViewCycles = 1000;  // a younger view is not renewed
 
 // By one lane: renews the view (and ends the epoch where it is due) unless
 // another warp of the block is at it.
-static __device__ __noinline__ void refresh_view(View *s_view, const Params &P, unsigned long long t_begin) {
+static __device__ __noinline__ void refresh_view(View *s_view, const Params &P, unsigned long long t_begin,
+                                                long long out_soft) {
   volatile View *v = s_view;
   if ((unsigned)clock64() - v->time < kViewCycles || v->lock || atomicCAS(&s_view->lock, 0, 1) != 0) return;
   Ctl *ctl = P.ctl;
@@ -241,7 +255,7 @@ static __device__ __noinline__ void refresh_view(View *s_view, const Params &P, 
   const int busy2 = *((volatile int *)&ctl->busy);
   const int nwarps = (int)(((long long)gridDim.x * blockDim.x) >> 5);
   if (!d) {
-    d = now - t_begin > (unsigned long long)P.epoch_ns || nout > P.out_soft;
+    d = now - t_begin > (unsigned long long)P.epoch_ns || nout > out_soft;
     // starving.  Work spreads inside an epoch only through donated nodes,
     // which a few deep warps hand out one at a time: a job whose subtrees
     // are shallow would run on a few warps for a long time.  When more
@@ -354,9 +368,8 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
   const long long batch = ctl->batch;
   const int chunk = (int)max(1ll, min((long long)kInputChunk, batch / (kInputChunks * (long long)gridDim.x)));
   const int tag = ctl->launches + 1;  // marks pool slots written in this launch
-  // handed-over machines come back to the frontier: no more of them than it
-  // has room for beside an epoch's outputs
-  const int long_cap = PERSIST ? (int)max(0ll, min((long long)kLongCap, P.stack_cap - top0 - P.out_nodes)) : 0;
+  const int long_cap = PERSIST ? (int)min((long long)kLongCap, long_room(P, top0)) : 0;
+  const long long out_soft = PERSIST ? P.out_soft - long_taken(P, top0) : 0;
   const int D = P.wdepth;
   Node *wst = PERSIST ? P.wstack + gwarp * D : nullptr;
   const unsigned long long t_begin = PERSIST ? globaltimer() : 0ull;
@@ -452,7 +465,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
               const unsigned long long k = atomicAdd(&ctl->nout, 1ull);
               if ((long long)k < P.out_cap) dst = P.out + k;
               else atomicOr(&ctl->error, kErrOutFull);
-              spilled_past = (long long)k >= P.out_soft;
+              spilled_past = (long long)k >= out_soft;
             }
             if (dst) lane_store(L, dst, tcol, rcol, stride, P.nq, fork_cell, keep, vm);
           }
@@ -646,7 +659,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
           }
           volatile View *v = &s_view;
           for (;;) {
-            refresh_view(&s_view, P, t_begin);
+            refresh_view(&s_view, P, t_begin, out_soft);
             done = v->dump || !v->more;
             if (done || (v->tokens > 0 && atomicSub(&s_view.tokens, 1) > 0)) break;
             __nanosleep(100);
@@ -659,7 +672,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
       }
       int d = 0;
       if (lane == 0) {
-        if ((rounds & 7) == 0) refresh_view(&s_view, P, t_begin);  // the control words are in L2: every 8th round
+        if ((rounds & 7) == 0) refresh_view(&s_view, P, t_begin, out_soft);  // the control words are in L2: every 8th round
         d = ((volatile View *)&s_view)->dump | (((volatile View *)&s_view)->starving << 1);
       }
       d = __shfl_sync(kFull, d, 0);
@@ -922,11 +935,11 @@ static __device__ __forceinline__ void take_child(Lane &L, u32 *rows, int lane, 
 // between the search kernel and move_outputs.
 __global__ void __launch_bounds__(kLongBlock) long_kernel(const __grid_constant__ Params P) {
   Ctl *ctl = P.ctl;
-  const long long slack = P.stack_cap - ctl->top - P.out_nodes;
-  const int n = (int)min((long long)ctl->nlong, max(0ll, min((long long)kLongCap, slack)));
+  const long long room = long_room(P, ctl->top);
+  const int n = (int)min((long long)ctl->nlong, min((long long)kLongCap, room));
   if (n == 0) return;
   // each machine and each queued child may come back as one frontier node
-  const int item_cap = (int)min((long long)kLongItems, slack - n);
+  const int item_cap = (int)min((long long)kLongItems, room - n);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const KeyTabs K = key_tables(smem_raw);
   u64 *span = reinterpret_cast<u64 *>(smem_raw + kKeySmemBytes);
@@ -1653,8 +1666,8 @@ static Params make_params(const e13_ctx *c, const e13_tuning &tu, int nq, long l
   // what an epoch may still write once out_soft nodes are out: dump_room and
   // end_room
   P.out_cap = c->out_cap - (tu.kernel == E13_KERNEL_PERSISTENT ? kLongOut : 0);
-  P.out_soft = P.out_cap - dump_room - end_room(c, nwarps) - 1024;
   P.out_nodes = 2 * dump_room + 65536;
+  P.out_soft = P.out_nodes - dump_room - 1024;  // (by the frontier's room, also where the buffer is larger)
   P.stack_cap = stack_cap;
   P.surv_cap = c->surv_cap;
   P.epoch_ns = (long long)tu.epoch_us * 1000LL;

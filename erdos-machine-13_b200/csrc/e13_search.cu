@@ -235,13 +235,13 @@ struct View {
   int tokens;    // pool nodes waiting that this block's idle warps have not gone for
   int starving;  // many warps wait for work, and the pool holds less than one node for each
   unsigned time;  // of the last renewal, SM cycles
+  long long out_soft;  // outputs beyond which the epoch ends
 };
 constexpr unsigned kViewCycles = 1000;  // a younger view is not renewed
 
 // By one lane: renews the view (and ends the epoch where it is due) unless
 // another warp of the block is at it.
-static __device__ __noinline__ void refresh_view(View *s_view, const Params &P, unsigned long long t_begin,
-                                                long long out_soft) {
+static __device__ __noinline__ void refresh_view(View *s_view, const Params &P, unsigned long long t_begin) {
   volatile View *v = s_view;
   if ((unsigned)clock64() - v->time < kViewCycles || v->lock || atomicCAS(&s_view->lock, 0, 1) != 0) return;
   Ctl *ctl = P.ctl;
@@ -255,7 +255,7 @@ static __device__ __noinline__ void refresh_view(View *s_view, const Params &P, 
   const int busy2 = *((volatile int *)&ctl->busy);
   const int nwarps = (int)(((long long)gridDim.x * blockDim.x) >> 5);
   if (!d) {
-    d = now - t_begin > (unsigned long long)P.epoch_ns || nout > out_soft;
+    d = now - t_begin > (unsigned long long)P.epoch_ns || nout > v->out_soft;
     // starving.  Work spreads inside an epoch only through donated nodes,
     // which a few deep warps hand out one at a time: a job whose subtrees
     // are shallow would run on a few warps for a long time.  When more
@@ -335,6 +335,8 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
   // persistent: the block's view of the control words (refresh_view)
   __shared__ View s_view;
   __shared__ Input s_in;
+  __shared__ unsigned char s_full[32];  // persistent: this warp put a node on the outputs beyond View::out_soft
+  if (threadIdx.x < 32) s_full[threadIdx.x] = 0;
   __shared__ unsigned long long s_stat[5];
   if (threadIdx.x < 5) s_stat[threadIdx.x] = 0;
   if (PERSIST && threadIdx.x == 0) {
@@ -346,6 +348,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
     s_view.dump = 0;
     s_view.more = 1;
     s_view.tokens = 0;
+    s_view.out_soft = P.out_soft - long_taken(P, P.ctl->top);
     s_view.starving = kIdlePark * P.ctl->batch < ((long long)gridDim.x * blockDim.x >> 5);
   }
   fill_key_tables(K);
@@ -369,7 +372,6 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
   const int chunk = (int)max(1ll, min((long long)kInputChunk, batch / (kInputChunks * (long long)gridDim.x)));
   const int tag = ctl->launches + 1;  // marks pool slots written in this launch
   const int long_cap = PERSIST ? (int)min((long long)kLongCap, long_room(P, top0)) : 0;
-  const long long out_soft = PERSIST ? P.out_soft - long_taken(P, top0) : 0;
   const int D = P.wdepth;
   Node *wst = PERSIST ? P.wstack + gwarp * D : nullptr;
   const unsigned long long t_begin = PERSIST ? globaltimer() : 0ull;
@@ -410,7 +412,6 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
   bool top_dirty = false;      // persistent: the stack top lives only in the shared copy (its HBM slot is stale)
   bool counted_idle = false;   // persistent, lane 0: this warp is counted in ctl->idle
   bool counted_deep = false;   // persistent, lane 0: this warp is counted in ctl->deep
-  bool outputs_full = false;   // persistent: this warp put a node on the outputs beyond Params::out_soft
   bool starving = PERSIST && kIdlePark * batch < nwarps_all;  // persistent: many warps wait for work
   int rounds = 0;              // slices run: a warp dumps only after one (progress every epoch)
   unsigned long long st_lane_rounds = 0, st_polls = 0;
@@ -454,7 +455,6 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
             }
           }
           __syncwarp();
-          bool spilled_past = false;
           if (more) {
             Node *dst = nullptr;
             if (rank < npush - 1) {
@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
               const unsigned long long k = atomicAdd(&ctl->nout, 1ull);
               if ((long long)k < P.out_cap) dst = P.out + k;
               else atomicOr(&ctl->error, kErrOutFull);
-              spilled_past = (long long)k >= out_soft;
+              if ((long long)k >= s_view.out_soft) s_full[threadIdx.x >> 5] = 1;
             }
             if (dst) lane_store(L, dst, tcol, rcol, stride, P.nq, fork_cell, keep, vm);
           }
@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
             sp += npush;
             have_cur = true;
           }
-          if (__any_sync(kFull, spilled_past)) outputs_full = true;
+          __syncwarp();
         }
         if (status == kStFork) {
           if (first < 0) {
@@ -659,7 +659,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
           }
           volatile View *v = &s_view;
           for (;;) {
-            refresh_view(&s_view, P, t_begin, out_soft);
+            refresh_view(&s_view, P, t_begin);
             done = v->dump || !v->more;
             if (done || (v->tokens > 0 && atomicSub(&s_view.tokens, 1) > 0)) break;
             __nanosleep(100);
@@ -672,16 +672,16 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
       }
       int d = 0;
       if (lane == 0) {
-        if ((rounds & 7) == 0) refresh_view(&s_view, P, t_begin, out_soft);  // the control words are in L2: every 8th round
+        if ((rounds & 7) == 0) refresh_view(&s_view, P, t_begin);  // the control words are in L2: every 8th round
         d = ((volatile View *)&s_view)->dump | (((volatile View *)&s_view)->starving << 1);
+        if (s_full[threadIdx.x >> 5]) {
+          *((volatile int *)&ctl->dump) = 1;
+          d |= 1;
+        }
       }
       d = __shfl_sync(kFull, d, 0);
       starving = d & 2;
       d &= 1;
-      if (outputs_full) {
-        if (lane == 0) *((volatile int *)&ctl->dump) = 1;
-        d = 1;
-      }
       if (d && rounds > 0) {
         // dump: live lanes as resume nodes, then this warp's stack
         if (status == kStRun) {

@@ -1560,25 +1560,39 @@ extern "C" int e13_last_stats(const e13_ctx *c, e13_stats *out) {
 
 extern "C" bool *e13_ctx_filter_tables(e13_ctx *c, int which) { return &c->filter_tables[which]; }
 
+// Frees what the context only keeps for later calls: every scratch slot but
+// those of the call `but` (-1: all), and the serve sessions' second stack.
+static void give_back(e13_ctx *c, int but) {
+  for (int k = 0; k < kScratchSlots; ++k) {
+    if (e13_scratch_call(k) == but) continue;
+    cudaFree(c->scratch[k]);
+    c->scratch[k] = nullptr;
+    c->scratch_cap[k] = 0;
+  }
+  cudaFree(c->alt);
+  c->alt = nullptr;
+  c->alt_cap = 0;
+}
+
+// cudaMalloc; where memory has run out, once more without what the context
+// keeps (scratch slots of the call `but` stay).
+static cudaError_t ctx_malloc(e13_ctx *c, void **p, size_t bytes, int but = -1) {
+  if (cudaMalloc(p, bytes) == cudaSuccess) return cudaSuccess;
+  cudaGetLastError();
+  give_back(c, but);
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaSuccess) return e;
+  cudaGetLastError();
+  *p = nullptr;
+  return e;
+}
+
 extern "C" void *e13_ctx_scratch(e13_ctx *c, int slot, size_t bytes) {
   if (c->scratch_cap[slot] >= bytes) return c->scratch[slot];
   cudaFree(c->scratch[slot]);
   c->scratch[slot] = nullptr;
   c->scratch_cap[slot] = 0;
-  if (cudaMalloc(&c->scratch[slot], bytes) != cudaSuccess) {
-    // give back what other calls left, and try once more
-    cudaGetLastError();
-    for (int k = 0; k < kScratchSlots; ++k) {
-      if (e13_scratch_call(k) == e13_scratch_call(slot)) continue;  // this call's own
-      cudaFree(c->scratch[k]);
-      c->scratch[k] = nullptr;
-      c->scratch_cap[k] = 0;
-    }
-    if (cudaMalloc(&c->scratch[slot], bytes) != cudaSuccess) {
-      cudaGetLastError();
-      return nullptr;
-    }
-  }
+  if (ctx_malloc(c, &c->scratch[slot], bytes, e13_scratch_call(slot)) != cudaSuccess) return nullptr;
   c->scratch_cap[slot] = bytes;
   return c->scratch[slot];
 }
@@ -1593,20 +1607,20 @@ extern "C" void e13_ctx_scratch_done(e13_ctx *c) {
 }
 
 template <typename T>
-static int grow(T **p, long long *cap, long long want) {
+static int grow(e13_ctx *c, T **p, long long *cap, long long want) {
   if (*cap >= want) return E13_OK;
   if (*p) cudaFree(*p);
   *p = nullptr;
   *cap = 0;
-  CK(cudaMalloc(p, sizeof(T) * (size_t)want));
+  CK(ctx_malloc(c, (void **)p, sizeof(T) * (size_t)want));
   *cap = want;
   return E13_OK;
 }
 
 // The long-machine kernel's buffers.
 static int grow_long(e13_ctx *c) {
-  const int rc = grow(&c->longq, &c->longq_cap, (long long)kLongCap + kLongNodes);
-  return rc ? rc : grow(&c->long_items, &c->long_items_cap, (long long)kLongItems);
+  const int rc = grow(c, &c->longq, &c->longq_cap, (long long)kLongCap + kLongNodes);
+  return rc ? rc : grow(c, &c->long_items, &c->long_items_cap, (long long)kLongItems);
 }
 
 static void decode_survivor(const SurvRec &r, int nq, e13_survivor *s) {
@@ -1862,7 +1876,7 @@ int ckpt_load(e13_ctx *c, const e13_job *job, const e13_checkpoint *ck, long lon
   fclose(f);
 
   int rc;
-  if ((rc = grow(&c->surv, &c->surv_cap, std::max<long long>((long long)hd.nrec, c->surv_cap)))) return rc;
+  if ((rc = grow(c, &c->surv, &c->surv_cap, std::max<long long>((long long)hd.nrec, c->surv_cap)))) return rc;
   memset(c->ctl_host, 0, sizeof(Ctl));
   c->ctl_host->top = hd.top;
   c->ctl_host->batch = std::min<long long>(hd.top, batch_max);
@@ -1963,6 +1977,7 @@ static int split_share(e13_ctx *c, const e13_job *job, const e13_tuning &tu, int
   const long long target = kSplitPerShard * nshards;
   // the last level starts below target nodes and each node has at most `fan` children
   const long long stack_n = target * fan + nwarps * 32 + 1024, out_n = stack_n, surv_n = 4096;
+  const ScratchCall call(c);
   Node *stack = (Node *)e13_ctx_scratch(c, kScratchSplitStack, sizeof(Node) * (size_t)stack_n);
   Node *out = (Node *)e13_ctx_scratch(c, kScratchSplitOut, sizeof(Node) * (size_t)out_n);
   Ctl *ctl = (Ctl *)e13_ctx_scratch(c, kScratchSplitCtl, sizeof(Ctl));
@@ -2045,7 +2060,6 @@ static int split_share(e13_ctx *c, const e13_job *job, const e13_tuning &tu, int
     }
   }
   cudaStreamSynchronize(c->stream);
-  e13_ctx_scratch_done(c);
   return rc;
 }
 
@@ -2081,17 +2095,17 @@ static int search_impl(e13_ctx *c, const e13_job *job, const e13_tuning *tuning,
     batch_max = tu.batch > 0 ? tu.batch : 16384;
     out_nodes = batch_max * (4LL * job->nq + 1) + nwarps * 32 + 1024;
   }
-  if ((rc = grow(&c->stack, &c->stack_cap, stack_nodes))) return rc;
+  if ((rc = grow(c, &c->stack, &c->stack_cap, stack_nodes))) return rc;
   // the frontier capacity of this search: exactly what the tuning asks for,
   // else all that the context holds (a larger stack left by a serve session)
   const long long cap = tu.stack_nodes > 0 ? tu.stack_nodes : c->stack_cap;
-  if ((rc = grow(&c->out, &c->out_cap, out_nodes + (persist ? end_room(c, nwarps) + kLongOut : 0)))) return rc;
-  if (persist && (rc = grow(&c->wstack, &c->wstack_nodes, nwarps * tu.warp_stack))) return rc;
-  if (persist && (rc = grow(&c->pool, &c->pool_cap, kPoolNodes))) return rc;
-  if (persist && (rc = grow(&c->pool_ready, &c->pool_ready_cap, kPoolNodes))) return rc;
+  if ((rc = grow(c, &c->out, &c->out_cap, out_nodes + (persist ? end_room(c, nwarps) + kLongOut : 0)))) return rc;
+  if (persist && (rc = grow(c, &c->wstack, &c->wstack_nodes, nwarps * tu.warp_stack))) return rc;
+  if (persist && (rc = grow(c, &c->pool, &c->pool_cap, kPoolNodes))) return rc;
+  if (persist && (rc = grow(c, &c->pool_ready, &c->pool_ready_cap, kPoolNodes))) return rc;
   if (persist && (rc = grow_long(c))) return rc;
   const long long scap = std::max<long long>(surv_cap, 1024);
-  if ((rc = grow(&c->surv, &c->surv_cap, scap))) return rc;
+  if ((rc = grow(c, &c->surv, &c->surv_cap, scap))) return rc;
 
   JobParam jp[kMaxJobs];
   memset(jp, 0, sizeof jp);
@@ -2320,6 +2334,7 @@ extern "C" int e13_run_full(e13_ctx *c, const int32_t *tabs, int n, int nq, int6
   CK(cudaSetDevice(c->device));
   int rc = ensure_consts(c);
   if (rc) return rc;
+  const ScratchCall call(c);
   int *d_tabs = (int *)e13_ctx_scratch(c, kScratchFullTabs, sizeof(int) * E13_MAXCELLS * (size_t)n);
   long long *d_out = (long long *)e13_ctx_scratch(c, kScratchFullOut, sizeof(long long) * 7 * (size_t)n);
   int *d_list = (int *)e13_ctx_scratch(c, kScratchFullList, sizeof(int) * ((size_t)n + 2));
@@ -2335,7 +2350,6 @@ extern "C" int e13_run_full(e13_ctx *c, const int32_t *tabs, int n, int nq, int6
   CK(cudaGetLastError());
   CK(d2h(c, out, d_out, sizeof(long long) * 7 * (size_t)n));
   CK(cudaStreamSynchronize(c->stream));
-  e13_ctx_scratch_done(c);
   return E13_OK;
 }
 
@@ -2353,13 +2367,13 @@ extern "C" int e13_selftest_pool_wait(e13_ctx *c, int32_t wait_us) {
   e13_resolve_tuning(nullptr, 0, &tu);
   const long long nwarps = (long long)c->nsm * tu.block / 32;
   const long long dump_room = nwarps * (32 + tu.warp_stack);
-  if ((rc = grow(&c->stack, &c->stack_cap, 1024))) return rc;
-  if ((rc = grow(&c->out, &c->out_cap, 2 * dump_room + 65536 + end_room(c, nwarps) + kLongOut))) return rc;
-  if ((rc = grow(&c->wstack, &c->wstack_nodes, nwarps * tu.warp_stack))) return rc;
-  if ((rc = grow(&c->pool, &c->pool_cap, kPoolNodes))) return rc;
-  if ((rc = grow(&c->pool_ready, &c->pool_ready_cap, kPoolNodes))) return rc;
+  if ((rc = grow(c, &c->stack, &c->stack_cap, 1024))) return rc;
+  if ((rc = grow(c, &c->out, &c->out_cap, 2 * dump_room + 65536 + end_room(c, nwarps) + kLongOut))) return rc;
+  if ((rc = grow(c, &c->wstack, &c->wstack_nodes, nwarps * tu.warp_stack))) return rc;
+  if ((rc = grow(c, &c->pool, &c->pool_cap, kPoolNodes))) return rc;
+  if ((rc = grow(c, &c->pool_ready, &c->pool_ready_cap, kPoolNodes))) return rc;
   if ((rc = grow_long(c))) return rc;
-  if ((rc = grow(&c->surv, &c->surv_cap, 1024))) return rc;
+  if ((rc = grow(c, &c->surv, &c->surv_cap, 1024))) return rc;
   Params P = make_params(c, tu, 16, nwarps, dump_room, c->stack_cap);
   P.wait_ns = (long long)wait_us * 1000LL;
   const size_t smem = search_smem(tu.block);
@@ -2560,7 +2574,7 @@ struct e13_serve {
           *p = next;
           break;
         }
-      if (!c->alt) {
+      if (!c->alt && alt_cap <= kAltKeepNodes) {
         std::swap(c->alt, alt);
         c->alt_cap = alt_cap;
       }
@@ -2596,14 +2610,14 @@ extern "C" int e13_serve_create(e13_ctx *c, const e13_tuning *tuning, int64_t re
   s->large_reserve = dump_room;
   // serving keeps many frontiers resident: 16 Mi nodes (5 GB) by default
   const long long stack_nodes = tu.stack_nodes > 0 ? tu.stack_nodes : (16LL << 20);
-  if ((rc = grow(&c->stack, &c->stack_cap, stack_nodes))) return rc;
+  if ((rc = grow(c, &c->stack, &c->stack_cap, stack_nodes))) return rc;
   s->cap = tu.stack_nodes > 0 ? tu.stack_nodes : c->stack_cap;
-  if ((rc = grow(&c->out, &c->out_cap, s->out_nodes + end_room(c, nwarps) + kLongOut))) return rc;
-  if ((rc = grow(&c->wstack, &c->wstack_nodes, nwarps * tu.warp_stack))) return rc;
-  if ((rc = grow(&c->pool, &c->pool_cap, kPoolNodes))) return rc;
-  if ((rc = grow(&c->pool_ready, &c->pool_ready_cap, kPoolNodes))) return rc;
+  if ((rc = grow(c, &c->out, &c->out_cap, s->out_nodes + end_room(c, nwarps) + kLongOut))) return rc;
+  if ((rc = grow(c, &c->wstack, &c->wstack_nodes, nwarps * tu.warp_stack))) return rc;
+  if ((rc = grow(c, &c->pool, &c->pool_cap, kPoolNodes))) return rc;
+  if ((rc = grow(c, &c->pool_ready, &c->pool_ready_cap, kPoolNodes))) return rc;
   if ((rc = grow_long(c))) return rc;
-  if ((rc = grow(&c->surv, &c->surv_cap, 1LL << 20))) return rc;
+  if ((rc = grow(c, &c->surv, &c->surv_cap, 1LL << 20))) return rc;
   memset(s->jp, 0, sizeof s->jp);
   s->P = make_params(c, tu, 16, nwarps, dump_room, s->cap);
   s->smem = search_smem(tu.block);
@@ -2618,7 +2632,7 @@ extern "C" int e13_serve_create(e13_ctx *c, const e13_tuning *tuning, int64_t re
     cudaFree(c->alt);
     c->alt = nullptr;
     c->alt_cap = 0;
-    CK(cudaMalloc(&c->alt, sizeof(Node) * (size_t)c->stack_cap));
+    CK(ctx_malloc(c, (void **)&c->alt, sizeof(Node) * (size_t)c->stack_cap));
     c->alt_cap = c->stack_cap;
   }
   std::swap(s->alt, c->alt);

@@ -214,8 +214,9 @@ extern "C" int e13_raw_run(e13_ctx *ctx, const uint8_t *codes, uint64_t seed, in
   long long *d_out = nullptr;
   RawWork *d_work = nullptr;
   int *d_list = nullptr;
-  // the macro simulator counts steps in 32 bits and lists machines by int
-  const bool park = max_steps > kRawSteps && max_steps <= kRawIntMax && n <= 0x7FFFFFFFLL;
+  // the macro simulator counts steps in 32 bits and lists machines by int;
+  // without room for the list (4 bytes a machine) the first kernel runs them all
+  bool park = max_steps > kRawSteps && max_steps <= kRawIntMax && n <= 0x7FFFFFFFLL;
   int rc = E13_OK;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
@@ -224,7 +225,8 @@ extern "C" int e13_raw_run(e13_ctx *ctx, const uint8_t *codes, uint64_t seed, in
   if (out) d_out = (long long *)e13_ctx_scratch(ctx, kScratchRawOut, sizeof(long long) * 4 * (size_t)n);
   d_work = (RawWork *)e13_ctx_scratch(ctx, kScratchRawWork, sizeof(RawWork));
   if (park) d_list = (int *)e13_ctx_scratch(ctx, kScratchRawList, sizeof(int) * (size_t)n);
-  if ((codes && !d_codes) || (out && !d_out) || !d_work || (park && !d_list)) rc = E13_ERR_CUDA;
+  park = d_list != nullptr;
+  if ((codes && !d_codes) || (out && !d_out) || !d_work) rc = E13_ERR_CUDA;
   if (!rc) {
     int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, e13_ctx_device(ctx));

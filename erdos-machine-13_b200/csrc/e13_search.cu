@@ -2993,19 +2993,23 @@ extern "C" int e13_serve_step(e13_serve *s, e13_serve_result *done, int cap, int
   //    job's frontier nodes and counters go to host memory and it goes back to
   //    the head of the queue; re-admitted, it goes on where it stopped (its
   //    counts stay exact).  A job that does not fit alone fails with
-  //    E13_ERR_OVERFLOW.
+  //    E13_ERR_OVERFLOW: after an epoch that it had to itself.  (If it shared
+  //    the epoch, it is swapped out like the others, whether these have ended in
+  //    that epoch or not: which of the two it is depends on the speed alone.)
   const long long cur_top = c->ctl_host->top;
   if (complete && n > 0 && cur_top + s->out_nodes > s->cap) {
     int first = 0;  // order[0..first) leave the frontier, order[first..n) stay
     long long after = cur_top;
     while (n - first > 1 && after + s->out_nodes > s->cap) after -= (long long)nodes[order[first++]];
     if (after + s->out_nodes > s->cap) {
-      // one job left and it alone does not fit: it fails, its nodes are dropped
+      // one job left and it alone does not fit
       const int k = order[first++];
-      ServeJob &j = *s->slot_job[k];
-      fill_result(done[(*ndone)++], j, cnt + k * kJobCounters, E13_ERR_OVERFLOW, tdone);
-      s->finished_surv[j.id] = std::move(j.surv);
-      s->slot_job[k].reset();
+      if (running == 1) {  // it fails, its nodes are dropped
+        ServeJob &j = *s->slot_job[k];
+        fill_result(done[(*ndone)++], j, cnt + k * kJobCounters, E13_ERR_OVERFLOW, tdone);
+        s->finished_surv[j.id] = std::move(j.surv);
+        s->slot_job[k].reset();
+      }
       after -= (long long)nodes[k];
     }
     int rc;

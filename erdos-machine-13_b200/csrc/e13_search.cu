@@ -107,6 +107,12 @@ constexpr int kLongMemoBits = 11;
 constexpr int kLongBlock = 192;
 constexpr int kLongPerSm = 1;
 constexpr long long kLongMinNs = 1000000;  // shortest time bound of long_kernel: 1 ms (else a tenth of the epoch)
+// An epoch's time bound (e13_tuning::epoch_us) holds for both kernels, so the
+// search has what long_kernel's bound leaves of it, but no less than 1.5 ms of
+// it: shorter ones cost more than they hold back.  FMAX = 4 search of X = 9 with
+// epochs of 2 ms: 34.1 ms with 2 ms for the search, 36.2 with 1 ms; with epochs
+// of 0.2 ms 66 and, halved, 198.
+constexpr long long kLeastSearchNs = 1500000;
 constexpr int kIdlePark = 8;             // many warps wait: more than an eighth
 constexpr int kParkMin = 2048;
 constexpr int kNeverPark = 0x7FFFFFFF;
@@ -1684,7 +1690,9 @@ static Params make_params(const e13_ctx *c, const e13_tuning &tu, int nq, long l
   P.out_soft = P.out_nodes - dump_room - 1024;  // (by the frontier's room, also where the buffer is larger)
   P.stack_cap = stack_cap;
   P.surv_cap = c->surv_cap;
+  // the search's part of an epoch; the rest is long_kernel's
   P.epoch_ns = (long long)tu.epoch_us * 1000LL;
+  P.epoch_ns = std::max(P.epoch_ns - P.long_ns, std::min(P.epoch_ns, kLeastSearchNs));
   P.wait_ns = kPoolWaitNs;
   P.min_epoch_ns = kMinEpochNs;
   P.stack = c->stack;

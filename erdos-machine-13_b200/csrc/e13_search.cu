@@ -236,7 +236,7 @@ static __device__ __forceinline__ long long long_room(const Params &P, long long
 // renews.
 struct View {
   int lock;
-  int dump;      // end the epoch now
+  int dump;      // end the epoch now (also set by a warp whose own node passes out_soft)
   int more;      // work may still come: some warp holds work, or the pool does
   int tokens;    // pool nodes waiting that this block's idle warps have not gone for
   int starving;  // many warps wait for work, and the pool holds less than one node for each
@@ -273,7 +273,7 @@ static __device__ __noinline__ void refresh_view(View *s_view, const Params &P, 
     if (now - t_begin > (unsigned long long)P.min_epoch_ns && 2 * idle > nwarps && deep > 0) d = 1;
     if (d) *((volatile int *)&ctl->dump) = 1;
   }
-  v->dump = d;
+  if (d) v->dump = 1;  // (never back: a warp of the block may have set it)
   v->more = busy != 0 || wait > 0 || busy2 != 0;
   v->tokens = (wait + (int)gridDim.x - 1) / (int)gridDim.x;
   v->starving = kIdlePark * idle > nwarps && wait < idle;
@@ -341,8 +341,6 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
   // persistent: the block's view of the control words (refresh_view)
   __shared__ View s_view;
   __shared__ Input s_in;
-  __shared__ unsigned char s_full[32];  // persistent: this warp put a node on the outputs beyond View::out_soft
-  if (threadIdx.x < 32) s_full[threadIdx.x] = 0;
   __shared__ unsigned long long s_stat[5];
   if (threadIdx.x < 5) s_stat[threadIdx.x] = 0;
   if (PERSIST && threadIdx.x == 0) {
@@ -471,7 +469,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
               const unsigned long long k = atomicAdd(&ctl->nout, 1ull);
               if ((long long)k < P.out_cap) dst = P.out + k;
               else atomicOr(&ctl->error, kErrOutFull);
-              if ((long long)k >= s_view.out_soft) s_full[threadIdx.x >> 5] = 1;
+              if ((long long)k >= s_view.out_soft) *((volatile int *)&s_view.dump) = 1;
             }
             if (dst) lane_store(L, dst, tcol, rcol, stride, P.nq, fork_cell, keep, vm);
           }
@@ -680,10 +678,6 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
       if (lane == 0) {
         if ((rounds & 7) == 0) refresh_view(&s_view, P, t_begin);  // the control words are in L2: every 8th round
         d = ((volatile View *)&s_view)->dump | (((volatile View *)&s_view)->starving << 1);
-        if (s_full[threadIdx.x >> 5]) {
-          *((volatile int *)&ctl->dump) = 1;
-          d |= 1;
-        }
       }
       d = __shfl_sync(kFull, d, 0);
       starving = d & 2;

@@ -100,10 +100,11 @@ struct Ctl {
   int idle;                      // persistent: warps waiting for work (starved)
   int deep;                      // persistent: warps holding 2 or more stack nodes (work a dump would spread)
   // persistent: machines handed to the long-machine kernel in this epoch; in
-  // that kernel, fork nodes kept, children queued, and queue items taken and
-  // finished
+  // that kernel, fork nodes kept, children queued, queue items taken and
+  // finished, and items waiting less the machines handed over
   alignas(128) int nlong;
   int long_nodes;
+  alignas(128) int long_avail;
   alignas(128) int long_head;
   alignas(128) int long_more;
   alignas(128) int long_done;

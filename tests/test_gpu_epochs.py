@@ -22,3 +22,19 @@ def test_epochs_keep_their_bound(searches):
             srv.step()
             ms.append(srv.stats()[0])
     assert statistics.median(b - a for a, b in list(zip(ms, ms[1:]))[2:]) < 5.6
+
+
+def test_epochs_with_many_long_machines_keep_their_bound(searches):
+    """Epochs of 20 ms of the same search, which gathers long machines: from the
+    sixth on thousands of them are unfinished at the end of each epoch.  Beside
+    the 0.2 ms above an epoch may wait for a survivor's read mask (a run of
+    some 271,500 steps by visits, below 1 ms); 22 ms holds both, and not the
+    4 to 8 ms that handing out so many machines one by one took.  (One epoch may
+    be longer: a survivor found by the search kernel itself is run step by step.)"""
+    with E.Server(ctx(), E.tuning(epoch_us=20000)) as srv:
+        srv.submit(make_job(searches["local_edits_f4"], 8), 0)
+        ms = [0.0]
+        for _ in range(14):
+            srv.step()
+            ms.append(srv.stats()[0])
+    assert sorted(b - a for a, b in zip(ms, ms[1:]))[-2] < 22

@@ -131,6 +131,7 @@ struct Params {
   unsigned long long *jobcnt;  // kMaxJobs x kJobCounters totals
   int nq;
   int slice, step_cap, wdepth, pool_low, run_skip;
+  int exact_cap;             // plain: step_cap holds to the step, not to the slice
   int park_after, park_idle; // persistent: hand a machine over after this many steps since its load (while
                              // warps wait for work)
   long long out_cap, out_soft, surv_cap, pool_cap;
@@ -754,6 +755,12 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
       if (rm) {
         int left = L.deadline + 1 - L.t;
         u32 row = (u32)L.st << 2;
+        // the expansion of shards: a lane stops exactly at its step cap, as it
+        // would at a deadline, whatever the other lanes of its warp do, so that
+        // the frontier is a function of the job (split_share)
+        int deadline = L.deadline;
+        const int last = !PERSIST && P.exact_cap ? L.tseg + P.step_cap - 1 : 0x7FFFFFFF;
+        if (!PERSIST) L.deadline = min(deadline, last);
         // (a warp with idle lanes takes up new machines; a starving one has
         // forks that others wait for)
         const int least = min(kLeastLanes, __popc(rm)), most = PERSIST && starving ? (P.slice + 2) / 3 : P.slice;
@@ -782,6 +789,10 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
               ev = lane_act<false>(L, tcol, rcol, K, stride, cell, e);
               if (!ev) ev = lane_act<false>(L, tcol, rcol, K, stride, cell, e);
             }
+            if (!PERSIST && ev == kEvDead && L.t > last && L.t <= deadline) {
+              status = kStCap;
+              ev = 0;
+            }
             // the stage test of a hash match, once per iteration outside
             // lane_act: one copy of it in the loop instead of one per
             // inlined action (the second action waits for it)
@@ -789,9 +800,16 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
               if (PERSIST) {
                 L.t = L.deadline + 1 - left;
                 L.st = (int)(row >> 2);
+              } else {
+                L.deadline = deadline;
               }
               ev = stage_check(L, tcol, K, stride);
-              left = L.deadline + 1 - L.t;
+              if (PERSIST) {
+                left = L.deadline + 1 - L.t;
+              } else {
+                deadline = L.deadline;
+                L.deadline = min(deadline, last);
+              }
             }
             if (ev == kEvCell) {
               if (e == kEntHalt) {
@@ -826,6 +844,8 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
         if (PERSIST) {
           L.t = L.deadline + 1 - left;
           L.st = (int)(row >> 2);
+        } else {
+          L.deadline = deadline;
         }
         if (__any_sync(kFull, status >= kStDead)) {
           if (status >= kStDead) {
@@ -860,7 +880,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
             }
           }
         }
-        if (!PERSIST && status == kStRun && L.t - L.tseg >= P.step_cap) {
+        if (!PERSIST && (status == kStCap || (status == kStRun && L.t - L.tseg >= P.step_cap))) {
           acc_steps += (u32)(L.t - L.tseg);
           L.tseg = L.t;
           if (acc_steps >= 0x80000000u) flush_counts();
@@ -1954,7 +1974,7 @@ static ShardKey shard_key(const Node &n) {
 
 constexpr long long kSplitPerShard = 512;  // frontier nodes per shard before the deal
 constexpr int kSplitLevels = 24;           // most plain launches of the split
-constexpr int kSplitSlice = 24;            // the split's slice and step cap (fixed: they shape the frontier)
+constexpr int kSplitSlice = 24;            // the split's slice and step cap (fixed: the cap shapes the frontier)
 constexpr int kSplitStepCap = 20000;
 
 // One share of a search split over nshards (the reference's SPLIT frontier,
@@ -1967,10 +1987,13 @@ constexpr int kSplitStepCap = 20000;
 // are zero / empty for the other shards.  Runs on scratch buffers of its own,
 // so a serve session's frontier is left alone; `slot` is
 // the job slot written into the nodes.  The expansion runs with a fixed
-// slice, step cap and run skip: a lane is requeued at the first slice end
-// past the step cap, so those settings shape the frontier, and with them fixed
+// slice, step cap and run skip: a lane is requeued at the step cap, so the cap
+// shapes the frontier, and with it fixed
 // every shard's content depends on the job alone, whatever tuning the caller's
-// search then uses (the autotuner compares shard 0 across tunings).
+// search then uses (the autotuner compares shard 0 across tunings).  (Where a
+// lane went on to the end of its slice, as long as its warp's other lanes made
+// it, shares of 18 or more did not add up: FMAX = 3, X = 8 in 64 shares was up
+// to 1849 leaves and 5 survivors off.)
 static int split_share(e13_ctx *c, const e13_job *job, const e13_tuning &tu, int shard, int nshards, int slot,
                        std::vector<Node> &mine, unsigned long long cnt[kJobCounters], std::vector<SurvRec> &recs,
                        long long *launches) {
@@ -2018,6 +2041,7 @@ static int split_share(e13_ctx *c, const e13_job *job, const e13_tuning &tu, int
     t.step_cap = kSplitStepCap;
     t.run_skip = 1;
     Params S = make_params(c, t, job->nq, nwarps, nwarps * 32, stack_n);
+    S.exact_cap = 1;
     S.jobs = jobs;
     S.jobcnt = jobcnt;
     S.stack = stack;

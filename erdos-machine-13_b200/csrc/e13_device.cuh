@@ -3,8 +3,10 @@
 //
 // One Turing machine per lane.  A lane's tape (1364 cells, bit-packed into 43
 // words) and its table (16 rows of two 16-bit cell slots) live in shared
-// memory, interleaved by lane: word w of lane l sits at [w * blockDim + l], so
-// every lane always hits its own bank and a warp-wide access never conflicts.
+// memory, a warp's columns together and interleaved by lane: word w of lane l
+// sits at [32 * w + l] of its warp's part, so every lane always hits its own
+// bank and a warp-wide access never conflicts.  (run_full_kernel and raw_kernel
+// interleave a whole block's columns, [w * blockDim + l].)
 //
 // Semantics follow the reference's run() (src/e13search.c:134-177) step for
 // step: stage test, deadline, read, fork on a first read, halt, write + hash,
@@ -23,6 +25,13 @@ constexpr int kTapeWords = 43;    // ceil(1364 / 32)
 constexpr int kLeft = 64;
 constexpr int kStages = 9;
 constexpr int kCounterCells = 62; // cells < -2 hash into the counter hash hc
+
+// erdos_14's step at the start of each stage, and the deadline of stage n for
+// every machine (src/e13search.c:70, :159).
+__host__ __device__ constexpr int stage_deadline(int n) {
+  constexpr int step[kStages + 1] = {0, 2, 22, 90, 268, 944, 3434, 13450, 52068, 208864};
+  return 4 * step[n] + 64;
+}
 
 // Cell entry (one byte): 0..63 a move (the reference's code), plus flags.
 constexpr u32 kEntHalt = 0x40;    // halt
@@ -119,7 +128,7 @@ constexpr int kErrOverflow = 1, kErrOutFull = 2, kErrTimeout = 4;
 // The filter's constant tables (set by the host from e13_keys()).
 __constant__ u64 c_key[kTapeCells];
 __constant__ u64 c_tgt[kStages + 2];
-__constant__ int c_deadline[kStages + 2];  // 4 * erdos_14 stage step + 64 (src/e13search.c:159)
+__constant__ int c_deadline[kStages + 2];  // stage_deadline
 __constant__ int c_exc[kStages + 1];       // exceptions by stage (src/e13search.c:71)
 
 // Shared-memory key tables of the filter, in one block of kKeySmemBytes:
@@ -352,6 +361,22 @@ __device__ __forceinline__ int row_slot(u32 row, bool one) {
   return e;
 }
 
+// lane_steps<N> tests the deadline after N steps: a machine that reports t =
+// deadline + 1 and dies may have gone N steps on from there, and written on its
+// way.  Whether the words that the lane's next load clears (tape_extent of t)
+// hold all of these cells: a stale bit would change the next machine.  t steps
+// lead at most t cells to the right, and t - 2 past stage 1, whose block has the
+// one at cell -1 in it.  (N = 9: cell 223 of words 0..6 for the deadline of
+// stage 2; N = 10 would reach cell 224.)
+__host__ __device__ constexpr bool overrun_cleared(int n) {
+  for (int s = 1; s <= kStages; ++s) {
+    const int t = stage_deadline(s) + 1, last = kTapeCells - 1;
+    const int reach = kLeft + t + n - 1 - (s > 1 ? 2 : 0), cleared = kLeft + t;
+    if (((reach < last ? reach : last) >> 5) > ((cleared < last ? cleared : last) >> 5) || kLeft - t >= 32) return false;
+  }
+  return true;
+}
+
 // N steps of a running lane whose table and tape columns are 32 words apart:
 // the persistent search's hot loop.  left: steps that still pass the deadline
 // test (deadline + 1 - t); row: 4 times the state.  Returns 0 (all N taken), or
@@ -377,6 +402,7 @@ template <int N>
 __device__ __forceinline__ int lane_steps(Lane &L, int &left, u32 &row, u32 *__restrict__ tcol,
                                           const u32 *__restrict__ rcol, const u32 *__restrict__ keyb, int &cell,
                                           u32 &ecell) {
+  static_assert(overrun_cleared(N), "cells written past the deadline must be cleared with the machine's own");
   bool stop = false;  // the last step left the window or led to a match
 #pragma unroll
   for (int i = 0; i <= N; ++i) {

@@ -111,7 +111,7 @@ static inline void build_root(const e13_job *job, int slot, Node *root, bool run
   memset(root, 0, sizeof *root);
   root->job = (unsigned char)slot;
   root->p = kLeft;
-  root->deadline = 4 * 2 + 64;
+  root->deadline = stage_deadline(1);
   root->nt = 1;
   root->st0 = -1;
   root->p0 = kLeft;  // head0 = 0 until stage 1 sets it (src/e13search.c:123-129)
@@ -140,13 +140,12 @@ static inline void build_root(const e13_job *job, int slot, Node *root, bool run
 static inline cudaError_t upload_filter_tables() {
   uint64_t key[kTapeCells], tgt[E13_STAGES + 1];
   e13_keys(key, tgt);
-  static const long erdos14_stage_step[E13_STAGES + 1] = {0, 2, 22, 90, 268, 944, 3434, 13450, 52068, 208864};
   static const int exc[E13_STAGES + 1] = {0, 0, 0, 1, 1, 1, 1, 1, 1, 2};
   u64 t11[E13_STAGES + 2] = {0};
   int dl[E13_STAGES + 2] = {0};
   for (int n = 0; n <= E13_STAGES; ++n) {
     t11[n] = tgt[n];
-    dl[n] = (int)(4 * erdos14_stage_step[n] + 64);
+    dl[n] = stage_deadline(n);
   }
   t11[0] = ~0ull;  // never a target
   cudaError_t e;

@@ -77,6 +77,8 @@ constexpr int kLoneSteps = 512;
 // lanes 593 / 30.6 / 146, 24 lanes 616 / 32.7 / 152).
 // While warps wait for work slices stay at 72 steps: with 216 some counter
 // neighbourhoods took a second epoch, 4.8 instead of 3.2 ms.
+// (12 and 24 steps were timed only: with more than 9, a lane's next load would
+// have to clear more of its tape, see overrun_cleared.)
 constexpr int kSteps = 9;
 constexpr int kLeastLanes = 16;
 

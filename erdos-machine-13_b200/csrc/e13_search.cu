@@ -133,7 +133,6 @@ struct Params {
   unsigned long long *jobcnt;  // kMaxJobs x kJobCounters totals
   int nq;
   int slice, step_cap, wdepth, pool_low, run_skip;
-  int exact_cap;             // plain: step_cap holds to the step, not to the slice
   int park_after, park_idle; // persistent: hand a machine over after this many steps since its load (while
                              // warps wait for work)
   long long out_cap, out_soft, surv_cap, pool_cap;
@@ -324,7 +323,11 @@ static __device__ __noinline__ long long next_input(Input *in, Ctl *ctl, long lo
 
 __device__ __forceinline__ int wrap(int s, int d) { return s >= d ? s - d : s; }
 
-template <bool PERSIST>
+// EXACT (plain): the expansion of shards (split_share), where a lane stops
+// exactly at its step cap, as it would at a deadline, whatever the other lanes
+// of its warp do: the frontier is then a function of the job.  (A kernel of its
+// own: with the test of a flag the plain kernel's searches took 2-10 % longer.)
+template <bool PERSIST, bool EXACT = false>
 __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ Params P) {
   // an epoch with nothing to do (the search ended inside its graph of epochs)
   if (P.ctl->top == 0 && P.ctl->pool_tail == 0) return;
@@ -757,12 +760,9 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
       if (rm) {
         int left = L.deadline + 1 - L.t;
         u32 row = (u32)L.st << 2;
-        // the expansion of shards: a lane stops exactly at its step cap, as it
-        // would at a deadline, whatever the other lanes of its warp do, so that
-        // the frontier is a function of the job (split_share)
-        int deadline = L.deadline;
-        const int last = !PERSIST && P.exact_cap ? L.tseg + P.step_cap - 1 : 0x7FFFFFFF;
-        if (!PERSIST) L.deadline = min(deadline, last);
+        int deadline = L.deadline;  // EXACT: the machine's own
+        const int last = L.tseg + P.step_cap - 1;
+        if (EXACT) L.deadline = min(deadline, last);
         // (a warp with idle lanes takes up new machines; a starving one has
         // forks that others wait for)
         const int least = min(kLeastLanes, __popc(rm)), most = PERSIST && starving ? (P.slice + 2) / 3 : P.slice;
@@ -791,7 +791,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
               ev = lane_act<false>(L, tcol, rcol, K, stride, cell, e);
               if (!ev) ev = lane_act<false>(L, tcol, rcol, K, stride, cell, e);
             }
-            if (!PERSIST && ev == kEvDead && L.t > last && L.t <= deadline) {
+            if (EXACT && ev == kEvDead && L.t > last && L.t <= deadline) {
               status = kStCap;
               ev = 0;
             }
@@ -802,13 +802,11 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
               if (PERSIST) {
                 L.t = L.deadline + 1 - left;
                 L.st = (int)(row >> 2);
-              } else {
-                L.deadline = deadline;
               }
+              if (EXACT) L.deadline = deadline;
               ev = stage_check(L, tcol, K, stride);
-              if (PERSIST) {
-                left = L.deadline + 1 - L.t;
-              } else {
+              left = L.deadline + 1 - L.t;
+              if (EXACT) {
                 deadline = L.deadline;
                 L.deadline = min(deadline, last);
               }
@@ -846,9 +844,8 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
         if (PERSIST) {
           L.t = L.deadline + 1 - left;
           L.st = (int)(row >> 2);
-        } else {
-          L.deadline = deadline;
         }
+        if (EXACT) L.deadline = deadline;
         if (__any_sync(kFull, status >= kStDead)) {
           if (status >= kStDead) {
             acc_steps += (u32)(L.t - L.tseg);
@@ -882,7 +879,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
             }
           }
         }
-        if (!PERSIST && (status == kStCap || (status == kStRun && L.t - L.tseg >= P.step_cap))) {
+        if (!PERSIST && ((EXACT && status == kStCap) || (status == kStRun && L.t - L.tseg >= P.step_cap))) {
           acc_steps += (u32)(L.t - L.tseg);
           L.tseg = L.t;
           if (acc_steps >= 0x80000000u) flush_counts();
@@ -2043,7 +2040,6 @@ static int split_share(e13_ctx *c, const e13_job *job, const e13_tuning &tu, int
     t.step_cap = kSplitStepCap;
     t.run_skip = 1;
     Params S = make_params(c, t, job->nq, nwarps, nwarps * 32, stack_n);
-    S.exact_cap = 1;
     S.jobs = jobs;
     S.jobcnt = jobcnt;
     S.stack = stack;
@@ -2054,9 +2050,9 @@ static int split_share(e13_ctx *c, const e13_job *job, const e13_tuning &tu, int
     S.surv_cap = surv_n;
     S.ctl = ctl;
     const size_t smem = search_smem(tu.block);
-    fail(cudaFuncSetAttribute(search_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "attr");
+    fail(cudaFuncSetAttribute(search_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "attr");
     for (int level = 0; rc == E13_OK && level < kSplitLevels && top > 0 && top < target; ++level) {
-      search_kernel<false><<<c->nsm, tu.block, smem, c->stream>>>(S);
+      search_kernel<false, true><<<c->nsm, tu.block, smem, c->stream>>>(S);
       move_outputs<<<c->nsm * 4, 256, 0, c->stream>>>(ctl, stack, out, c->pool, 0, stack_n);
       finish_launch<<<1, 1, 0, c->stream>>>(ctl, stack_n, kWholeFrontier, 0);
       *launches += 3;

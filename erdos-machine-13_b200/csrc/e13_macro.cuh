@@ -101,7 +101,7 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem<BITS> &M, co
   // before it and the cells it changed)
   int noted = 0, v_b = 0, v_left = 0;
   u32 v_key = 0, v_d = 0;
-  int snap_b = 0, snap_left = 0, snaps = 0;
+  int snap_b = 0, snaps = 0;
   u32 snap_at = 0, snap0 = 0, snap1 = 0, snap2 = 0;  // words snap_b - 1 .. snap_b + 1
   bool far = true;                  // left those words, or reached a stage, since the snapshot
   // bare runs: batches until the next look at what visits yield, steps left and
@@ -222,7 +222,7 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem<BITS> &M, co
       // word and its neighbours were entered and ended as they were
       const int b0 = __shfl_sync(kAll, v_b, 0);
       const u32 key0 = __shfl_sync(kAll, v_key, 0);
-      if (__any_sync(kAll, lane < noted && (unsigned)(v_b - snap_b + 1) > 2u)) far = true;
+      if (HASH && __any_sync(kAll, lane < noted && (unsigned)(v_b - snap_b + 1) > 2u)) far = true;
       m = __ballot_sync(kAll, lane > 0 && lane < noted && v_b == b0 && v_key == key0);
       for (int tries = 0; m && tries < kLoopTries; ++tries, m &= m - 1) {
         const int j = __ffs(m) - 1;
@@ -306,30 +306,31 @@ __device__ __forceinline__ int macro_run(Lane &L, u64 &hb, MacroMem<BITS> &M, co
       single = inside || window_left > 0;
       continue;
     }
-    // single steps until the head is in another word
-    // a loop that passes through here every turn: the same configuration
-    // again, on words not left since the snapshot?
-    if ((unsigned)(b - snap_b + 1) > 2u) far = true;
-    const u32 at_here = ((u32)p << 4) | (u32)st;
-    if (!far && at_here == snap_at && M.tape[b] == snap1 && M.tape[b - 1] == snap0 && M.tape[b + 1] == snap2) {
-      if (HASH) left = 0;
-      else left %= snap_left - left;
-      far = true;
-    }
-    if (--snaps < 0 && (unsigned)(b - 1) < (unsigned)(kLastWord - 1)) {
-      snaps = kSnapEvery;
-      snap_b = b;
-      snap_at = at_here;
-      snap_left = left;
-      snap0 = M.tape[b - 1];
-      snap1 = M.tape[b];
-      snap2 = M.tape[b + 1];
-      far = false;
-      if (HASH && macro_late(t_end)) {
-        L.p = p;
-        L.st = st;
-        L.t = L.deadline + 1 - left;
-        return kEvRun;
+    // single steps until the head is in another word (bare runs: in the first
+    // and last word only)
+    if (HASH) {
+      // a loop that passes through here every turn: the same configuration
+      // again, on words not left since the snapshot?
+      if ((unsigned)(b - snap_b + 1) > 2u) far = true;
+      const u32 at_here = ((u32)p << 4) | (u32)st;
+      if (!far && at_here == snap_at && M.tape[b] == snap1 && M.tape[b - 1] == snap0 && M.tape[b + 1] == snap2) {
+        left = 0;
+        far = true;
+      }
+      if (--snaps < 0 && (unsigned)(b - 1) < (unsigned)(kLastWord - 1)) {
+        snaps = kSnapEvery;
+        snap_b = b;
+        snap_at = at_here;
+        snap0 = M.tape[b - 1];
+        snap1 = M.tape[b];
+        snap2 = M.tape[b + 1];
+        far = false;
+        if (macro_late(t_end)) {
+          L.p = p;
+          L.st = st;
+          L.t = L.deadline + 1 - left;
+          return kEvRun;
+        }
       }
     }
     u32 word = M.tape[b];

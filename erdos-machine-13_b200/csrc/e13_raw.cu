@@ -4,14 +4,15 @@
 // with the stage test and the deadline removed).
 //
 // Most random tables halt or leave the window within 1,300 steps; one in nine
-// of 13 states loops in place to the limit, and these took 99 % of the steps.  raw_kernel runs one machine per lane in the search's
-// lock-step form for at most kRawSteps steps and lists the machines that live
-// longer; raw_long_kernel runs each of those in a warp of its own, a tape word
-// at a time (e13_macro.cuh), which leaves out whole turns of a repeated
-// configuration.  A million machines of at most 2^18 steps, one B200: 132 ms
-// in one kernel, now 4.9 ms and 18.9 ms (31 ms with the rows' copy); the second
-// is the time of the few machines that neither loop nor sweep (a counter in
-// one word), 80 cycles a step.
+// of 13 states loops in place to the limit, and these took 99 % of the steps.
+// raw_kernel runs one machine per lane in the search's lock-step form for at
+// most kRawSteps steps and lists the machines that live longer; raw_long_kernel
+// runs each of those in a warp of its own, a tape word at a time
+// (e13_macro.cuh), which leaves out whole turns of a repeated configuration.  A
+// million machines of at most 2^18 steps, one B200: 132 ms in one kernel, now
+// 4.9 ms and 19 ms (a call that returns totals 25 ms, one that copies the rows
+// 28-31); the second is the time of the few machines that neither loop nor
+// sweep (a counter in one word), 80 cycles a step.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -30,9 +31,23 @@ constexpr long long kRawIntMax = 1 << 30; // longer limits are run in raw_kernel
 constexpr int kRawLongBlock = 256;
 constexpr int kRawLongPerSm = 3;          // 68 KB of shared memory a block
 // 24 warps an SM with 512 visits each: the listed machines are many and short
-// lived, so warps count for more than visits (a million draws: 38 ms; 12 warps
-// with 1024 visits 38-41, 6 with 2048 45).
+// lived, so warps count for more than visits (a million machines with their
+// rows, three seeds: 28-31 ms; 12 warps with 1024 visits 29-30, 6 with 2048
+// 36-37).
 typedef MacroMem<9> RawMem;
+
+// Steps beyond kRawSteps from which the listed machines are better off in
+// raw_long_kernel, which starts each of them anew and runs 3,552 at a time, than
+// in the lanes that they have.  With 13 states the two take the same time at
+// 230 steps for 500 machines, 435 for 20,000, 1480 for 100,000, 2900 for
+// 200,000, 5000 for a million, 7200 for 4 million and 8000 for 16 million (a
+// million: limit 2000 6.5 ms in lanes, 9.6 listed; limit 12,000 15.2 and 11.5);
+// with two states, where fewer machines live, at 165, 310, 650, 1180, 4000,
+// 6800 and 8700.
+long long raw_list_from(long long n, int nq) {
+  const long long by_count = n / 75 < 2200 + n / 400 ? n / 75 : 2200 + n / 400;
+  return (200 + (by_count < 7500 ? by_count : 7500)) * (16 + nq) / 29;
+}
 
 __device__ __forceinline__ u64 splitmix_at(u64 seed, u64 k) {
   // draw k (1-based) of splitmix64 started at `seed`
@@ -216,7 +231,7 @@ extern "C" int e13_raw_run(e13_ctx *ctx, const uint8_t *codes, uint64_t seed, in
   int *d_list = nullptr;
   // the macro simulator counts steps in 32 bits and lists machines by int;
   // without room for the list (4 bytes a machine) the first kernel runs them all
-  bool park = max_steps > kRawSteps && max_steps <= kRawIntMax && n <= 0x7FFFFFFFLL;
+  bool park = max_steps > kRawSteps + raw_list_from(n, nq) && max_steps <= kRawIntMax && n <= 0x7FFFFFFFLL;
   int rc = E13_OK;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);

@@ -63,12 +63,12 @@ def test_working_memory_leaves_room_for_a_search(searches):
 
 def test_raw_machines_run_without_room_for_their_list():
     """Totals of machines generated on the device need no memory by their number:
-    where the list of the ones that live long (4 bytes a machine) finds no room,
-    they run all the same."""
-    n, most = 1 << 27, 1100
+    where the list of the ones that live long (4 bytes a machine, for a limit
+    that makes it worth while) finds no room, they run all the same."""
+    n, most = 1 << 24, 12000
     with E.Context(0) as c:
         c.raw_run(1000, max_steps=most, want_out=False)
-        held = torch.empty(free_bytes() - (256 << 20), dtype=torch.uint8, device="cuda")
+        held = torch.empty(free_bytes() - (32 << 20), dtype=torch.uint8, device="cuda")
         try:
             _, without = c.raw_run(n, max_steps=most, want_out=False)
         finally:

@@ -59,11 +59,12 @@ __device__ __forceinline__ unsigned long long macro_clock() {
   return t;
 }
 
-// By the whole warp: has the clock passed t_end?  Lanes read clocks of their
-// own, which may differ, and all take the way that follows from the answer: it
-// is lane 0's.
+// By the whole warp: has the clock passed t_end (kNoEnd: there is none)?  Lanes
+// read clocks of their own, which may differ, and all take the way that follows
+// from the answer: it is lane 0's.
+constexpr unsigned long long kNoEnd = ~0ull;
 __device__ __forceinline__ bool macro_late(unsigned long long t_end) {
-  return __shfl_sync(kAll, macro_clock() > t_end ? 1 : 0, 0) != 0;
+  return t_end != kNoEnd && __shfl_sync(kAll, macro_clock() > t_end ? 1 : 0, 0) != 0;
 }
 
 // After a change of M.rows: the expanded table, and an empty memory of visits.

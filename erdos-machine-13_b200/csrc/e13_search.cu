@@ -1379,7 +1379,7 @@ __global__ void __launch_bounds__(kLongBlock) full_long_kernel(const int *tabs, 
     u64 hb = 0;
     u32 reads = 0, ecell = 0;
     int cell = 0;
-    int ev = macro_run<true>(L, hb, M, K, span, lane, reads, cell, ecell, ~0ull);
+    int ev = macro_run<true>(L, hb, M, K, span, lane, reads, cell, ecell, kNoEnd);
     if (ev == kEvCell) ev = kEvDead;
     if (lane == 0) full_result(L, ev, out + 7LL * m);
     __syncwarp();

@@ -1291,8 +1291,8 @@ __global__ void finish_launch(Ctl *ctl, long long cap, long long batch_max, long
 // steps and lists the ones that live longer, which full_long_kernel runs one
 // per warp from the blank tape.  In one kernel the longest machine of each
 // warp held up the other 31, and a loop to the deadline took 80 ms (20,000
-// mutants with 2 changed cells: 26-85 ms, now 5.6 ms: 0.7 ms and 3 ms for the
-// two kernels, the rest copies and allocation).
+// mutants with 2 changed cells: 7.5-112 ms, now 3.0 ms: 0.62 ms and 2.1 ms for
+// the two kernels, the rest copies).
 constexpr int kFullSteps = 1024;
 
 __device__ u32 full_row(const int *tab, int nq, int s) {
@@ -2497,10 +2497,11 @@ extern "C" int e13_autotune_jobs(e13_ctx *c, const e13_job *jobs, int n, int32_t
   // block: lanes per CTA (one CTA per SM); slice: iterations between a
   // warp's refill rounds; warp_stack: the depth of subtree a warp keeps to
   // itself before it spills or donates; pool_low_pct: the threshold below
-  // which warps with deep stacks fork work off to idle warps; run_skip: the
-  // machine age (steps) from which a warp takes word-at-a-time run skips
+  // which warps with deep stacks fork work off to idle warps; run_skip: half
+  // the steps after which a machine goes to the long-machine kernel (1024: the
+  // least it takes, kParkMin)
   const Axis axes[] = {
-      {&e13_tuning::run_skip, {1, 1024, 4096, 8192, 32768}, 5},
+      {&e13_tuning::run_skip, {kParkMin / 2, 4096, 8192, 32768, 0}, 4},
       {&e13_tuning::block, {512, 640, 768, 0, 0}, 3},
       {&e13_tuning::slice, {8, 12, 16, 24, 32}, 5},
       {&e13_tuning::warp_stack, {64, 128, 256, 512, 0}, 4},

@@ -97,13 +97,14 @@ typedef struct e13_tuning {
   int32_t step_cap;          /* plain kernel: steps per work item before it is requeued */
   int32_t batch;             /* nodes taken from the frontier per launch / epoch (0 = auto: the whole
                                 frontier for the persistent kernel, 16384 for the plain one) */
-  int32_t epoch_us;          /* persistent: wall-clock bound of one epoch, microseconds */
+  int32_t epoch_us;          /* persistent: wall-clock bound of one epoch, microseconds (below 2500 the
+                                long-machine kernel may add up to 1 ms) */
   int32_t epochs_per_graph;  /* persistent: epochs captured in one CUDA graph */
   int32_t pool_low_pct;      /* persistent: warps donate stack nodes while the pool holds fewer than this % of warps */
   int32_t run_skip;          /* old machines advance by more than a step at a time (exact in every form):
-                                0 never, 1 as early as possible, N >= 2: the persistent kernel hands a
-                                machine over to the long-machine kernel once it has run 2 N steps since it
-                                was loaded (sooner while warps wait for work).  The plain kernel crosses runs
+                                0 never, N >= 1: the persistent kernel hands a machine over to the
+                                long-machine kernel once it has run 2 N steps since it was loaded, 2048 at
+                                least (2048 while warps wait for work).  The plain kernel crosses runs
                                 of a self-loop a tape word at a time for every N >= 1, since each of its
                                 launches waits for its oldest machine */
   int64_t stack_nodes;       /* frontier stack capacity in nodes (0 = auto) */
@@ -179,7 +180,9 @@ int e13_resolve_tuning(const e13_tuning *in, int serve, e13_tuning *out);
 /* ---- device path ---- */
 
 /* Creates a context on CUDA device `device` (allocations happen lazily on
-   the first search and are kept for reuse).  Returns E13_OK or an error. */
+   the first search and are kept for reuse, working memory of a call up to 1 GiB
+   a buffer and a session's second stack up to 16 Mi nodes; what is only kept is
+   given back when another buffer of the context finds no room).  Returns E13_OK or an error. */
 int e13_ctx_create(int device, e13_ctx **out);
 void e13_ctx_destroy(e13_ctx *ctx);
 

@@ -323,11 +323,11 @@ static __device__ __noinline__ long long next_input(Input *in, Ctl *ctl, long lo
 
 __device__ __forceinline__ int wrap(int s, int d) { return s >= d ? s - d : s; }
 
-// EXACT (plain): the expansion of shards (split_share), where a lane stops
-// exactly at its step cap, as it would at a deadline, whatever the other lanes
-// of its warp do: the frontier is then a function of the job.  (A kernel of its
-// own: with the test of a flag the plain kernel's searches took 2-10 % longer.)
-template <bool PERSIST, bool EXACT = false>
+// ALONE (plain): the expansion of shards (split_share), where a warp takes its
+// next node only when it is done with the last one.  How far a machine goes
+// past the step cap hangs on what else its warp runs, which is then nothing but
+// its siblings: the frontier is a function of the job.
+template <bool PERSIST, bool ALONE = false>
 __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ Params P) {
   // an epoch with nothing to do (the search ended inside its graph of epochs)
   if (P.ctl->top == 0 && P.ctl->pool_tail == 0) return;
@@ -538,6 +538,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
         } else {
           const Node *src = nullptr;
           bool from_pool = false;
+          if (ALONE && im != kFull) break;
           if (!input_done) {
             if (PERSIST && !busy) {
               if (lane == 0) atomicAdd(&ctl->busy, 1);  // before any claim, so idle warps see work in flight
@@ -760,9 +761,6 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
       if (rm) {
         int left = L.deadline + 1 - L.t;
         u32 row = (u32)L.st << 2;
-        int deadline = L.deadline;  // EXACT: the machine's own
-        const int last = L.tseg + P.step_cap - 1;
-        if (EXACT) L.deadline = min(deadline, last);
         // (a warp with idle lanes takes up new machines; a starving one has
         // forks that others wait for)
         const int least = min(kLeastLanes, __popc(rm)), most = PERSIST && starving ? (P.slice + 2) / 3 : P.slice;
@@ -791,10 +789,6 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
               ev = lane_act<false>(L, tcol, rcol, K, stride, cell, e);
               if (!ev) ev = lane_act<false>(L, tcol, rcol, K, stride, cell, e);
             }
-            if (EXACT && ev == kEvDead && L.t > last && L.t <= deadline) {
-              status = kStCap;
-              ev = 0;
-            }
             // the stage test of a hash match, once per iteration outside
             // lane_act: one copy of it in the loop instead of one per
             // inlined action (the second action waits for it)
@@ -803,13 +797,8 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
                 L.t = L.deadline + 1 - left;
                 L.st = (int)(row >> 2);
               }
-              if (EXACT) L.deadline = deadline;
               ev = stage_check(L, tcol, K, stride);
               left = L.deadline + 1 - L.t;
-              if (EXACT) {
-                deadline = L.deadline;
-                L.deadline = min(deadline, last);
-              }
             }
             if (ev == kEvCell) {
               if (e == kEntHalt) {
@@ -845,7 +834,6 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
           L.t = L.deadline + 1 - left;
           L.st = (int)(row >> 2);
         }
-        if (EXACT) L.deadline = deadline;
         if (__any_sync(kFull, status >= kStDead)) {
           if (status >= kStDead) {
             acc_steps += (u32)(L.t - L.tseg);
@@ -879,7 +867,7 @@ __global__ void __launch_bounds__(768, 1) search_kernel(const __grid_constant__ 
             }
           }
         }
-        if (!PERSIST && ((EXACT && status == kStCap) || (status == kStRun && L.t - L.tseg >= P.step_cap))) {
+        if (!PERSIST && status == kStRun && L.t - L.tseg >= P.step_cap) {
           acc_steps += (u32)(L.t - L.tseg);
           L.tseg = L.t;
           if (acc_steps >= 0x80000000u) flush_counts();
@@ -1973,7 +1961,7 @@ static ShardKey shard_key(const Node &n) {
 
 constexpr long long kSplitPerShard = 512;  // frontier nodes per shard before the deal
 constexpr int kSplitLevels = 24;           // most plain launches of the split
-constexpr int kSplitSlice = 24;            // the split's slice and step cap (fixed: the cap shapes the frontier)
+constexpr int kSplitSlice = 24;            // the split's slice and step cap (fixed: they shape the frontier)
 constexpr int kSplitStepCap = 20000;
 
 // One share of a search split over nshards (the reference's SPLIT frontier,
@@ -1986,13 +1974,13 @@ constexpr int kSplitStepCap = 20000;
 // are zero / empty for the other shards.  Runs on scratch buffers of its own,
 // so a serve session's frontier is left alone; `slot` is
 // the job slot written into the nodes.  The expansion runs with a fixed
-// slice, step cap and run skip: a lane is requeued at the step cap, so the cap
-// shapes the frontier, and with it fixed
+// slice, step cap and run skip: a lane is requeued at the first slice end
+// past the step cap, so those settings shape the frontier, and with them fixed
 // every shard's content depends on the job alone, whatever tuning the caller's
-// search then uses (the autotuner compares shard 0 across tunings).  (Where a
-// lane went on to the end of its slice, as long as its warp's other lanes made
-// it, shares of 18 or more did not add up: FMAX = 3, X = 8 in 64 shares was up
-// to 1849 leaves and 5 survivors off.)
+// search then uses (the autotuner compares shard 0 across tunings).  Its
+// warps take one node at a time, for how long a slice is hangs on what a warp
+// runs (where they took nodes as lanes fell idle, shares of 18 or more did not
+// add up: FMAX = 3, X = 8 in 64 shares was up to 1849 leaves and 5 survivors off).
 static int split_share(e13_ctx *c, const e13_job *job, const e13_tuning &tu, int shard, int nshards, int slot,
                        std::vector<Node> &mine, unsigned long long cnt[kJobCounters], std::vector<SurvRec> &recs,
                        long long *launches) {

@@ -1,6 +1,6 @@
 """Many shares of one job: each call expands the job again, so they add up only if
-every expansion leaves the same frontier.  From 18 shares on the expansion of a
-job with long machines runs some of them to its step cap."""
+every expansion leaves the same frontier, with long machines of the job stopped
+at the same steps."""
 import pytest
 
 import e13b200 as E
